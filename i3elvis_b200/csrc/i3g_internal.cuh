@@ -30,6 +30,10 @@ __device__ __forceinline__ void pdl_enter()
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// the two halves, for kernels that fetch data their predecessor does not write before they wait
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 inline bool pdl_enabled()
 {
     static const bool on = getenv("I3G_PDL") == nullptr || atoi(getenv("I3G_PDL")) != 0;
@@ -73,6 +77,9 @@ struct BcList {
     int na = -1;
     int *first = nullptr;
     int *writer = nullptr;
+    // the same rows packed for homogeneous systems (stokes.cu, bc_packed)
+    bool packed = false;
+    int4 *inl = nullptr, *w4 = nullptr, *ext = nullptr;
 };
 
 template <typename T>
@@ -183,6 +190,7 @@ struct i3g_ctx {
     int fuse = 1;                               // boundary rows inside the relaxation kernels of levels >= 1
                                                 // (3: level 0 too), residual and four-component transfer
                                                 // launches (0: one launch per pass)
+    long pro_nodes = 0;                         // largest level whose relaxations start before their predecessor ends
     int coop_blocks = 0;                        // its grid: every CTA resident at once (0: no cooperative launch)
     unsigned *dbar = nullptr;                   // its grid barrier: arrival count, generation
     int *dbar_err = nullptr;                    // set when a grid barrier wait timed out

@@ -135,134 +135,201 @@ __device__ __forceinline__ T cf(T a, T n, T k)   // ((a*n)*2)*k: -ynval*nueff*2.
     return Ar<T>::mul(Ar<T>::mul(Ar<T>::mul(a, n), T(2)), k);
 }
 
-// x-momentum row at node n = (i,j,k) (xstokserr, move3mg.c:718-903): accumulates the 17
-// slots in the reference's order into s and returns the diagonal.
+// Coefficients of a momentum row: the own component's six neighbours (c[0..5], in the order each row
+// function lists them), the four shear coefficients (c[6..9]), the pressure factor k and the diagonal
+// d.  They depend on the viscosities and the grid only, not on the unknowns, so the relaxation kernels
+// of small levels compute them before they wait for their predecessor (PRO).
+template <typename T>
+struct Row {
+    T c[10], k, d;
+};
+
+// x-momentum row at node n = (i,j,k) (xstokserr, move3mg.c:718-903): c = A, B, Sy, Ny, Fz, Kz, Sx,
+// Nx, Fx, Kx
+template <typename T>
+__device__ __forceinline__ Row<T> xcoef(const View<T> &L, int i, int j, int k, long n)
+{
+    using A = Ar<T>;
+    const long NY = L.ny, NXY = L.nxy;
+    Row<T> R;
+    const T XK = A::mul(T(2), L.isx[i]), YK = L.icy[j + 1], ZK = L.icz[k + 1];
+    R.c[0] = cf(XK, L.etac[n + NXY + 1], L.icx[i]);
+    R.c[1] = cf(XK, L.etac[n + NXY + NY + 1], L.icx[i + 1]);
+    const T nS = L.etaxy[n], nN = L.etaxy[n + 1], xkS = L.isx[i];
+    R.c[2] = cf(YK, nS, L.isy[j]); R.c[6] = cf(YK, nS, xkS);
+    R.c[3] = cf(YK, nN, L.isy[j + 1]); R.c[7] = cf(YK, nN, xkS);
+    const T nF = L.etaxz[n], nK = L.etaxz[n + NXY];
+    R.c[4] = cf(ZK, nF, L.isz[k]); R.c[8] = cf(ZK, nF, xkS);
+    R.c[5] = cf(ZK, nK, L.isz[k + 1]); R.c[9] = cf(ZK, nK, xkS);
+    T d = -R.c[0];
+#pragma unroll
+    for (int q = 1; q < 6; q++) d = A::add(d, -R.c[q]);
+    R.d = d;
+    R.k = XK;
+    return R;
+}
+
+// accumulates the row's 17 slots in the reference's order into s
+template <typename T, bool RES>
+__device__ __forceinline__ void xsum(const View<T> &L, const Row<T> &R, long n, T &s)
+{
+    const long NY = L.ny, NXY = L.nxy;
+    const T *vx = L.u1, *vy = L.u2, *vz = L.u3, *p = L.u0;
+    acc<T, RES>(s, R.d, vx[n]);
+    acc<T, RES>(s, R.c[0], vx[n - NY]);
+    acc<T, RES>(s, R.c[1], vx[n + NY]);
+    acc<T, RES>(s, R.c[2], vx[n - 1]);
+    acc<T, RES>(s, R.c[3], vx[n + 1]);
+    acc<T, RES>(s, R.c[4], vx[n - NXY]);
+    acc<T, RES>(s, R.c[5], vx[n + NXY]);
+    acc<T, RES>(s, R.c[6], vy[n - NY]);
+    acc<T, RES>(s, -R.c[7], vy[n - NY + 1]);
+    acc<T, RES>(s, -R.c[6], vy[n]);
+    acc<T, RES>(s, R.c[7], vy[n + 1]);
+    acc<T, RES>(s, R.c[8], vz[n - NY]);
+    acc<T, RES>(s, -R.c[9], vz[n - NY + NXY]);
+    acc<T, RES>(s, -R.c[8], vz[n]);
+    acc<T, RES>(s, R.c[9], vz[n + NXY]);
+    acc<T, RES>(s, R.k, p[n + NXY + 1]);
+    acc<T, RES>(s, -R.k, p[n + NXY + NY + 1]);
+}
+
+// y-momentum row (ystokserr, move3mg.c:910-1101): c = A, B, Wx, Ex, Fz, Kz, Wy, Ey, Fy, Ky
+template <typename T>
+__device__ __forceinline__ Row<T> ycoef(const View<T> &L, int i, int j, int k, long n)
+{
+    using A = Ar<T>;
+    const long NY = L.ny, NXY = L.nxy;
+    Row<T> R;
+    const T XK = L.icx[i + 1], YK = A::mul(T(2), L.isy[j]), ZK = L.icz[k + 1];
+    R.c[0] = cf(YK, L.etac[n + NY + NXY], L.icy[j]);
+    R.c[1] = cf(YK, L.etac[n + NY + 1 + NXY], L.icy[j + 1]);
+    const T nW = L.etaxy[n], nE = L.etaxy[n + NY], ykW = L.isy[j];
+    R.c[6] = cf(XK, nW, ykW); R.c[2] = cf(XK, nW, L.isx[i]);
+    R.c[7] = cf(XK, nE, ykW); R.c[3] = cf(XK, nE, L.isx[i + 1]);
+    const T nF = L.etayz[n], nK = L.etayz[n + NXY];
+    R.c[4] = cf(ZK, nF, L.isz[k]); R.c[8] = cf(ZK, nF, ykW);
+    R.c[5] = cf(ZK, nK, L.isz[k + 1]); R.c[9] = cf(ZK, nK, ykW);
+    T d = -R.c[0];
+#pragma unroll
+    for (int q = 1; q < 6; q++) d = A::add(d, -R.c[q]);
+    R.d = d;
+    R.k = YK;
+    return R;
+}
+
+template <typename T, bool RES>
+__device__ __forceinline__ void ysum(const View<T> &L, const Row<T> &R, long n, T &s)
+{
+    const long NY = L.ny, NXY = L.nxy;
+    const T *vx = L.u1, *vy = L.u2, *vz = L.u3, *p = L.u0;
+    acc<T, RES>(s, R.d, vy[n]);
+    acc<T, RES>(s, R.c[2], vy[n - NY]);
+    acc<T, RES>(s, R.c[3], vy[n + NY]);
+    acc<T, RES>(s, R.c[0], vy[n - 1]);
+    acc<T, RES>(s, R.c[1], vy[n + 1]);
+    acc<T, RES>(s, R.c[4], vy[n - NXY]);
+    acc<T, RES>(s, R.c[5], vy[n + NXY]);
+    acc<T, RES>(s, R.c[6], vx[n - 1]);
+    acc<T, RES>(s, -R.c[6], vx[n]);
+    acc<T, RES>(s, -R.c[7], vx[n + NY - 1]);
+    acc<T, RES>(s, R.c[7], vx[n + NY]);
+    acc<T, RES>(s, R.c[8], vz[n - 1]);
+    acc<T, RES>(s, -R.c[8], vz[n]);
+    acc<T, RES>(s, -R.c[9], vz[n - 1 + NXY]);
+    acc<T, RES>(s, R.c[9], vz[n + NXY]);
+    acc<T, RES>(s, R.k, p[n + NY + NXY]);
+    acc<T, RES>(s, -R.k, p[n + NY + 1 + NXY]);
+}
+
+// z-momentum row (zstokserr, move3mg.c:1109-1301): c = A, B, Wx, Ex, Sy, Ny, Wz, Ez, Sz, Nz
+template <typename T>
+__device__ __forceinline__ Row<T> zcoef(const View<T> &L, int i, int j, int k, long n)
+{
+    using A = Ar<T>;
+    const long NY = L.ny, NXY = L.nxy;
+    Row<T> R;
+    const T XK = L.icx[i + 1], YK = L.icy[j + 1], ZK = A::mul(T(2), L.isz[k]);
+    R.c[0] = cf(ZK, L.etac[n + NY + 1], L.icz[k]);
+    R.c[1] = cf(ZK, L.etac[n + NY + 1 + NXY], L.icz[k + 1]);
+    const T nW = L.etaxz[n], nE = L.etaxz[n + NY], zkW = L.isz[k];
+    R.c[6] = cf(XK, nW, zkW); R.c[2] = cf(XK, nW, L.isx[i]);
+    R.c[7] = cf(XK, nE, zkW); R.c[3] = cf(XK, nE, L.isx[i + 1]);
+    const T nS = L.etayz[n], nN = L.etayz[n + 1];
+    R.c[8] = cf(YK, nS, zkW); R.c[4] = cf(YK, nS, L.isy[j]);
+    R.c[9] = cf(YK, nN, zkW); R.c[5] = cf(YK, nN, L.isy[j + 1]);
+    T d = -R.c[0];
+#pragma unroll
+    for (int q = 1; q < 6; q++) d = A::add(d, -R.c[q]);
+    R.d = d;
+    R.k = ZK;
+    return R;
+}
+
+template <typename T, bool RES>
+__device__ __forceinline__ void zsum(const View<T> &L, const Row<T> &R, long n, T &s)
+{
+    const long NY = L.ny, NXY = L.nxy;
+    const T *vx = L.u1, *vy = L.u2, *vz = L.u3, *p = L.u0;
+    acc<T, RES>(s, R.d, vz[n]);
+    acc<T, RES>(s, R.c[2], vz[n - NY]);
+    acc<T, RES>(s, R.c[3], vz[n + NY]);
+    acc<T, RES>(s, R.c[4], vz[n - 1]);
+    acc<T, RES>(s, R.c[5], vz[n + 1]);
+    acc<T, RES>(s, R.c[0], vz[n - NXY]);
+    acc<T, RES>(s, R.c[1], vz[n + NXY]);
+    acc<T, RES>(s, R.c[8], vy[n - NXY]);
+    acc<T, RES>(s, -R.c[9], vy[n + 1 - NXY]);
+    acc<T, RES>(s, -R.c[8], vy[n]);
+    acc<T, RES>(s, R.c[9], vy[n + 1]);
+    acc<T, RES>(s, R.c[6], vx[n - NXY]);
+    acc<T, RES>(s, -R.c[6], vx[n]);
+    acc<T, RES>(s, -R.c[7], vx[n + NY - NXY]);
+    acc<T, RES>(s, R.c[7], vx[n + NY]);
+    acc<T, RES>(s, R.k, p[n + NY + 1]);
+    acc<T, RES>(s, -R.k, p[n + NY + 1 + NXY]);
+}
+
+// a whole row: accumulates it into s and returns the diagonal
 template <typename T, bool RES>
 __device__ __forceinline__ T xrow(const View<T> &L, int i, int j, int k, long n, T &s)
 {
-    using A = Ar<T>;
-    const long NY = L.ny, NXY = L.nxy;
-    const T XK = A::mul(T(2), L.isx[i]), YK = L.icy[j + 1], ZK = L.icz[k + 1];
-    const T cA = cf(XK, L.etac[n + NXY + 1], L.icx[i]);
-    const T cB = cf(XK, L.etac[n + NXY + NY + 1], L.icx[i + 1]);
-    const T nS = L.etaxy[n], nN = L.etaxy[n + 1], xkS = L.isx[i];
-    const T cSy = cf(YK, nS, L.isy[j]), cSx = cf(YK, nS, xkS);
-    const T cNy = cf(YK, nN, L.isy[j + 1]), cNx = cf(YK, nN, xkS);
-    const T nF = L.etaxz[n], nK = L.etaxz[n + NXY];
-    const T cFz = cf(ZK, nF, L.isz[k]), cFx = cf(ZK, nF, xkS);
-    const T cKz = cf(ZK, nK, L.isz[k + 1]), cKx = cf(ZK, nK, xkS);
-    T d = -cA;
-    d = A::add(d, -cB); d = A::add(d, -cSy); d = A::add(d, -cNy); d = A::add(d, -cFz); d = A::add(d, -cKz);
-    const T *vx = L.u1, *vy = L.u2, *vz = L.u3, *p = L.u0;
-    acc<T, RES>(s, d, vx[n]);
-    acc<T, RES>(s, cA, vx[n - NY]);
-    acc<T, RES>(s, cB, vx[n + NY]);
-    acc<T, RES>(s, cSy, vx[n - 1]);
-    acc<T, RES>(s, cNy, vx[n + 1]);
-    acc<T, RES>(s, cFz, vx[n - NXY]);
-    acc<T, RES>(s, cKz, vx[n + NXY]);
-    acc<T, RES>(s, cSx, vy[n - NY]);
-    acc<T, RES>(s, -cNx, vy[n - NY + 1]);
-    acc<T, RES>(s, -cSx, vy[n]);
-    acc<T, RES>(s, cNx, vy[n + 1]);
-    acc<T, RES>(s, cFx, vz[n - NY]);
-    acc<T, RES>(s, -cKx, vz[n - NY + NXY]);
-    acc<T, RES>(s, -cFx, vz[n]);
-    acc<T, RES>(s, cKx, vz[n + NXY]);
-    acc<T, RES>(s, XK, p[n + NXY + 1]);
-    acc<T, RES>(s, -XK, p[n + NXY + NY + 1]);
-    return d;
+    const Row<T> R = xcoef(L, i, j, k, n);
+    xsum<T, RES>(L, R, n, s);
+    return R.d;
 }
-
-// y-momentum row (ystokserr, move3mg.c:910-1101)
 template <typename T, bool RES>
 __device__ __forceinline__ T yrow(const View<T> &L, int i, int j, int k, long n, T &s)
 {
-    using A = Ar<T>;
-    const long NY = L.ny, NXY = L.nxy;
-    const T XK = L.icx[i + 1], YK = A::mul(T(2), L.isy[j]), ZK = L.icz[k + 1];
-    const T cA = cf(YK, L.etac[n + NY + NXY], L.icy[j]);
-    const T cB = cf(YK, L.etac[n + NY + 1 + NXY], L.icy[j + 1]);
-    const T nW = L.etaxy[n], nE = L.etaxy[n + NY], ykW = L.isy[j];
-    const T cWy = cf(XK, nW, ykW), cWx = cf(XK, nW, L.isx[i]);
-    const T cEy = cf(XK, nE, ykW), cEx = cf(XK, nE, L.isx[i + 1]);
-    const T nF = L.etayz[n], nK = L.etayz[n + NXY];
-    const T cFz = cf(ZK, nF, L.isz[k]), cFy = cf(ZK, nF, ykW);
-    const T cKz = cf(ZK, nK, L.isz[k + 1]), cKy = cf(ZK, nK, ykW);
-    T d = -cA;
-    d = A::add(d, -cB); d = A::add(d, -cWx); d = A::add(d, -cEx); d = A::add(d, -cFz); d = A::add(d, -cKz);
-    const T *vx = L.u1, *vy = L.u2, *vz = L.u3, *p = L.u0;
-    acc<T, RES>(s, d, vy[n]);
-    acc<T, RES>(s, cWx, vy[n - NY]);
-    acc<T, RES>(s, cEx, vy[n + NY]);
-    acc<T, RES>(s, cA, vy[n - 1]);
-    acc<T, RES>(s, cB, vy[n + 1]);
-    acc<T, RES>(s, cFz, vy[n - NXY]);
-    acc<T, RES>(s, cKz, vy[n + NXY]);
-    acc<T, RES>(s, cWy, vx[n - 1]);
-    acc<T, RES>(s, -cWy, vx[n]);
-    acc<T, RES>(s, -cEy, vx[n + NY - 1]);
-    acc<T, RES>(s, cEy, vx[n + NY]);
-    acc<T, RES>(s, cFy, vz[n - 1]);
-    acc<T, RES>(s, -cFy, vz[n]);
-    acc<T, RES>(s, -cKy, vz[n - 1 + NXY]);
-    acc<T, RES>(s, cKy, vz[n + NXY]);
-    acc<T, RES>(s, YK, p[n + NY + NXY]);
-    acc<T, RES>(s, -YK, p[n + NY + 1 + NXY]);
-    return d;
+    const Row<T> R = ycoef(L, i, j, k, n);
+    ysum<T, RES>(L, R, n, s);
+    return R.d;
 }
-
-// z-momentum row (zstokserr, move3mg.c:1109-1301)
 template <typename T, bool RES>
 __device__ __forceinline__ T zrow(const View<T> &L, int i, int j, int k, long n, T &s)
 {
-    using A = Ar<T>;
-    const long NY = L.ny, NXY = L.nxy;
-    const T XK = L.icx[i + 1], YK = L.icy[j + 1], ZK = A::mul(T(2), L.isz[k]);
-    const T cA = cf(ZK, L.etac[n + NY + 1], L.icz[k]);
-    const T cB = cf(ZK, L.etac[n + NY + 1 + NXY], L.icz[k + 1]);
-    const T nW = L.etaxz[n], nE = L.etaxz[n + NY], zkW = L.isz[k];
-    const T cWz = cf(XK, nW, zkW), cWx = cf(XK, nW, L.isx[i]);
-    const T cEz = cf(XK, nE, zkW), cEx = cf(XK, nE, L.isx[i + 1]);
-    const T nS = L.etayz[n], nN = L.etayz[n + 1];
-    const T cSz = cf(YK, nS, zkW), cSy = cf(YK, nS, L.isy[j]);
-    const T cNz = cf(YK, nN, zkW), cNy = cf(YK, nN, L.isy[j + 1]);
-    T d = -cA;
-    d = A::add(d, -cB); d = A::add(d, -cWx); d = A::add(d, -cEx); d = A::add(d, -cSy); d = A::add(d, -cNy);
-    const T *vx = L.u1, *vy = L.u2, *vz = L.u3, *p = L.u0;
-    acc<T, RES>(s, d, vz[n]);
-    acc<T, RES>(s, cWx, vz[n - NY]);
-    acc<T, RES>(s, cEx, vz[n + NY]);
-    acc<T, RES>(s, cSy, vz[n - 1]);
-    acc<T, RES>(s, cNy, vz[n + 1]);
-    acc<T, RES>(s, cA, vz[n - NXY]);
-    acc<T, RES>(s, cB, vz[n + NXY]);
-    acc<T, RES>(s, cSz, vy[n - NXY]);
-    acc<T, RES>(s, -cNz, vy[n + 1 - NXY]);
-    acc<T, RES>(s, -cSz, vy[n]);
-    acc<T, RES>(s, cNz, vy[n + 1]);
-    acc<T, RES>(s, cWz, vx[n - NXY]);
-    acc<T, RES>(s, -cWz, vx[n]);
-    acc<T, RES>(s, -cEz, vx[n + NY - NXY]);
-    acc<T, RES>(s, cEz, vx[n + NY]);
-    acc<T, RES>(s, ZK, p[n + NY + 1]);
-    acc<T, RES>(s, -ZK, p[n + NY + 1 + NXY]);
-    return d;
+    const Row<T> R = zcoef(L, i, j, k, n);
+    zsum<T, RES>(L, R, n, s);
+    return R.d;
 }
 
 // continuity row of the cell with upper corner n = (i,j,k) (continerr, move3mg.c:1310-1425)
 template <typename T, bool RES>
-__device__ __forceinline__ void crow(const View<T> &L, int i, int j, int k, long n, T &s)
+__device__ __forceinline__ void csum(const View<T> &L, T xk, T yk, T zk, long n, T &s)
 {
     const long NY = L.ny, NXY = L.nxy;
     const long v0 = n - NXY - NY - 1;
-    const T xk = L.icx[i], yk = L.icy[j], zk = L.icz[k];
     acc<T, RES>(s, -xk, L.u1[v0]);
     acc<T, RES>(s, xk, L.u1[v0 + NY]);
     acc<T, RES>(s, -yk, L.u2[v0]);
     acc<T, RES>(s, yk, L.u2[v0 + 1]);
     acc<T, RES>(s, -zk, L.u3[v0]);
     acc<T, RES>(s, zk, L.u3[v0 + NXY]);
+}
+template <typename T, bool RES>
+__device__ __forceinline__ void crow(const View<T> &L, int i, int j, int k, long n, T &s)
+{
+    csum<T, RES>(L, L.icx[i], L.icy[j], L.icz[k], n, s);
 }
 
 // ------------------------------------------------------------------------------------
@@ -285,16 +352,30 @@ __device__ __forceinline__ long vel_row_node(const View<T> &L, long t, int color
     return (long)k * L.nxy + (long)i * L.ny + j;
 }
 
+template <typename T, int V>
+__device__ __forceinline__ Row<T> vcoef(const View<T> &L, int i, int j, int k, long n)
+{
+    return V == 1 ? xcoef(L, i, j, k, n) : V == 2 ? ycoef(L, i, j, k, n) : zcoef(L, i, j, k, n);
+}
+
+// the value the relaxation gives velocity row n of coefficients R
+template <typename T, int V>
+__device__ __forceinline__ T relaxed(const View<T> &L, const Row<T> &R, long n, T koef)
+{
+    using A = Ar<T>;
+    T s = -(V == 1 ? L.f1[n] : V == 2 ? L.f2[n] : L.f3[n]);
+    if (V == 1) xsum<T, false>(L, R, n, s);
+    if (V == 2) ysum<T, false>(L, R, n, s);
+    if (V == 3) zsum<T, false>(L, R, n, s);
+    return A::sub(V == 1 ? L.u1[n] : V == 2 ? L.u2[n] : L.u3[n], A::mul(A::div(s, R.d), koef));
+}
+
 // the relaxation update of velocity row n; returns the new value
 template <typename T, int V>
 __device__ __forceinline__ T relax_vel_row(const View<T> &L, int i, int j, int k, long n, T koef)
 {
-    using A = Ar<T>;
-    T s, d, u;
-    if (V == 1) { s = -L.f1[n]; d = xrow<T, false>(L, i, j, k, n, s); u = L.u1[n] = A::sub(L.u1[n], A::mul(A::div(s, d), koef)); }
-    if (V == 2) { s = -L.f2[n]; d = yrow<T, false>(L, i, j, k, n, s); u = L.u2[n] = A::sub(L.u2[n], A::mul(A::div(s, d), koef)); }
-    if (V == 3) { s = -L.f3[n]; d = zrow<T, false>(L, i, j, k, n, s); u = L.u3[n] = A::sub(L.u3[n], A::mul(A::div(s, d), koef)); }
-    return u;
+    T *u = V == 1 ? L.u1 : V == 2 ? L.u2 : L.u3;
+    return u[n] = relaxed<T, V>(L, vcoef<T, V>(L, i, j, k, n), n, koef);
 }
 
 template <typename T, int V>
@@ -306,13 +387,36 @@ __device__ __forceinline__ void relax_vel_at(const View<T> &L, long t, int color
     relax_vel_row<T, V>(L, i, j, k, n, koef);
 }
 
-template <typename T, int V>
-__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 6 : 4) k_relax_vel(View<T> L, int color, T koef)
+// PRO (levels of up to kProNodes nodes, where a sweep is bound by the latency of its dependent
+// launches): the row's index, boundary byte, coefficients and boundary entry, which no relaxation
+// writes, are fetched before the kernel waits for its predecessor, and the successor may launch from
+// the start and do the same.  What is left after the wait is one round of loads, the sum and the
+// store.  The kernel before a run of relaxations (a restriction, prolongation or conversion) lets its
+// successor launch only after its own wait, and it writes no operator data, so whatever set the
+// operator up has completed by then.  On B200 a sweep went from 25 to 16 us on levels of 12^3 to 33^3
+// (22 with the packed boundary rows alone) and from 30 to 22 at 65^3; a level of 129^3 takes 108 us, of
+// which latency is a small part, and keeps the plain form with larger blocks.
+constexpr long kProNodes = 400000;
+
+template <typename T, int V, bool PRO>
+__global__ void __launch_bounds__(PRO ? 128 : 256, PRO ? 1 : sizeof(T) == 4 ? 6 : 4) k_relax_vel(View<T> L, int color, T koef)
 {
-    pdl_enter();
-    long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long)((L.ny + 1) >> 1) * L.nx * L.nz) return;
-    relax_vel_at<T, V>(L, t, color, koef);
+    const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (!PRO) {
+        pdl_enter();
+        if (t >= (long)((L.ny + 1) >> 1) * L.nx * L.nz) return;
+        relax_vel_at<T, V>(L, t, color, koef);
+        return;
+    }
+    pdl_trigger();
+    int i, j, k;
+    const long n = t < (long)((L.ny + 1) >> 1) * L.nx * L.nz ? vel_row_node<V>(L, t, color, i, j, k) : -1;
+    const bool row = n >= 0 && !(L.bc[n] & (1 << V));
+    Row<T> R;
+    if (row) R = vcoef<T, V>(L, i, j, k, n);
+    pdl_wait();
+    if (!row) return;
+    (V == 1 ? L.u1 : V == 2 ? L.u2 : L.u3)[n] = relaxed<T, V>(L, R, n, koef);
 }
 
 // All interior pressure rows: p -= (div v - f) * nd * p0koef (move3mg.c:3105-3116)
@@ -373,6 +477,7 @@ struct BcDev {
     int n, na;
     const int *node, *pnode, *depth, *onode, *ocomp, *first, *writer;
     const double *c, *k, *ok;
+    const int4 *inl, *w4, *ext;     // packed homogeneous rows (PACK kernels)
 };
 
 // In-kernel boundary rows (BcList::na >= 0).  A sweep's separate boundary pass writes each
@@ -403,17 +508,75 @@ __device__ __forceinline__ void bc_writer_rows(T *u, const BcDev &B, int e0, lon
     }
 }
 
+// Packed form of the same rows (PACK) for homogeneous systems whose chains multiply to -1, 0 or 1 and
+// whose writers are their partners, as walls make them.  A writer's entries walk four or five
+// dependent loads each (writer, partner, depth, factors), which made the kernels that finish a
+// component 2.6 times as long as the others on the coarse levels (8300 against 3200 cycles at 19^3 on
+// B200).  Here one 16-byte load, issued before the row's own, holds up to three of them: x, y, z the
+// boundary nodes, w bits 0-1 their number, bits 2 + 2 q the factor of node q plus 1, bit 8 set when
+// further entries follow in the list.  inl is indexed by the row (levels up to kBcInline nodes; on
+// larger ones occupancy hides the extra load through first).  Entries [na, n) are {node, partner or -1,
+// factor as a float's bits}.
+__device__ __forceinline__ int4 bc_packed(const BcDev &B, long n)
+{
+    return B.inl ? __ldg(B.inl + n) : __ldg(B.w4 + __ldg(B.first + n));
+}
+template <typename T>
+__device__ __forceinline__ void bc_packed_rows(T *u, const BcDev &B, int4 e, long n, T un)
+{
+    using A = Ar<T>;
+    const int cnt = e.w & 3;
+    auto val = [&](int k) { return k == 1 ? T(0) : A::add(T(0), k == 0 ? -un : un); };
+    if (cnt > 0) u[e.x] = val((e.w >> 2) & 3);
+    if (cnt > 1) u[e.y] = val((e.w >> 4) & 3);
+    if (cnt > 2) u[e.z] = val((e.w >> 6) & 3);
+    if (e.w & 256) bc_writer_rows<T>(u, B, __ldg(B.first + n) + 3, n, un, 0);
+}
+template <typename T>
+__device__ __forceinline__ void bc_packed_extra(T *u, int4 e)
+{
+    u[e.x] = Ar<T>::add(T(0), Ar<T>::mul((T)__int_as_float(e.z), e.y >= 0 ? u[e.y] : T(0)));
+}
+
 // Colour 1 of velocity component V with the component's boundary rows; blocks from rowblocks on
 // write entries [na, n).
-template <typename T, int V>
-__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 6 : 4) k_relax_vel_bc(View<T> L, T koef, BcDev B, int use_c,
-                                                                               unsigned rowblocks)
+template <typename T, int V, bool PACK, bool PRO>
+__global__ void __launch_bounds__(PRO ? 128 : 256, PRO ? 1 : sizeof(T) == 4 ? 6 : 4) k_relax_vel_bc(View<T> L, T koef, BcDev B, int use_c,
+                                                                                                   unsigned rowblocks)
 {
-    pdl_enter();
     T *u = V == 1 ? L.u1 : V == 2 ? L.u2 : L.u3;
+    if (PRO) {
+        static_assert(!PRO || PACK, "the prologue takes packed boundary rows");
+        pdl_trigger();
+        if (blockIdx.x >= rowblocks) {
+            const int t = (int)(blockIdx.x - rowblocks) * (int)blockDim.x + (int)threadIdx.x;
+            const int4 e = t < B.n - B.na ? __ldg(B.ext + t) : make_int4(-1, -1, 0, 0);
+            pdl_wait();
+            if (e.x >= 0) bc_packed_extra<T>(u, e);
+            return;
+        }
+        const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
+        int i, j, k;
+        const long n = t < (long)((L.ny + 1) >> 1) * L.nx * L.nz ? vel_row_node<V>(L, t, 1, i, j, k) : -1;
+        const uint8_t b = n >= 0 ? L.bc[n] : 0;
+        const bool row = n >= 0 && !(b & (1 << V));
+        Row<T> R;
+        int4 e = make_int4(0, 0, 0, 0);
+        if (row) {
+            if (b & (16 << V)) e = bc_packed(B, n);
+            R = vcoef<T, V>(L, i, j, k, n);
+        }
+        pdl_wait();
+        if (!row) return;
+        const T un = u[n] = relaxed<T, V>(L, R, n, koef);
+        if (e.w) bc_packed_rows<T>(u, B, e, n, un);
+        return;
+    }
+    pdl_enter();
     if (blockIdx.x >= rowblocks) {
-        const int e = B.na + (int)(blockIdx.x - rowblocks) * (int)blockDim.x + (int)threadIdx.x;
-        if (e < B.n) bc_apply_at<T>(u, e, B.node, B.pnode, B.depth, B.c, B.k, use_c);
+        const int e = (int)(blockIdx.x - rowblocks) * (int)blockDim.x + (int)threadIdx.x;
+        if (PACK) { if (e < B.n - B.na) bc_packed_extra<T>(u, __ldg(B.ext + e)); }
+        else if (B.na + e < B.n) bc_apply_at<T>(u, B.na + e, B.node, B.pnode, B.depth, B.c, B.k, use_c);
         return;
     }
     const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -423,24 +586,68 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 6 : 4) k_relax_vel_bc(Vi
     if (n < 0) return;
     const uint8_t b = L.bc[n];
     if (b & (1 << V)) return;
+    if (PACK) {
+        const int4 e = (b & (16 << V)) ? bc_packed(B, n) : make_int4(0, 0, 0, 0);
+        const T un = relax_vel_row<T, V>(L, i, j, k, n, koef);
+        if (e.w) bc_packed_rows<T>(u, B, e, n, un);
+        return;
+    }
     const int e0 = (b & (16 << V)) ? __ldg(B.first + n) : B.na;
     const T un = relax_vel_row<T, V>(L, i, j, k, n, koef);
     if (e0 < B.na) bc_writer_rows<T>(u, B, e0, n, un, use_c);
 }
 
 // All pressure rows with the pressure boundary rows (no pressure row reads another pressure).
-template <typename T>
+template <typename T, bool PACK, bool PRO>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 6 : 4) k_relax_p_bc(View<T> L, T koef, BcDev B, int use_c,
                                                                              unsigned rowblocks)
 {
+    if (PRO) {
+        using A = Ar<T>;
+        pdl_trigger();
+        if (blockIdx.x >= rowblocks) {
+            const int t = (int)(blockIdx.x - rowblocks) * (int)blockDim.x + (int)threadIdx.x;
+            const int4 e = t < B.n - B.na ? __ldg(B.ext + t) : make_int4(-1, -1, 0, 0);
+            pdl_wait();
+            if (e.x >= 0) bc_packed_extra<T>(L.u0, e);
+            return;
+        }
+        const long n = (long)blockIdx.x * blockDim.x + threadIdx.x;
+        int i = 0, j = 0, k = 0;
+        bool row = n < L.nxy * L.nz;
+        if (row) node_ijk(L, n, i, j, k);
+        const uint8_t b = row ? L.bc[n] : 0;
+        row = row && i > 0 && j > 0 && k > 0 && !(b & 1);
+        int4 e = make_int4(0, 0, 0, 0);
+        T xk = 0, yk = 0, zk = 0, nd = 0;
+        if (row) {
+            if (b & 16) e = bc_packed(B, n);
+            xk = L.icx[i]; yk = L.icy[j]; zk = L.icz[k];
+            nd = (T)L.nd[n];
+        }
+        pdl_wait();
+        if (!row) return;
+        T s = -L.f0[n];
+        csum<T, false>(L, xk, yk, zk, n, s);
+        const T un = L.u0[n] = A::sub(L.u0[n], A::mul(A::mul(s, nd), koef));
+        if (e.w) bc_packed_rows<T>(L.u0, B, e, n, un);
+        return;
+    }
     pdl_enter();
     if (blockIdx.x >= rowblocks) {
-        const int e = B.na + (int)(blockIdx.x - rowblocks) * (int)blockDim.x + (int)threadIdx.x;
-        if (e < B.n) bc_apply_at<T>(L.u0, e, B.node, B.pnode, B.depth, B.c, B.k, use_c);
+        const int e = (int)(blockIdx.x - rowblocks) * (int)blockDim.x + (int)threadIdx.x;
+        if (PACK) { if (e < B.n - B.na) bc_packed_extra<T>(L.u0, __ldg(B.ext + e)); }
+        else if (B.na + e < B.n) bc_apply_at<T>(L.u0, B.na + e, B.node, B.pnode, B.depth, B.c, B.k, use_c);
         return;
     }
     const long n = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (n >= L.nxy * L.nz) return;
+    if (PACK) {
+        const int4 e = (L.bc[n] & 16) ? bc_packed(B, n) : make_int4(0, 0, 0, 0);
+        T un = 0;
+        if (relax_p_at<T>(L, n, koef, nullptr, &un) && e.w) bc_packed_rows<T>(L.u0, B, e, n, un);
+        return;
+    }
     const int e0 = (L.bc[n] & 16) ? __ldg(B.first + n) : B.na;
     uint8_t b = 0;
     T un = 0;
@@ -1383,6 +1590,57 @@ static int upload_f32_scaled(i3g_ctx *c, float *&dst, const std::vector<double> 
     return upload(c, dst, f);
 }
 
+// The packed form of one component's boundary rows (bc_packed); left out where a chain's factors do
+// not multiply to -1, 0 or 1 or a writer is not the partner.
+constexpr long kBcInline = 400000;
+__global__ void k_bc_inline(int4 *inl, const int4 *w4, const int *writer, int na)
+{
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e < na && w4[e].w) inl[writer[e]] = w4[e];   // a writer's first entry holds its rows
+}
+static int pack_bc(i3g_ctx *c, const Level &L, BcList &B, int na, const std::vector<int> &node, const std::vector<int> &pnode,
+                   const std::vector<int> &depth, const std::vector<double> &kk, const std::vector<int> &writer, const std::vector<int> &first)
+{
+    const int n = (int)node.size();
+    auto factor = [&](int e) {
+        double K = pnode[e] >= 0 ? 1.0 : 0.0;
+        for (int d = 0; d < depth[e]; d++) {
+            const double k = kk[(size_t)e * kMaxBcDepth + d];
+            if (k != 0.0 && k != 1.0 && k != -1.0) return 2.0;
+            K *= k;
+        }
+        return K;
+    };
+    std::vector<int4> w4(na, make_int4(0, 0, 0, 0)), ext;
+    for (int e = 0; e < na; e++) {
+        const double K = factor(e);
+        if (K == 2.0 || (pnode[e] != writer[e] && K != 0.0)) return 0;
+        const int f = first[writer[e]], q = e - f;
+        int4 &x = w4[f];
+        if (q >= 3) { x.w |= 256; continue; }
+        (q == 0 ? x.x : q == 1 ? x.y : x.z) = node[e];
+        x.w = (x.w & ~3) | (q + 1) | ((int)K + 1) << (2 + 2 * q);
+    }
+    for (int e = na; e < n; e++) {
+        const double K = factor(e);
+        if (K == 2.0) return 0;
+        const float k = (float)K;
+        int bits;
+        memcpy(&bits, &k, sizeof bits);
+        ext.push_back(make_int4(node[e], pnode[e], bits, 0));
+    }
+    int rc;
+    if ((rc = upload(c, B.w4, w4)) || (rc = upload(c, B.ext, ext))) return rc;
+    if (L.n <= kBcInline && na > 0) {
+        ALLOC(B.inl, int4, L.n);
+        I3G_CUDA(cudaMemsetAsync(B.inl, 0, sizeof(int4) * L.n, c->st));
+        k_bc_inline<<<nblk(na), 256, 0, c->st>>>(B.inl, B.w4, B.writer, na);
+        c->launches++;
+    }
+    B.packed = true;
+    return 0;
+}
+
 // Boundary rows: flatten chains to an interior partner; reject cycles, partners that are
 // not rows of the system and interior rows whose stencil leaves the grid.
 static int build_bc(i3g_ctx *c)
@@ -1551,6 +1809,7 @@ static int build_bc(i3g_ctx *c)
                 (rc = upload(c, B.onode, onode[v])) || (rc = upload(c, B.ocomp, ocomp[v])) ||
                 (rc = upload(c, B.oc, oc[v])) || (rc = upload(c, B.ok, ok[v])))
                 return rc;
+            if (na[v] >= 0 && (rc = pack_bc(c, L, B, na[v], node[v], pnode[v], depth[v], kk[v], writer[v], first[v]))) return rc;
         }
     }
     return 0;
@@ -1568,6 +1827,8 @@ int stokes_alloc(i3g_ctx *c)
     // I3G_FUSE: 0 one launch per boundary pass, residual part and transfer component; 1 boundary
     // rows in-kernel on levels >= 1 (default); 3 on level 0 too
     if (const char *e = getenv("I3G_FUSE")) c->fuse = atoi(e);
+    c->pro_nodes = kProNodes;
+    if (const char *e = getenv("I3G_PRO_NODES")) c->pro_nodes = atol(e);
     if (const char *e = getenv("I3G_ND_SCHUR")) c->nd_schur = std::max(0, atoi(e));
     if (c->tail_cluster > 8) {
         I3G_CUDA(cudaFuncSetAttribute(k_vcycle_cluster<float>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
@@ -1685,6 +1946,7 @@ void stokes_free(i3g_ctx *c)
             BcList &B = L.bcl[v];
             cudaFree(B.node); cudaFree(B.pnode); cudaFree(B.depth); cudaFree(B.c); cudaFree(B.k);
             cudaFree(B.onode); cudaFree(B.ocomp); cudaFree(B.oc); cudaFree(B.ok); cudaFree(B.first); cudaFree(B.writer);
+            cudaFree(B.inl); cudaFree(B.w4); cudaFree(B.ext);
         }
         cudaFree(L.d.etac); cudaFree(L.d.etaxy); cudaFree(L.d.etaxz); cudaFree(L.d.etayz); cudaFree(L.d.nd);
         cudaFree(L.s.etac); cudaFree(L.s.etaxy); cudaFree(L.s.etaxz); cudaFree(L.s.etayz); cudaFree(L.s.nd);
@@ -1774,7 +2036,8 @@ static void bc_apply(i3g_ctx *c, int l, int v, bool use_c)
 
 static BcDev bcdev(const BcList &B)
 {
-    return BcDev{B.n, B.na, B.node, B.pnode, B.depth, B.onode, B.ocomp, B.first, B.writer, B.c, B.k, B.ok};
+    return BcDev{B.n, B.na, B.node, B.pnode, B.depth, B.onode, B.ocomp, B.first, B.writer, B.c, B.k, B.ok,
+                 B.inl, B.w4, B.ext};
 }
 
 template <typename T>
@@ -1807,36 +2070,52 @@ static void smooth_t(i3g_ctx *c, int l, int nsweeps, bool homogeneous, bool with
     const long total = (long)((L.ny + 1) / 2) * L.nx * L.nz;
     const T v0 = (T)c->p.v0koef, p0 = (T)c->p.p0koef;
     const bool use_c = l == 0 && !homogeneous;
-    const unsigned rows = nblk(total), prows = nblk(L.n);
+    const unsigned rows = nblk(total), rows128 = nblk(total, 128), prows = nblk(L.n);
     // in-kernel boundary rows: coarse levels always (latency-bound launches), level 0 with
-    // I3G_FUSE=3 (its launches are bandwidth-bound and the writers' loads lengthen them)
-    const bool inkernel = c->fuse && (l > 0 || c->fuse >= 3);
+    // I3G_FUSE=3 (its launches are bandwidth-bound and the writers' loads lengthen them), or where it
+    // is small enough for the prologue
+    const bool packed = c->fuse && !use_c && L.bcl[0].packed && L.bcl[1].packed && L.bcl[2].packed && L.bcl[3].packed;
+    const bool pro = packed && L.n <= c->pro_nodes, inkernel = c->fuse && (l > 0 || c->fuse >= 3 || pro);
+#define FIRST_COLOUR(V_)                                                                                \
+    do {                                                                                                \
+        if (pro) LAUNCH((k_relax_vel<T, V_, true>), rows128, 128, V, 0, v0);                            \
+        else LAUNCH((k_relax_vel<T, V_, false>), rows, 256, V, 0, v0);                                  \
+    } while (0)
     // colour 1 of a component, with its boundary rows when set-up admitted them in-kernel
 #define LAST_COLOUR(V_)                                                                                 \
     do {                                                                                                \
         const BcList &B = L.bcl[V_];                                                                    \
-        if (inkernel && B.na >= 0)                                                                      \
-            LAUNCH((k_relax_vel_bc<T, V_>), rows + nblk(B.n - B.na), 256, V, v0, bcdev(B), (int)use_c, rows); \
+        if (pro)                                                                                        \
+            LAUNCH((k_relax_vel_bc<T, V_, true, true>), rows128 + nblk(B.n - B.na, 128), 128, V, v0, bcdev(B), 0, rows128); \
+        else if (inkernel && packed)                                                                    \
+            LAUNCH((k_relax_vel_bc<T, V_, true, false>), rows + nblk(B.n - B.na), 256, V, v0, bcdev(B), 0, rows); \
+        else if (inkernel && B.na >= 0)                                                                 \
+            LAUNCH((k_relax_vel_bc<T, V_, false, false>), rows + nblk(B.n - B.na), 256, V, v0, bcdev(B), (int)use_c, rows); \
         else {                                                                                          \
-            LAUNCH((k_relax_vel<T, V_>), rows, 256, V, 1, v0);                                          \
+            LAUNCH((k_relax_vel<T, V_, false>), rows, 256, V, 1, v0);                                   \
             bc_apply<T>(c, l, V_, use_c);                                                               \
         }                                                                                               \
     } while (0)
     for (int s = 0; s < nsweeps; s++) {
-        LAUNCH((k_relax_vel<T, 1>), rows, 256, V, 0, v0);
+        FIRST_COLOUR(1);
         LAST_COLOUR(1);
-        LAUNCH((k_relax_vel<T, 2>), rows, 256, V, 0, v0);
+        FIRST_COLOUR(2);
         LAST_COLOUR(2);
-        LAUNCH((k_relax_vel<T, 3>), rows, 256, V, 0, v0);
+        FIRST_COLOUR(3);
         LAST_COLOUR(3);
         const BcList &B = L.bcl[0];
-        if (inkernel && B.na >= 0)
-            LAUNCH(k_relax_p_bc<T>, prows + nblk(B.n - B.na), 256, V, p0, bcdev(B), (int)use_c, prows);
+        if (pro)
+            LAUNCH((k_relax_p_bc<T, true, true>), prows + nblk(B.n - B.na), 256, V, p0, bcdev(B), 0, prows);
+        else if (inkernel && packed)
+            LAUNCH((k_relax_p_bc<T, true, false>), prows + nblk(B.n - B.na), 256, V, p0, bcdev(B), 0, prows);
+        else if (inkernel && B.na >= 0)
+            LAUNCH((k_relax_p_bc<T, false, false>), prows + nblk(B.n - B.na), 256, V, p0, bcdev(B), (int)use_c, prows);
         else {
             LAUNCH(k_relax_p<T>, prows, 256, V, p0);
             bc_apply<T>(c, l, 0, use_c);
         }
     }
+#undef FIRST_COLOUR
 #undef LAST_COLOUR
     if (with_residual) residual_t<T>(c, l);
 }
@@ -3009,8 +3288,8 @@ int stokes_time_kernel(i3g_ctx *c, int kind, int reps, double *ms, double *bytes
     int r = 0;
     auto launch = [&]() -> int {
         switch (kind) {
-        case 0: LAUNCH((k_relax_vel<double, 1>), nblk(total), 256, V, r & 1, c->p.v0koef); break;
-        case 7: LAUNCH((k_relax_vel<float, 1>), nblk(total), 256, Vf, r & 1, (float)c->p.v0koef); break;
+        case 0: LAUNCH((k_relax_vel<double, 1, false>), nblk(total), 256, V, r & 1, c->p.v0koef); break;
+        case 7: LAUNCH((k_relax_vel<float, 1, false>), nblk(total), 256, Vf, r & 1, (float)c->p.v0koef); break;
         case 8: smooth_t<float>(c, 0, 1, true, false); break;
         case 10: smooth_t<double>(c, 0, 1, false, false); break;
         case 1: LAUNCH(k_residual<double>, nblk(L.n), 256, V); break;
