@@ -33,7 +33,7 @@ constexpr int NBOX = NBX * NBY * NBZ;
 enum { A_NU, W_NU, A_XX, W_XX, A_XY, W_XY, A_XZ, W_XZ, A_YZ, W_YZ, A_RO, A_CP, A_KT, A_HT, A_ET, A_TK, A_RR, W_P, NACC };
 enum { R_N0, R_N1, R_S0, R_S1, R_NU, R_DH, R_DV, R_SS, R_MM, R_LL, R_A0, R_A1, R_B0, R_B1, R_E0, R_E1,
        R_RO, R_BB, R_AA, R_CP, R_KT, R_KF, R_KP, R_HT };
-enum { ERR_TYPE = 1, ERR_GRAIN = 2, ERR_WATER = 4, ERR_MELT = 8, ERR_DENSI = 16 };
+enum { ERR_TYPE = 1, ERR_GRAIN = 2, ERR_WATER = 4, ERR_MELT = 8, ERR_DENSI = 16, ERR_REDO = 32 };
 
 struct Marks {
     float *x, *y, *z, *k, *w, *d, *v, *e, *ex, *ft, *rr, *rn;
@@ -1090,6 +1090,181 @@ __global__ void __launch_bounds__(32 * kR2nWarps) k_r2n_cells(Marks M, const int
     (void)cx0; (void)cy0; (void)cz0;
 }
 
+// The same sums for the ordinary call, a time step whose markers all have a viscosity and finite
+// properties.  Stage 2 as matrix products: a step multiplies the staged properties
+// [8 quantities x 4 markers] with the weights [4 markers x 8 targets] (mma.m8n8k4, FP64 products and
+// sums), four times:
+//   tile 1  ro, cp ro, kt, ht, alpha, T, rr, 1       x  trilinear weight of the 8 nodes
+//   tile 2  viscosity, 1                             x  the same where the nukoef gate is open
+//   tile 3  viscosity, 1                             x  tents of the 4 xy and 4 xz stress points
+//   tile 4  viscosity, 1                             x  tents of the 4 yz points and the cell centre
+// so the sums over markers need no shuffles and a lane keeps 8 sums instead of 18; without the
+// viscosity of new markers the kernel fits 64 registers, twice the warps of k_r2n_cells.  A marker
+// without a viscosity, or with a value that is not finite (0 x inf is NaN in a matrix product, while
+// k_r2n_cells skips the zero weight), raises ERR_REDO: the caller then repeats the pass with
+// k_r2n_cells, which leaves what it would have left alone.  Bound by FP64 issue and latency; 5.3 ms
+// against 7.0 for k_r2n_cells at 129^3 nodes with 56.6 M markers (B200, default arithmetic).
+// Staged doubles per marker: weights (3, or the reference's 6), viscosity, 7 quantities, 1.  A stride
+// of 12 keeps the operand reads (4 markers x 4 quantities per half warp) free of bank conflicts.
+template <bool EX>
+constexpr int kMmaStage = EX ? 15 : 12;
+
+__device__ __forceinline__ void dmma(double (&d)[2], double a, double b)
+{
+    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};" : "+d"(d[0]), "+d"(d[1]) : "d"(a), "d"(b));
+}
+
+__device__ __forceinline__ double half_over(double w) { return w > 0.5 ? w - 0.5 : 0.0; }
+__device__ __forceinline__ double tent(double w) { return 0.5 - fabs(w - 0.5); }
+
+// per-axis weight of node side s (0, 1) of a staged marker
+template <bool EX>
+__device__ __forceinline__ double side(const double *st, int axis, int s)
+{
+    if (EX) return st[2 * axis + s];
+    const double w = st[axis];
+    return s ? w : 1.0 - w;
+}
+
+template <bool EX, int W>
+__global__ void __launch_bounds__(32 * W) k_r2n_mma(const __grid_constant__ Marks M, const int *coff, const __grid_constant__ Grid Gg,
+                                                      const __grid_constant__ NodeF F, const __grid_constant__ Phys P, TileGeo T,
+                                                      double *stage)
+{
+    constexpr int K = kMmaStage<EX>, P0 = EX ? 6 : 3;
+    extern __shared__ double sm[];
+    double *sacc = sm;                                   // [NACC][NBOX]
+    double *stg = sm + NACC * NBOX;                      // [W][32][K]
+    double *shg = stg + W * 32 * K;                      // grid lines (and the fast tables)
+    for (int q = threadIdx.x; q < NACC * NBOX; q += blockDim.x) sacc[q] = 0;
+    Grid G;
+    load_grid<EX>(Gg, shg, G);   // contains __syncthreads
+    const int tile = blockIdx.x;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    double *my = stg + warp * 32 * K;
+    // operand coordinates: row (quantity) or column (target) g, marker m of the four
+    const int g = lane >> 2, mk4 = lane & 3;
+    const int iz = g >> 2, ix = (g >> 1) & 1, iy = g & 1;
+    const int hi = (g >> 1) & 1, lo = g & 1;             // node sides of stress point g & 3
+    const int vm = P.viscmod;
+    const double nk = P.nukoef;
+    for (int colour = 0; colour < 8; colour++) {
+        const int pz = colour >> 2, px = (colour >> 1) & 1, py = colour & 1;
+        for (int q = warp; q < CPT / 8; q += W) {
+            const int ly = 2 * (q % (TY / 2)) + py, r2 = q / (TY / 2);
+            const int lx = 2 * (r2 % (TX / 2)) + px, lz = 2 * (r2 / (TX / 2)) + pz;
+            const long cell = (long)tile * CPT + (lz * TX + lx) * TY + ly;
+            const int beg = coff[cell], end = coff[cell + 1];
+            if (beg == end) continue;   // uniform over the warp
+            double *acc0 = sacc + (lz * NBX + lx) * NBY + ly;
+            double d1[2] = {0, 0}, d2[2] = {0, 0}, d3[2] = {0, 0}, d4[2] = {0, 0};
+            for (int base = beg; base < end; base += 32) {
+                // stage 1: one marker per lane
+                bool ok = false, finite = true;
+                double *st = my + lane * K;
+                if (base + lane < end) {
+                    const int i = base + lane;
+                    int mm2 = M.t[i];
+                    const float fx = M.x[i], fy = M.y[i], fz = M.z[i];
+                    ok = M.k[i] > 0;
+                    if (ok && mm2 > 1 && fy < P.eroslev) { mm2 = 0; M.t[i] = 0; }
+                    if (ok && mm2 < 2) { atomicOr(P.err, ERR_WATER); ok = false; }
+                    if (ok && mm2 > 20) { atomicOr(P.err, ERR_MELT); ok = false; }
+                    if (ok && P.densimod >= 2) { atomicOr(P.err, ERR_DENSI); ok = false; }
+                    if (ok) {
+                        int wn[3];
+                        const double mpb = pr_at<EX>(G, F.pr, F.NY, F.NXY, fx, fy, fz, wn) * 1e-5;
+                        const double mtk = M.k[i];
+                        double mnu = M.v[i];
+                        if (mnu <= 0) finite = ok = false;
+                        if (ok) {
+                            double mbb = 0, mro = RK(P, R_RO, mm2);
+                            if (P.densimod != 0) {   // dencalc1 (mark3mg.c:3006-3024)
+                                const double bb = RK(P, R_BB, mm2);
+                                mbb = bb / (1.0 - bb * (mtk - 298.15));
+                                mro = mro * (1.0 - bb * (mtk - 298.15)) * (1.0 + RK(P, R_AA, mm2) * (mpb - 1.0) * 1e-3);
+                            }
+                            phase_density(P, mm2, mtk, mpb, mro);
+                            const double mcp = RK(P, R_CP, mm2);
+                            const double kp = RK(P, R_KP, mm2);   // exp(0) = 1 exactly: skip it
+                            const double mkt = (RK(P, R_KT, mm2) + RK(P, R_KF, mm2) / (mtk + 77.0)) * (kp != 0 ? exp(kp * mpb) : 1.0);
+                            if (fy > P.vdeep && mnu > P.nudeep) mnu = P.nudeep;
+                            if (fy < 5e+4 && fx > G.xsize - 1e+4 && fz > 1.5e+5 && fz < 8.7e+5 && mnu > 1e+19) mnu = 1e+19;
+                            const int m10 = wn[0], m20 = wn[1], m30 = wn[2];
+                            if (EX) {
+                                const double dx = G.gx[m10 + 1] - G.gx[m10], dy = G.gy[m20 + 1] - G.gy[m20], dz = G.gz[m30 + 1] - G.gz[m30];
+                                st[0] = 1.0 - fabs((G.gx[m10] - fx) / dx);
+                                st[1] = 1.0 - fabs((G.gx[m10 + 1] - fx) / dx);
+                                st[2] = 1.0 - fabs((G.gy[m20] - fy) / dy);
+                                st[3] = 1.0 - fabs((G.gy[m20 + 1] - fy) / dy);
+                                st[4] = 1.0 - fabs((G.gz[m30] - fz) / dz);
+                                st[5] = 1.0 - fabs((G.gz[m30 + 1] - fz) / dz);
+                            } else {
+                                // weight of the cell's upper node; the lower node's is 1 - it
+                                st[0] = (fx - G.gx[m10]) * G.rl[0][m10];
+                                st[1] = (fy - G.gy[m20]) * G.rl[1][m20];
+                                st[2] = (fz - G.gz[m30]) * G.rl[2][m30];
+                            }
+                            const double val[8] = {vm == 0 ? mnu : vm == 1 ? log(mnu) : 1.0 / mnu, mro, mcp * mro, mkt, RK(P, R_HT, mm2), mbb,
+                                                   mtk, (double)M.rr[i]};
+#pragma unroll
+                            for (int v = 0; v < 8; v++) {
+                                st[P0 + v] = val[v];
+                                finite = finite && fabs(val[v]) <= 1.7976931348623157e308;
+                            }
+                            st[P0 + 8] = 1.0;
+                        }
+                    }
+                }
+                if (!ok) {
+#pragma unroll
+                    for (int v = 0; v < K; v++) st[v] = 0.0;
+                }
+                if (!finite) atomicOr(P.err, ERR_REDO);
+                __syncwarp();
+                const int cnt = min(32, end - base);
+                // stage 2: four markers per step (the lanes past cnt staged zeros)
+                for (int m0 = 0; m0 < cnt; m0 += 4) {
+                    const double *sm4 = my + (m0 + mk4) * K;
+                    const double x = side<EX>(sm4, 0, ix), y = side<EX>(sm4, 1, iy), z = side<EX>(sm4, 2, iz);
+                    const double swt = x * y * z;
+                    const double vn = sm4[P0], one = sm4[P0 + 8];
+                    const double av = g == 0 ? vn : g == 1 ? one : 0.0;
+                    dmma(d1, sm4[P0 + 1 + g], swt);
+                    dmma(d2, av, x > nk && y > nk && z > nk ? swt : 0.0);
+                    // stress points: columns 0-3 xy (x side hi, y side lo) and yz (y side hi, z side lo),
+                    // 4-7 xz (x side hi, z side lo), 4 of tile 4 the cell centre
+                    const double xh = half_over(side<EX>(sm4, 0, hi)), xt = tent(side<EX>(sm4, 0, 1)), yt = tent(side<EX>(sm4, 1, 1)),
+                                 zt = tent(side<EX>(sm4, 2, 1)), zl = half_over(side<EX>(sm4, 2, lo));
+                    const double yl = half_over(side<EX>(sm4, 1, lo)), yh = half_over(side<EX>(sm4, 1, hi));
+                    dmma(d3, av, g < 4 ? xh * yl * zt : xh * yt * zl);
+                    dmma(d4, av, g < 4 ? xt * yh * zl : g == 4 ? xt * yt * zt : 0.0);
+                }
+                __syncwarp();
+            }
+            // a lane's sums: quantity g of targets c, c + 1
+            const int c = 2 * mk4;
+#pragma unroll
+            for (int u = 0; u < 2; u++) {
+                const int t = c + u, tz = t >> 2, tx = (t >> 1) & 1, ty = t & 1;
+                acc0[(A_RO + g) * NBOX + (tz * NBX + tx) * NBY + ty] += d1[u];
+                if (g < 2) {
+                    acc0[(A_NU + g) * NBOX + (tz * NBX + tx) * NBY + ty] += d2[u];
+                    if (t < 4) acc0[(A_XY + g) * NBOX + tx * NBY + ty] += 8.0 * d3[u];
+                    else acc0[(A_XZ + g) * NBOX + (ty * NBX + tx) * NBY] += 8.0 * d3[u];
+                    if (t < 4) acc0[(A_YZ + g) * NBOX + ty * NBX * NBY + tx] += 8.0 * d4[u];
+                    else if (t == 4) acc0[(A_XX + g) * NBOX + (NBX + 1) * NBY + 1] += 8.0 * d4[u];
+                }
+            }
+        }
+        __syncthreads();
+    }
+    // the whole node box of the tile to its staging slot; k_r2n_gather adds the boxes that share
+    // a node in a fixed order (no atomics, the same sums on every run)
+    double *dst = stage + (long)tile * NACC * NBOX;
+    for (int q = threadIdx.x; q < NACC * NBOX; q += blockDim.x) dst[q] = sacc[q];
+}
+
 // tiles whose node box holds node coordinate v along one axis (t * T <= v <= t * T + T)
 __device__ __forceinline__ void box_range(int v, int TT, int nt, int &t0, int &t1)
 {
@@ -1547,20 +1722,39 @@ static int move_occupancy(i3g_ctx *c, int *per_sm)
     return 0;
 }
 
-static void launch_r2n(i3g_ctx *c, const Marks &M, const int *coff, const TileGeo &T, double timestep, double *stage);
+static void launch_r2n(i3g_ctx *c, const Marks &M, const int *coff, const TileGeo &T, double timestep, double *stage, bool redo = false);
 static void launch_heat_mark(i3g_ctx *c, const Marks &M, const int *coff, const TkF &TK, const TileGeo &T, double timestep,
                              double *stage);
 static size_t r2n_smem(i3g_ctx *c) { return sizeof(double) * (NACC * NBOX + kR2nWarps * 32 * kStage) + grid_smem(c) + sizeof(int) * kR2nWarps * 32; }
+template <bool EX>
+static size_t r2n_mma_smem(i3g_ctx *c, int warps) { return sizeof(double) * (NACC * NBOX + warps * 32 * kMmaStage<EX>) + grid_smem(c); }
+
+// Warps per CTA of k_r2n_mma (one CTA per SM: the node sums take 119 KB): as many as the staging areas
+// leave room for, 32 while nx + ny + nz <= 479 (grid tables of 15 KB), 24 up to 1247, else 16; 16 in
+// the reference's operation order, whose staging is larger and whose stage 1 needs more registers.
+static int r2n_warps(i3g_ctx *c)
+{
+    if (mexact(c)) return 16;
+    return r2n_mma_smem<false>(c, 32) <= 227 * 1024 ? 32 : r2n_mma_smem<false>(c, 24) <= 227 * 1024 ? 24 : 16;
+}
+
 static size_t heat_mark_smem(i3g_ctx *c) { return sizeof(double) * (2 * NBOX + kR2nWarps * 32 * kHmStage) + grid_smem(c); }
 
-static void launch_r2n(i3g_ctx *c, const Marks &M, const int *coff, const TileGeo &T, double timestep, double *stage)
+// redo: the pass repeated because a marker raised ERR_REDO
+static void launch_r2n(i3g_ctx *c, const Marks &M, const int *coff, const TileGeo &T, double timestep, double *stage, bool redo)
 {
-    if (mexact(c))
-        LAUNCH(k_r2n_cells<true>, ms(c)->ntiles, 32 * kR2nWarps, r2n_smem(c), M, coff, grid_of(c), nodes_of(c), phys_of(c), T,
-               timestep, stage);
-    else
-        LAUNCH(k_r2n_cells<false>, ms(c)->ntiles, 32 * kR2nWarps, r2n_smem(c), M, coff, grid_of(c), nodes_of(c), phys_of(c), T,
-               timestep, stage);
+    const int w = r2n_warps(c), nt = ms(c)->ntiles;
+    const Grid G = grid_of(c);
+    const NodeF F = nodes_of(c);
+    const Phys P = phys_of(c);
+    if (timestep <= 0 || redo) {   // markers without a viscosity
+        if (mexact(c)) LAUNCH(k_r2n_cells<true>, nt, 32 * kR2nWarps, r2n_smem(c), M, coff, G, F, P, T, timestep, stage);
+        else LAUNCH(k_r2n_cells<false>, nt, 32 * kR2nWarps, r2n_smem(c), M, coff, G, F, P, T, timestep, stage);
+    }
+    else if (mexact(c)) LAUNCH((k_r2n_mma<true, 16>), nt, 32 * 16, r2n_mma_smem<true>(c, 16), M, coff, G, F, P, T, stage);
+    else if (w == 32) LAUNCH((k_r2n_mma<false, 32>), nt, 32 * 32, r2n_mma_smem<false>(c, 32), M, coff, G, F, P, T, stage);
+    else if (w == 24) LAUNCH((k_r2n_mma<false, 24>), nt, 32 * 24, r2n_mma_smem<false>(c, 24), M, coff, G, F, P, T, stage);
+    else LAUNCH((k_r2n_mma<false, 16>), nt, 32 * 16, r2n_mma_smem<false>(c, 16), M, coff, G, F, P, T, stage);
 }
 
 static void launch_heat_mark(i3g_ctx *c, const Marks &M, const int *coff, const TkF &TK, const TileGeo &T, double timestep,
@@ -1649,6 +1843,12 @@ int markers_alloc(i3g_ctx *c)
     }
     I3G_CUDA(cudaFuncSetAttribute(k_r2n_cells<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)r2n_smem(c)));
     I3G_CUDA(cudaFuncSetAttribute(k_r2n_cells<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)r2n_smem(c)));
+    I3G_CUDA(cudaFuncSetAttribute((k_r2n_mma<true, 16>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)r2n_mma_smem<true>(c, 16)));
+    I3G_CUDA(cudaFuncSetAttribute((k_r2n_mma<false, 16>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)r2n_mma_smem<false>(c, 16)));
+    if (r2n_mma_smem<false>(c, 24) <= 227 * 1024)
+        I3G_CUDA(cudaFuncSetAttribute((k_r2n_mma<false, 24>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)r2n_mma_smem<false>(c, 24)));
+    if (r2n_mma_smem<false>(c, 32) <= 227 * 1024)
+        I3G_CUDA(cudaFuncSetAttribute((k_r2n_mma<false, 32>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)r2n_mma_smem<false>(c, 32)));
     I3G_CUDA(cudaFuncSetAttribute((k_heat_mark_cells<true, 1>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)heat_mark_smem(c)));
     I3G_CUDA(cudaFuncSetAttribute((k_heat_mark_cells<true, 2>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)heat_mark_smem(c)));
     I3G_CUDA(cudaFuncSetAttribute((k_heat_mark_cells<false, 1>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)heat_mark_smem(c)));
@@ -1760,7 +1960,7 @@ static int check_err(i3g_ctx *c, const char *what)
     MarkerState *S = ms(c);
     I3G_CUDA(cudaMemcpyAsync(S->herr, S->err, sizeof(int), cudaMemcpyDeviceToHost, c->st));
     I3G_CUDA(cudaStreamSynchronize(c->st));
-    const int e = *S->herr;
+    const int e = *S->herr & ~ERR_REDO;
     if (!e) return 0;
     if (e & ERR_TYPE) return set_error(c, I3G_E_UNSUPPORTED, "%s: fluid or immobile marker types (>= 50) are not supported", what);
     if (e & ERR_GRAIN) return set_error(c, I3G_E_UNSUPPORTED, "%s: grain-damage rheology (markdh < 0) is not supported", what);
@@ -1828,14 +2028,28 @@ int markers_to_nodes(i3g_ctx *c, double timestep)
     else
         I3G_CUDA(cudaMemsetAsync(S->stage, 0, sizeof(double) * (size_t)S->ntiles * NACC * NBOX, c->st));
     NodeOut O{c->lev[0].nu, c->nxx, c->nxy, c->nxz, c->nyz, c->ro, c->cp, c->kt, c->ht, c->et, c->tk, c->rr, S->tk1};
-    LAUNCH(k_r2n_gather, nb(N), 256, 0, (const double *)S->stage, T, (int)c->m.xnumx, (int)c->m.ynumy, (int)c->m.znumz, O,
-           c->p.viscmod, c->p.nubeg, c->p.nuend);
-    if (S->tbc_n)
-        LAUNCH(k_tk_bc, nb(S->tbc_n), 256, 0, c->tk, (const float *)S->tk1, S->tbc_n, (const int *)S->tbc_node,
-               (const int *)S->tbc_p, (const double *)S->tbc_c, (const double *)S->tbc_k);
+    auto average = [&]() {
+        LAUNCH(k_r2n_gather, nb(N), 256, 0, (const double *)S->stage, T, (int)c->m.xnumx, (int)c->m.ynumy, (int)c->m.znumz, O,
+               c->p.viscmod, c->p.nubeg, c->p.nuend);
+        if (S->tbc_n)
+            LAUNCH(k_tk_bc, nb(S->tbc_n), 256, 0, c->tk, (const float *)S->tk1, S->tbc_n, (const int *)S->tbc_node,
+                   (const int *)S->tbc_p, (const double *)S->tbc_c, (const double *)S->tbc_k);
+    };
+    average();
     I3G_CUDA(cudaGetLastError());
     I3G_CUDA(cudaEventRecord(e1, c->st));
     rc = check_err(c, "ronurecalc");
+    if (*S->herr & ERR_REDO) {
+        // a marker that k_r2n_mma does not take: the pass again from the temperatures before the
+        // boundary rows (nodes without markers keep theirs)
+        I3G_CUDA(cudaMemcpyAsync(c->tk, S->tk1, sizeof(float) * N, cudaMemcpyDeviceToDevice, c->st));
+        I3G_CUDA(cudaMemsetAsync(S->err, 0, sizeof(int), c->st));
+        launch_r2n(c, S->a, (const int *)S->coff, T, timestep, S->stage, true);
+        average();
+        I3G_CUDA(cudaGetLastError());
+        I3G_CUDA(cudaEventRecord(e1, c->st));
+        rc = check_err(c, "ronurecalc");
+    }
     float ms_ = 0;
     cudaEventElapsedTime(&ms_, e0, e1);
     c->st_.ms_r2n = ms_;

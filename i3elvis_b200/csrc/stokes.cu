@@ -394,8 +394,8 @@ __device__ __forceinline__ void relax_vel_at(const View<T> &L, long t, int color
 // store.  The kernel before a run of relaxations (a restriction, prolongation or conversion) lets its
 // successor launch only after its own wait, and it writes no operator data, so whatever set the
 // operator up has completed by then.  On B200 a sweep went from 25 to 16 us on levels of 12^3 to 33^3
-// (22 with the packed boundary rows alone) and from 30 to 22 at 65^3; a level of 129^3 takes 108 us, of
-// which latency is a small part, and keeps the plain form with larger blocks.
+// (22 with the packed boundary rows alone) and from 30 to 22 at 65^3; at 129^3 it takes 107 us plain and
+// 114 with the prologue (blocks of 128 threads, registers held over the wait).
 constexpr long kProNodes = 400000;
 
 template <typename T, int V, bool PRO>

@@ -7,6 +7,7 @@ import cases
 import oracle as O
 from conftest import golden
 from i3elvis_b200 import abi, config, lib, model
+from test_oracle_markers import marker_setup
 
 pytestmark = pytest.mark.gpu
 
@@ -65,3 +66,63 @@ def test_vcycles_bit_exact_for_wall_factors(factor, pro, monkeypatch):
 def test_vcycles_bit_exact_on_boxes(shape, multinum, pro, monkeypatch):
     monkeypatch.setenv("I3G_PRO_NODES", pro)
     _vcycles_match(*_random_box(shape, multinum, seed=sum(shape)))
+
+
+def _cloud(seed=5):
+    """Reference fields of the 13^3 case with markers of every rock moved to uneven places: empty cells,
+    cells of a few markers and cells of several hundred (more than a warp stages at once)."""
+    p, mode, fx, buf = marker_setup("sphere13")
+    rng = np.random.default_rng(seed)
+    n = buf.f32["markx"].size
+    L = 1e5
+    for f in ("markx", "marky", "markz"):
+        a = rng.uniform(0.001 * L, 0.999 * L, n)
+        a[: n // 2] = rng.uniform(0.30 * L, 0.42 * L, n // 2)
+        buf.f32[f][:] = a
+    buf.f32["markk"][:] = rng.uniform(300, 1500, n)
+    buf.f32["markv"][:] = 1e21 * np.exp(rng.normal(0, 2, n))
+    return p, mode, fx, buf
+
+
+NODE_SUMS = ("ro", "nu", "nxx", "nxy", "nxz", "nyz", "tk", "cp", "kt", "et", "ht", "rr")
+
+
+def _nodes_match(mode, dt, edit, exact, **fields):
+    bufs = []
+    for side in range(2):
+        _, _, _, buf = _cloud()
+        edit(buf)
+        par, fp = abi.make_params(mode, marker_exact=exact), abi.make_file_params(mode.files[0])
+        for k, v in fields.items():
+            setattr(par, k, v)
+        c = lib.Context(buf, par, fp) if side == 0 else O.Oracle(buf, par, fp)
+        if side == 0:
+            c.markers_to_nodes(dt)
+        else:
+            c.call("orc_markers_to_nodes", dt)
+        c.download(abi.SYNC_ALL)
+        c.close()
+        bufs.append(buf)
+    for f in NODE_SUMS:   # FP64 sums in another order, stored as FP32
+        np.testing.assert_allclose(bufs[0].f32[f], bufs[1].f32[f], rtol=3e-7, atol=0, err_msg=f)
+    np.testing.assert_allclose(bufs[0].f32["markv"], bufs[1].f32["markv"], rtol=2e-7)
+
+
+@pytest.mark.parametrize("exact", [0, 1])
+@pytest.mark.parametrize("viscmod,nukoef", [(0, 0.0), (1, 0.0), (2, 0.3)])
+def test_node_sums_of_uneven_cells(viscmod, nukoef, exact):
+    """Marker -> node sums over cells of 0 to several hundred markers, the three viscosity averages
+    and the nukoef gate, against the oracle."""
+    _, mode, _, _ = _cloud()
+    _nodes_match(mode, 1e10, lambda buf: None, exact, viscmod=viscmod, nukoef=nukoef)
+
+
+@pytest.mark.parametrize("exact", [0, 1])
+def test_node_sums_with_markers_without_viscosity(exact):
+    """A marker whose viscosity is still 0 in a time step gets one from the rheology, as in the
+    initial passes; the others' sums stay the same."""
+    _, mode, _, _ = _cloud()
+
+    def edit(buf):
+        buf.f32["markv"][[7, 300, 9000]] = 0.0
+    _nodes_match(mode, 1e10, edit, exact)
