@@ -126,3 +126,29 @@ def test_node_sums_with_markers_without_viscosity(exact):
     def edit(buf):
         buf.f32["markv"][[7, 300, 9000]] = 0.0
     _nodes_match(mode, 1e10, edit, exact)
+
+
+def test_partial_download_after_a_sort():
+    """A download that names a few marker arrays returns those in the original order, and fields that
+    the sort does not move stay with their markers."""
+    p, mode, fx, buf = marker_setup("sphere13")
+    n = buf.f32["markx"].size
+    rng = np.random.default_rng(9)
+    for f in ("markw", "markd", "markex", "markft", "markrn"):
+        buf.f32[f][:] = rng.uniform(0, 1, n)
+    keep = {f: buf.f32[f].copy() for f in ("markw", "markd", "markex", "markft", "markrn")}
+    g = lib.Context(buf, abi.make_params(mode), abi.make_file_params(mode.files[0]))
+    g.move_markers(float(fx["fld_dt"][0]))
+    g.markers_to_nodes(1e10)
+    g.download(abi.SYNC_MARKERS)
+    whole = {f: buf.f32[f].copy() for f in abi.MARK_F32}
+    for f, v in keep.items():
+        assert np.array_equal(whole[f], v), f
+    part = abi.Model.from_buffer_copy(buf.model)
+    got = np.zeros(n, np.float32)
+    for f in abi.MARK_F32:
+        setattr(part, f, got.ctypes.data_as(abi.c_f32p) if f == "marky" else abi.c_f32p())
+    part.markt = abi.c_i8p()
+    g.call("i3g_download", part, abi.SYNC_MARKERS)
+    assert np.array_equal(got, whole["marky"])
+    g.close()
