@@ -59,13 +59,18 @@ struct MarkerState {
     double *stage = nullptr;        // [ntiles][NACC][NBOX] per-tile node-box sums (no atomics)
     float *tk1 = nullptr;           // copy of T before boundary rows
     double *rock = nullptr;         // [24 * rocknum]
+    uint8_t *use = nullptr;         // [128] invariants the rheology of each rock type reads
     int *err = nullptr, *herr = nullptr;
     int tbc_n = 0;                  // temperature boundary rows (level 0)
     int *tbc_node = nullptr, *tbc_p = nullptr;
     double *tbc_c = nullptr, *tbc_k = nullptr;
     bool sorted = false;
     // register caps of the FP64-latency-bound marker kernels (resident CTAs per SM they allow)
-    int move_minb = 2;              // k_move: 2 (128 registers), 3 or 4 (I3G_MOVE_OCC)
+    // k_move without and with invariants: 2 (128 registers), 3 or 4 (I3G_MOVE_OCC).  Without them, 129^3
+    // with 56.6 M markers on B200: 5.86 ms with 2, 5.29 with 3 (28 bytes spilled), 6.47 with 4; with them
+    // the third CTA spills and gains nothing
+    int move_minb[2] = {3, 2};
+    bool any_use = true;            // some rock of the model reads an invariant
     // k_heat_mark_cells: 2 CTAs per SM (64 registers; 4.5 ms instead of 6.6 ms at 129^3 with 56.6 M
     // markers on B200, its FP64 dependency chains need the extra warps), 1 with I3G_HEAT_OCC=1
     int heat_minb = 2;
@@ -302,112 +307,58 @@ __device__ __forceinline__ void vxyz(const Grid &G, const NodeF &F, double x, do
     if (out) *out = S;
 }
 
-// one shear group of epscalc1: strain rate, stress and the dissipation term 2 s e w
+// the same sum of an FP64 field
 template <bool EX>
-__device__ __forceinline__ void edge_group(const float *__restrict__ fe, const float *__restrict__ fs, int NY, int NXY,
-                                           const Ax &AX, const Ax &AY, const Ax &AZ, double &e, double &s, double &d)
+__device__ __forceinline__ double tri64(const double *__restrict__ f, int NY, int NXY, const Ax &X, const Ax &Y, const Ax &Z)
 {
-    const int n0 = AZ.i * NXY + AX.i * NY + AY.i;
-    if (!EX) {
-        e += tri_fact(n0, NY, NXY, AX, AY, AZ, [&](int n) { return (double)__ldg(fe + n); });
-        s += tri_fact(n0, NY, NXY, AX, AY, AZ, [&](int n) { return (double)__ldg(fs + n); });
-        d += tri_fact(n0, NY, NXY, AX, AY, AZ, [&](int n) { return 2.0 * (double)__ldg(fs + n) * (double)__ldg(fe + n); });
-        return;
-    }
+    const int n0 = Z.i * NXY + X.i * NY + Y.i;
+    if (!EX) return tri_fact(n0, NY, NXY, X, Y, Z, [&](int n) { return __ldg(f + n); });
+    const double *p = f + n0;
+    double s = 0;
 #pragma unroll
-    for (int k3 = 0; k3 < 2; k3++) {
-        const double ddz = k3 ? AZ.w1 : AZ.w0;
+    for (int k3 = 0; k3 < 2; k3++)
 #pragma unroll
-        for (int k1 = 0; k1 < 2; k1++) {
-            const double ddx = k1 ? AX.w1 : AX.w0;
+        for (int k1 = 0; k1 < 2; k1++)
 #pragma unroll
-            for (int k2 = 0; k2 < 2; k2++) {
-                const double ddy = k2 ? AY.w1 : AY.w0;
-                const int n = n0 + k3 * NXY + k1 * NY + k2;
-                const double w = ddx * ddy * ddz;
-                const float ev = __ldg(fe + n), sv = __ldg(fs + n);
-                e += ev * w;
-                s += sv * w;
-                d += 2.0 * sv * ev * w;
-            }
-        }
-    }
+            for (int k2 = 0; k2 < 2; k2++)
+                s += __ldg(p + k3 * NXY + k1 * NY + k2) * ((k1 ? X.w1 : X.w0) * (k2 ? Y.w1 : Y.w0) * (k3 ? Z.w1 : Z.w0));
+    return s;
 }
 
-// epscalc1 (mark3mg.c:2535-2838) at the point of the first vxyz call, from its cell and
-// mid-point stencils: normal strain rates, stresses and pressure at cell centres, the three
-// shear groups on their edges, and the dissipation sum, each with weights clamped to [0, 1].
+// Stencils of one point for epscalc1 (mark3mg.c:2535-2838), weights clamped to [0, 1]: cell centres
+// for the normal components and pressure, clamped node lines and mid-points for the shear groups.
+struct EStencil {
+    Ax cx, cy, cz, ix, iy, iz, qx, qy, qz;
+};
+
+// from the cell and mid-point stencils of the first vxyz call
 template <bool EX>
-__device__ __forceinline__ void eps_from(const Grid &G, const NodeF &F, double x, double y, double z, const int *wn,
-                                         const VStencil &S, double *e, double *s, double *dis)
+__device__ __forceinline__ void eps_stencil(const Grid &G, double x, double y, double z, const int *wn, const VStencil &S, bool shear,
+                                            EStencil &E)
 {
-    const double *gx = G.gx, *gy = G.gy, *gz = G.gz;
-    const int X = G.nx, Y = G.ny, Z = G.nz;
     if (x < 0) x = 0; if (x > G.xsize) x = G.xsize;
     if (y < 0) y = 0; if (y > G.ysize) y = G.ysize;
     if (z < 0) z = 0; if (z > G.zsize) z = G.zsize;
-    const int NY = (int)F.NY, NXY = (int)F.NXY;
-    for (int i = 0; i < 7; i++) e[i] = 0;
-    for (int i = 0; i < 6; i++) s[i] = 0;
-    double d = 0;
-    if (!EX) {
-        const Ax cx = ax_cent<false>(G, 0, gx, X, wn[0], x), cy = ax_cent<false>(G, 1, gy, Y, wn[1], y),
-                 cz = ax_cent<false>(G, 2, gz, Z, wn[2], z);
-        const int n0 = cz.i * NXY + cx.i * NY + cy.i;
+    E.cx = ax_cent<EX>(G, 0, G.gx, G.nx, wn[0], x);
+    E.cy = ax_cent<EX>(G, 1, G.gy, G.ny, wn[1], y);
+    E.cz = ax_cent<EX>(G, 2, G.gz, G.nz, wn[2], z);
+    if (!shear) return;
+    // edge groups: node lines clamped to [1, n - 3] and the mid-point stencils
+    E.ix = clamped(ax_line<EX>(G, 0, G.gx, G.nx, wn[0], x, 1, 3));
+    E.iy = clamped(ax_line<EX>(G, 1, G.gy, G.ny, wn[1], y, 1, 3));
+    E.iz = clamped(ax_line<EX>(G, 2, G.gz, G.nz, wn[2], z, 1, 3));
+    E.qx = clamped(S.mx); E.qy = clamped(S.my); E.qz = clamped(S.mz);
+}
+
+// the six components of a strain-rate or stress field at the point
+template <bool EX>
+__device__ __forceinline__ void eps_fields(const float *const *f, int NY, int NXY, const EStencil &E, double *e)
+{
 #pragma unroll
-        for (int q = 0; q < 3; q++) {
-            e[q] = tri_fact(n0, NY, NXY, cx, cy, cz, [&](int n) { return (double)__ldg(F.e[q] + n); });
-            s[q] = tri_fact(n0, NY, NXY, cx, cy, cz, [&](int n) { return (double)__ldg(F.s[q] + n); });
-        }
-        e[6] = tri_fact(n0, NY, NXY, cx, cy, cz, [&](int n) { return __ldg(F.pr + n); });
-        // the dissipation of the normal components: the FP32 sum of the three products per corner
-        d = tri_fact(n0, NY, NXY, cx, cy, cz, [&](int n) {
-            return (double)__fadd_rn(__fadd_rn(__fmul_rn(__ldg(F.s[0] + n), __ldg(F.e[0] + n)),
-                                               __fmul_rn(__ldg(F.s[1] + n), __ldg(F.e[1] + n))),
-                                     __fmul_rn(__ldg(F.s[2] + n), __ldg(F.e[2] + n)));
-        });
-        const Ax ix = clamped(ax_line<false>(G, 0, gx, X, wn[0], x, 1, 3)), iy = clamped(ax_line<false>(G, 1, gy, Y, wn[1], y, 1, 3)),
-                 iz = clamped(ax_line<false>(G, 2, gz, Z, wn[2], z, 1, 3));
-        const Ax qx = clamped(S.mx), qy = clamped(S.my), qz = clamped(S.mz);
-        edge_group<false>(F.e[3], F.s[3], NY, NXY, ix, iy, qz, e[3], s[3], d);   // exy
-        edge_group<false>(F.e[4], F.s[4], NY, NXY, ix, qy, iz, e[4], s[4], d);   // exz
-        edge_group<false>(F.e[5], F.s[5], NY, NXY, qx, iy, iz, e[5], s[5], d);   // eyz
-        *dis = d;
-        return;
-    }
-    {
-        const Ax cx = ax_cent<true>(G, 0, gx, X, wn[0], x), cy = ax_cent<true>(G, 1, gy, Y, wn[1], y),
-                 cz = ax_cent<true>(G, 2, gz, Z, wn[2], z);
-        const int n0 = cz.i * NXY + cx.i * NY + cy.i;
-#pragma unroll
-        for (int k3 = 0; k3 < 2; k3++) {
-            const double ddz = k3 ? cz.w1 : cz.w0;
-#pragma unroll
-            for (int k1 = 0; k1 < 2; k1++) {
-                const double ddx = k1 ? cx.w1 : cx.w0;
-#pragma unroll
-                for (int k2 = 0; k2 < 2; k2++) {
-                    const double ddy = k2 ? cy.w1 : cy.w0;
-                    const int n = n0 + k3 * NXY + k1 * NY + k2;
-                    const double w = ddx * ddy * ddz;
-                    const float exx = __ldg(F.e[0] + n), eyy = __ldg(F.e[1] + n), ezz = __ldg(F.e[2] + n);
-                    const float sxx = __ldg(F.s[0] + n), syy = __ldg(F.s[1] + n), szz = __ldg(F.s[2] + n);
-                    e[0] += exx * w; e[1] += eyy * w; e[2] += ezz * w;
-                    s[0] += sxx * w; s[1] += syy * w; s[2] += szz * w;
-                    d += (double)(__fadd_rn(__fadd_rn(__fmul_rn(sxx, exx), __fmul_rn(syy, eyy)), __fmul_rn(szz, ezz))) * w;
-                    e[6] += __ldg(F.pr + n) * w;
-                }
-            }
-        }
-    }
-    // edge groups: node lines clamped to [1, n - 3] and the mid-point stencils, weights in [0, 1]
-    const Ax ix = clamped(ax_line<true>(G, 0, gx, X, wn[0], x, 1, 3)), iy = clamped(ax_line<true>(G, 1, gy, Y, wn[1], y, 1, 3)),
-             iz = clamped(ax_line<true>(G, 2, gz, Z, wn[2], z, 1, 3));
-    const Ax qx = clamped(S.mx), qy = clamped(S.my), qz = clamped(S.mz);
-    edge_group<true>(F.e[3], F.s[3], NY, NXY, ix, iy, qz, e[3], s[3], d);   // exy
-    edge_group<true>(F.e[4], F.s[4], NY, NXY, ix, qy, iz, e[4], s[4], d);   // exz
-    edge_group<true>(F.e[5], F.s[5], NY, NXY, qx, iy, iz, e[5], s[5], d);   // eyz
-    *dis = d;
+    for (int q = 0; q < 3; q++) e[q] = tri<EX>(f[q], NY, NXY, E.cx, E.cy, E.cz);
+    e[3] = tri<EX>(f[3], NY, NXY, E.ix, E.iy, E.qz);   // xy
+    e[4] = tri<EX>(f[4], NY, NXY, E.ix, E.qy, E.iz);   // xz
+    e[5] = tri<EX>(f[5], NY, NXY, E.qx, E.iy, E.iz);   // yz
 }
 
 // epscalc1 with the cell given (mark3mg.c:2535-2838)
@@ -538,8 +489,23 @@ struct Phys {
     int rocknum, densimod, viscmod, outgrid, markmod;
     double nubeg, nuend, nukoef, healrate, timesum;
     double zdeep, vdeep, tdeep, nudeep, teclmin, teclmax, eroslev, sedilev, waterlev;
+    const uint8_t *use;   // [128] per rock type: invariants its rheology reads (rheo_use)
     int *err;
 };
+
+// Invariants that visc() reads for a rock: the strain rate for yielding, power-law creep (ss != 0 and
+// mm != 1) and the nu < 0 branch, the stress (through the stress ratio) for yielding alone.  A rock
+// yields only if one end of its strength interpolation is positive, and a marker's accumulated
+// strain, which grows with the strain rate while it is positive, is made non-positive by visc()
+// unless it yields.  Type 0 and 1 never yield.
+constexpr int kUseStrain = 1, kUseStress = 2;
+static uint8_t rheo_use(const double *const *rock, int t)
+{
+    auto R = [&](int f) { return rock[f] ? rock[f][t] : 0.0; };
+    const bool yields = t > 1 && (!(R(R_A0) <= 0) || !(R(R_A1) <= 0) || !(R(R_B0) <= 0) || !(R(R_B1) <= 0));
+    const bool creep = R(R_NU) != 0 && ((R(R_SS) != 0 && R(R_MM) != 1.0) || !(R(R_NU) > 0));
+    return (uint8_t)((yields ? kUseStrain | kUseStress : 0) | (creep ? kUseStrain : 0));
+}
 
 __device__ __forceinline__ double RK(const Phys &P, int f, int t) { return P.rock[f * P.rocknum + t]; }
 
@@ -670,8 +636,8 @@ __device__ __forceinline__ double inv2(const double *e)
 // ------------------------------------------------------------------------------------
 // movemark: rheology update + RK4 (mark3mg.c:49-310)
 // ------------------------------------------------------------------------------------
-// one marker of movemark (mark3mg.c:49-310)
-template <bool EX>
+// one marker of movemark (mark3mg.c:49-310); USE = false: no rock of the model reads an invariant
+template <bool EX, bool USE>
 __device__ __forceinline__ void move_one(const Marks &M, long i, const Grid &G, const NodeF &F, const Phys &P, double timestep)
 {
     int t = M.t[i];
@@ -680,19 +646,32 @@ __device__ __forceinline__ void move_one(const Marks &M, long i, const Grid &G, 
     if (!(inbox || (P.outgrid != 1 && (t < 50 || t >= 100)))) return;
     if (t >= 50) { atomicOr(P.err, ERR_TYPE); return; }
     const double yold = fy;
-    double v1[3], e[7], s[6], dis;
+    double v1[3];
     int wn[3];
     VStencil S0;
     vxyz<EX>(G, F, fx, fy, fz, v1, wn, &S0);
-    eps_from<EX>(G, F, fx, fy, fz, wn, S0, e, s, &dis);
-    const double eii = inv2(e), sii = inv2(s);
-    const double mpb = e[6] * 1e-5;
     float mk = M.k[i], mv = M.v[i], me = M.e[i];
     int water0 = 0;   // bound water reset to 0 below
     const double mtk = mk;
     if (t < 50 && mtk > 0) {
+        // The strain-rate and stress invariants are interpolated only for rocks whose rheology reads
+        // them (rheo_use): 12 of the 13 nodal sums, both square roots and the power law of the
+        // stress ratio drop out for a Newtonian or diffusion-creep rock without a yield strength.
+        const int use = USE ? P.use[t & 127] : 0;
+        EStencil E;
+        eps_stencil<EX>(G, fx, fy, fz, wn, S0, use != 0, E);
+        const double mpb = tri64<EX>(F.pr, (int)F.NY, (int)F.NXY, E.cx, E.cy, E.cz) * 1e-5;
+        double eii = 0, sii = 0, q[6];
+        if (use) {
+            eps_fields<EX>(F.e, (int)F.NY, (int)F.NXY, E, q);
+            eii = inv2(q);
+        }
+        if (use & kUseStress) {
+            eps_fields<EX>(F.s, (int)F.NY, (int)F.NXY, E, q);
+            sii = inv2(q);
+        }
         double rii = 1.0;
-        if (mv > 0 && fx > G.gx[3] && fx < G.gx[G.nx - 4] && fy > G.gy[3] && fy < G.gy[G.ny - 4] && fz > G.gz[3] && fz < G.gz[G.nz - 4])
+        if ((use & kUseStress) && mv > 0 && fx > G.gx[3] && fx < G.gx[G.nx - 4] && fy > G.gy[3] && fy < G.gy[G.ny - 4] && fz > G.gz[3] && fz < G.gz[G.nz - 4])
             // the power law of the stress ratio; the fast arithmetic takes it as exp(0.87 log r)
             // (relative difference ~1e-15, far below the FP32 viscosity it feeds)
             rii *= EX ? pow(0.5 * sii / eii / mv, 0.87) : exp(0.87 * log(0.5 * sii / eii / mv));
@@ -743,14 +722,14 @@ __device__ __forceinline__ void move_one(const Marks &M, long i, const Grid &G, 
 // Persistent grid-stride launch (a few CTAs per SM): the grid lines are staged in shared memory
 // once per CTA instead of once per 256 markers.  Markers are in (tile, cell) order from the last
 // sort, so a warp's interpolation corners hit the same L1 lines.
-template <bool EX, int MINB>
+template <bool EX, int MINB, bool USE>
 __global__ void __launch_bounds__(256, MINB) k_move(Marks M, long n, Grid Gg, NodeF F, Phys P, double timestep)
 {
     extern __shared__ double shg[];
     Grid G;
     load_grid<EX>(Gg, shg, G);
     for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
-        move_one<EX>(M, i, G, F, P, timestep);
+        move_one<EX, USE>(M, i, G, F, P, timestep);
 }
 
 // ------------------------------------------------------------------------------------
@@ -1699,6 +1678,7 @@ static Phys phys_of(i3g_ctx *c)
     P.zdeep = c->p.zdeep; P.vdeep = c->p.vdeep; P.tdeep = c->p.tdeep; P.nudeep = c->p.nudeep;
     P.teclmin = c->p.teclmin; P.teclmax = c->p.teclmax;
     P.eroslev = c->p.eroslev; P.sedilev = c->p.sedilev; P.waterlev = c->p.waterlev;
+    P.use = S->use;
     P.err = S->err;
     return P;
 }
@@ -1709,34 +1689,36 @@ static size_t grid_smem(i3g_ctx *c) { return 4 * sizeof(double) * (c->m.xnumx + 
 // the marker kernels' arithmetic: the reference's operation order (marker_exact) or the fast one
 static bool mexact(i3g_ctx *c) { return c->p.marker_exact != 0; }
 
-template <bool EX>
-static void launch_move_t(i3g_ctx *c, unsigned grid, const Marks &M, long n, const Grid &G, const NodeF &F, const Phys &P,
-                          double dt)
+// k_move with the model's arithmetic, register cap and need of invariants
+using MoveKernel = void (*)(Marks, long, Grid, NodeF, Phys, double);
+template <bool EX, bool USE>
+static MoveKernel move_kernel_t(int minb)
 {
-    switch (ms(c)->move_minb) {
-    case 3: LAUNCH((k_move<EX, 3>), grid, 256, grid_smem(c), M, n, G, F, P, dt); break;
-    case 4: LAUNCH((k_move<EX, 4>), grid, 256, grid_smem(c), M, n, G, F, P, dt); break;
-    default: LAUNCH((k_move<EX, 2>), grid, 256, grid_smem(c), M, n, G, F, P, dt); break;
-    }
+    return minb == 4 ? k_move<EX, 4, USE> : minb == 3 ? k_move<EX, 3, USE> : k_move<EX, 2, USE>;
+}
+static MoveKernel move_kernel(i3g_ctx *c)
+{
+    const MarkerState *S = ms(c);
+    const int m = S->move_minb[S->any_use];
+    if (mexact(c)) return S->any_use ? move_kernel_t<true, true>(m) : move_kernel_t<true, false>(m);
+    return S->any_use ? move_kernel_t<false, true>(m) : move_kernel_t<false, false>(m);
+}
+
+// resident k_move CTAs on all SMs (the same for both arithmetic variants: both are capped at the same
+// register count by __launch_bounds__)
+static int move_blocks(i3g_ctx *c, int sms)
+{
+    int per_sm = 0;
+    I3G_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, move_kernel(c), 256, grid_smem(c)));
+    ms(c)->move_blocks = (unsigned)std::max(1, sms * std::max(per_sm, 1));
+    return 0;
 }
 
 static void launch_move(i3g_ctx *c, unsigned grid, const Marks &M, long n, const Grid &G, const NodeF &F, const Phys &P,
                         double dt)
 {
-    if (mexact(c)) launch_move_t<true>(c, grid, M, n, G, F, P, dt);
-    else launch_move_t<false>(c, grid, M, n, G, F, P, dt);
-}
-
-// resident k_move CTAs per SM (the same for both arithmetic variants: both are capped at the
-// same register count by __launch_bounds__)
-static int move_occupancy(i3g_ctx *c, int *per_sm)
-{
-    switch (ms(c)->move_minb) {
-    case 3: I3G_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k_move<false, 3>, 256, grid_smem(c))); break;
-    case 4: I3G_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k_move<false, 4>, 256, grid_smem(c))); break;
-    default: I3G_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k_move<false, 2>, 256, grid_smem(c))); break;
-    }
-    return 0;
+    move_kernel(c)<<<grid, 256, grid_smem(c), c->st>>>(M, n, G, F, P, dt);
+    c->launches++;
 }
 
 static void launch_r2n(i3g_ctx *c, const Marks &M, const int *coff, const TileGeo &T, double timestep, double *stage, bool redo = false);
@@ -1824,6 +1806,14 @@ int markers_alloc(i3g_ctx *c)
         for (int t = 0; t < rn; t++) rk[(size_t)f * rn + t] = c->m.rock[f] ? c->m.rock[f][t] : 0.0;
     I3G_CUDA(cudaMalloc((void **)&S->rock, sizeof(double) * rk.size()));
     I3G_CUDA(cudaMemcpyAsync(S->rock, rk.data(), sizeof(double) * rk.size(), cudaMemcpyHostToDevice, c->st));
+    std::vector<uint8_t> use(128, kUseStrain | kUseStress);
+    S->any_use = false;
+    for (int t = 0; t < std::min(rn, 128); t++) {
+        use[t] = rheo_use(c->m.rock, t);
+        S->any_use = S->any_use || use[t];
+    }
+    I3G_CUDA(cudaMalloc((void **)&S->use, use.size()));
+    I3G_CUDA(cudaMemcpyAsync(S->use, use.data(), use.size(), cudaMemcpyHostToDevice, c->st));
     I3G_CUDA(cudaMalloc((void **)&S->err, sizeof(int)));
     I3G_CUDA(cudaMallocHost((void **)&S->herr, sizeof(int)));
     // temperature boundary rows of level 0 (bondm[8*nodenum + node], heat3mg.c:859-889)
@@ -1850,13 +1840,11 @@ int markers_alloc(i3g_ctx *c)
         I3G_CUDA(cudaMemcpyAsync(S->tbc_k, tkk.data(), sizeof(double) * tkk.size(), cudaMemcpyHostToDevice, c->st));
     }
     {
-        int dev = 0, sms = 0, per_sm = 0;
+        int dev = 0, sms = 0;
         I3G_CUDA(cudaGetDevice(&dev));
         I3G_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        if (const char *e = getenv("I3G_MOVE_OCC")) S->move_minb = std::min(4, std::max(2, atoi(e)));
+        if (const char *e = getenv("I3G_MOVE_OCC")) S->move_minb[0] = S->move_minb[1] = std::min(4, std::max(2, atoi(e)));
         if (const char *e = getenv("I3G_HEAT_OCC")) S->heat_minb = std::min(2, std::max(1, atoi(e)));
-        if (int rc = move_occupancy(c, &per_sm)) return rc;
-        S->move_blocks = (unsigned)std::max(1, sms * std::max(per_sm, 1));
         int a = 0, b = 0;
         I3G_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_tile_key, 256, grid_smem(c)));
         I3G_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_heat_mark_anti<false>, 256, grid_smem(c)));
@@ -1874,8 +1862,15 @@ int markers_alloc(i3g_ctx *c)
     I3G_CUDA(cudaFuncSetAttribute((k_heat_mark_cells<true, 2>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)heat_mark_smem(c)));
     I3G_CUDA(cudaFuncSetAttribute((k_heat_mark_cells<false, 1>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)heat_mark_smem(c)));
     I3G_CUDA(cudaFuncSetAttribute((k_heat_mark_cells<false, 2>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)heat_mark_smem(c)));
-    for (auto f : {k_move<true, 2>, k_move<true, 3>, k_move<true, 4>, k_move<false, 2>, k_move<false, 3>, k_move<false, 4>})
-        I3G_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)grid_smem(c)));
+    for (int m = 2; m <= 4; m++)
+        for (MoveKernel f : {move_kernel_t<true, true>(m), move_kernel_t<true, false>(m), move_kernel_t<false, true>(m), move_kernel_t<false, false>(m)})
+            I3G_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)grid_smem(c)));
+    {
+        int dev = 0, sms = 0;
+        I3G_CUDA(cudaGetDevice(&dev));
+        I3G_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        if (int rc = move_blocks(c, sms)) return rc;
+    }
     for (auto f : {k_heat_mark_anti<true>, k_heat_mark_anti<false>})
         I3G_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)grid_smem(c)));
     I3G_CUDA(cudaFuncSetAttribute(k_tile_key, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)grid_smem(c)));
@@ -1893,7 +1888,7 @@ void markers_free(i3g_ctx *c)
     free_marks(S->b);
     for (float *p : {S->a.w, S->a.d, S->a.ex, S->a.ft, S->a.rn}) cudaFree(p);
     cudaFree(S->key); cudaFree(S->cnt); cudaFree(S->coff); cudaFree(S->off); cudaFree(S->cur); cudaFree(S->bsum); cudaFree(S->acc); cudaFree(S->stage); cudaFree(S->tk1);
-    cudaFree(S->rock); cudaFree(S->err);
+    cudaFree(S->rock); cudaFree(S->use); cudaFree(S->err);
     if (S->herr) cudaFreeHost(S->herr);
     if (S->up_ev) cudaEventDestroy(S->up_ev);
     cudaFree(S->tbc_node); cudaFree(S->tbc_p); cudaFree(S->tbc_c); cudaFree(S->tbc_k);

@@ -7,6 +7,7 @@ import cases
 import oracle as O
 from conftest import golden
 from i3elvis_b200 import abi, config, lib, model
+from i3elvis_b200.prn import ROCK_FIELDS
 from test_oracle_markers import marker_setup
 
 pytestmark = pytest.mark.gpu
@@ -152,3 +153,42 @@ def test_partial_download_after_a_sort():
     g.call("i3g_download", part, abi.SYNC_MARKERS)
     assert np.array_equal(got, whole["marky"])
     g.close()
+
+
+@pytest.mark.parametrize("exact", [0, 1])
+def test_marker_rheology_reads_what_it_needs(exact):
+    """Power-law rocks (with and without activation energy) use the strain rate, a yielding rock the
+    stress too, a Newtonian rock neither; positive strains of markers that do not yield turn negative."""
+    bufs = []
+    for side in range(2):
+        p, mode, fx, buf = marker_setup("sphere13")
+        rock = dict(zip(ROCK_FIELDS, buf.rocks))
+        rock["n0"][:], rock["n1"][:] = 1e5, 1e35
+        rng = np.random.default_rng(3)
+        n = buf.f32["markx"].size
+        buf.markt[:] = rng.integers(2, 4, n)
+        for f, v in dict(nu=1e9, ss=1e4, mm=3.0).items():   # type 2: power law
+            rock[f][2] = v
+        for f, v in dict(nu=1e-3, dh=2e5, ss=1e4, mm=3.0, a0=1e6, a1=1e6).items():   # type 3: with activation energy, yielding
+            rock[f][3] = v
+        buf.f32["marke"][:] = rng.uniform(-1, 1, n)
+        buf.f32["markv"][:] = 1e20
+        par, fp = abi.make_params(mode, marker_exact=exact), abi.make_file_params(mode.files[0])
+        fp.nubeg, fp.nuend = 1e5, 1e35
+        dt = float(fx["fld_dt"][0])
+        c = lib.Context(buf, par, fp) if side == 0 else O.Oracle(buf, par, fp)
+        if side == 0:
+            c.move_markers(dt)
+        else:
+            c.call("orc_move_markers", dt)
+        c.download(abi.SYNC_ALL)
+        c.close()
+        bufs.append(buf)
+    a, b = bufs
+    for f in ("markx", "marky", "markz"):
+        assert np.array_equal(a.f32[f], b.f32[f]), f
+    assert np.array_equal(a.markt, b.markt)
+    assert 0 < int((b.f32["marke"] > 0).sum()) < a.markt.size
+    # strains grow by dt * strain rate, stored as FP32; viscosities pass through pow and exp
+    np.testing.assert_allclose(a.f32["marke"], b.f32["marke"], rtol=2e-7, atol=0)
+    np.testing.assert_allclose(a.f32["markv"], b.f32["markv"], rtol=2e-7)
