@@ -1269,10 +1269,11 @@ __device__ __forceinline__ void box_range(int v, int TT, int nt, int &t0, int &t
 struct TkF { const float *tk0, *tk1, *tk, *tk2, *kt, *ro, *cp; long NY, NXY; };
 
 // tkcalc1 (mark3mg.c:2844-2910): cell, spacings, 8 weights and the 4 interpolated T arrays
-// wi[0..7] corner weights; wi[8..10] the cell's spacings (EX) or their reciprocals (fast)
+// wi[0..7] corner weights; wi[8..10] the cell's spacings (EX) or their reciprocals (fast); ws the
+// weights of the two sides along x, y, z
 template <bool EX>
 __device__ __forceinline__ void tk_at(const Grid &G, const TkF &T, double x, double y, double z, double *e, int *wn,
-                                      long *nodes, double *wi)
+                                      long *nodes, double *wi, double *ws = nullptr)
 {
     const int m10 = wn[0] = locate(G.gx, G.nx, x, G.ux), m20 = wn[1] = locate(G.gy, G.ny, y, G.uy), m30 = wn[2] = locate(G.gz, G.nz, z, G.uz);
     e[0] = e[1] = e[2] = e[3] = 0;
@@ -1293,6 +1294,7 @@ __device__ __forceinline__ void tk_at(const Grid &G, const TkF &T, double x, dou
         wx[0] = (G.gx[m10 + 1] - x) * rx; wx[1] = (x - G.gx[m10]) * rx;
         wy[0] = (G.gy[m20 + 1] - y) * ry; wy[1] = (y - G.gy[m20]) * ry;
     }
+    if (ws) { ws[0] = wx[0]; ws[1] = wx[1]; ws[2] = wy[0]; ws[3] = wy[1]; ws[4] = wz[0]; ws[5] = wz[1]; }
     int q = 0;
 #pragma unroll
     for (int k3 = 0; k3 < 2; k3++) {
@@ -1311,9 +1313,13 @@ __device__ __forceinline__ void tk_at(const Grid &G, const TkF &T, double x, dou
 }
 
 // One CTA per tile, one warp per cell (8 parity classes, as in k_r2n_cells): stage 1 updates
-// up to 32 markers of the cell (one per lane) and stages their node weights and subgrid
-// change; stage 2 sums them per node (lane = 2 * node + quantity) without atomics.
-constexpr int kHmStage = 9;   // wi[0..7], dtk1
+// up to 32 markers of the cell (one per lane) and stages their axis weights and subgrid change;
+// stage 2 sums the change and 1 per node as FP64 matrix products, four markers a step (dmma, as in
+// k_r2n_mma; the serial sum over the markers took a third of the kernel): 3.89 -> 2.91 ms at 129^3 with
+// 56.6 M markers on B200.
+// Staged doubles per marker: weights of the two node sides per axis x, y, z, change, 1 (an odd stride
+// keeps the reads of four markers free of bank conflicts).
+constexpr int kHmStage = 9;
 
 template <bool EX, int MINB>
 __global__ void __launch_bounds__(32 * kR2nWarps, MINB) k_heat_mark_cells(Marks M, const int *coff, Grid Gg, TkF T, TileGeo TG,
@@ -1332,8 +1338,8 @@ __global__ void __launch_bounds__(32 * kR2nWarps, MINB) k_heat_mark_cells(Marks 
     const int cx0 = tx * TX, cy0 = ty * TY, cz0 = tz * TZ;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     double *my = stg + warp * 32 * kHmStage;
-    const int nd = (lane >> 1) & 7, qty = lane & 1;
-    const int iz = nd >> 2, ix = (nd >> 1) & 1, iy = nd & 1;
+    const int g = lane >> 2, mk4 = lane & 3;   // node (or quantity), marker of the four
+    const int iz = g >> 2, ix = (g >> 1) & 1, iy = g & 1;
     for (int colour = 0; colour < 8; colour++) {
         const int pz = colour >> 2, px = (colour >> 1) & 1, py = colour & 1;
         for (int q = warp; q < CPT / 8; q += kR2nWarps) {
@@ -1342,16 +1348,16 @@ __global__ void __launch_bounds__(32 * kR2nWarps, MINB) k_heat_mark_cells(Marks 
             const long cell = (long)tile * CPT + (lz * TX + lx) * TY + ly;
             const int beg = coff[cell], end = coff[cell + 1];
             if (beg == end) continue;   // uniform over the warp
-            double acc_w = 0;
+            double d[2] = {0, 0};
             for (int base = beg; base < end; base += 32) {
                 bool staged = false;
                 if (base + lane < end) {
                     const int i = base + lane;
                     const float fx = M.x[i], fy = M.y[i], fz = M.z[i];
-                    double e[4], wi[11];
+                    double e[4], wi[11], ws[6];
                     int wn[3];
                     long nodes[8];
-                    tk_at<EX>(G, T, fx, fy, fz, e, wn, nodes, wi);
+                    tk_at<EX>(G, T, fx, fy, fz, e, wn, nodes, wi, ws);
                     float mk = M.k[i];
                     if (mk <= 0) {
                         mk = (float)e[3];
@@ -1375,25 +1381,36 @@ __global__ void __launch_bounds__(32 * kR2nWarps, MINB) k_heat_mark_cells(Marks 
                         dtk1 = dtk * (1.0 - exp(dtk1));
                         mk = __fadd_rn(mk, (float)dtk1);
                         double *st = my + lane * kHmStage;
-                        for (int qq = 0; qq < 8; qq++) st[qq] = wi[qq];
-                        st[8] = dtk1;
+#pragma unroll
+                        for (int qq = 0; qq < 6; qq++) st[qq] = ws[qq];
+                        st[6] = dtk1;
+                        st[7] = 1.0;
                         staged = true;
                     }
                     mk = __fadd_rn(mk, (float)(e[2] - e[3]));
                     M.k[i] = mk;
                 }
-                unsigned valid = __ballot_sync(0xffffffffu, staged);
+                if (!staged) {
+                    double *st = my + lane * kHmStage;
+#pragma unroll
+                    for (int qq = 0; qq < 8; qq++) st[qq] = 0.0;
+                }
                 __syncwarp();
-                // wi[] is ordered z, x, y (tk_at loops m3, m1, m2): node index = (iz*2 + ix)*2 + iy = nd
-                for (; valid; valid &= valid - 1) {
-                    const double *st = my + (__ffs(valid) - 1) * kHmStage;
-                    acc_w += qty ? st[8] * st[nd] : st[nd];
+                const int cnt = heatdif != 0 ? min(32, end - base) : 0;
+                for (int m0 = 0; m0 < cnt; m0 += 4) {
+                    const double *st = my + (m0 + mk4) * kHmStage;
+                    dmma(d, g == 0 ? st[7] : g == 1 ? st[6] : 0.0, st[ix] * st[2 + iy] * st[4 + iz]);
                 }
                 __syncwarp();
             }
-            if (lane < 16) {
-                const int lb = ((lz + iz) * NBX + (lx + ix)) * NBY + (ly + iy);
-                (qty ? sw1 : sw0)[lb] += acc_w;
+            // lanes 0-3 hold the weights of nodes 2 lane, 2 lane + 1, lanes 4-7 the changes
+            if (lane < 8) {
+                double *sw = lane < 4 ? sw0 : sw1;
+#pragma unroll
+                for (int u = 0; u < 2; u++) {
+                    const int t = 2 * mk4 + u;
+                    sw[((lz + (t >> 2)) * NBX + (lx + ((t >> 1) & 1))) * NBY + (ly + (t & 1))] += d[u];
+                }
             }
         }
         __syncthreads();
