@@ -198,31 +198,39 @@ struct ConvArgs {
     int *err;
 };
 
-template <int CIN, int COUT>
+// NT output channels per CTA (blockIdx.y selects them), a ring of ST stages, NTHR threads.  The whole
+// width in one CTA reads the input once; on the small grids of the coarse levels (3 row tiles at
+// 5^3 nodes) that leaves all but a few SMs idle and each step waits for 32 KB of operands behind three
+// stages.  There 16 channels per CTA give COUT / 16 times the CTAs, an eighth of the weights per step
+// and room for eight stages; every output is still the same sum in the same order.
+template <int CIN, int COUT, int NT = COUT, int ST = kStages, int THREADS = 128>
 struct ConvShape {
+    static constexpr int NTHR = THREADS;
     static constexpr int KC = CIN < 64 ? CIN : 64;             // channels per stage
     static constexpr int NKC = CIN / KC;
     static constexpr int NSTEP = 27 * NKC;
     static constexpr int ABYTES = kTileM * KC * 2;
-    static constexpr int BBYTES = COUT * KC * 2;
+    static constexpr int BBYTES = NT * KC * 2;
     static constexpr int SBYTES = ABYTES + BBYTES;
-    static constexpr uint32_t NCOL = COUT < 32 ? 32 : COUT;     // TMEM columns (power of 2 >= 32)
-    // kind::f16 instruction descriptor: D FP32, A and B BF16, both K-major, N = COUT, M = 128
-    static constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(COUT >> 3) << 17) |
+    static constexpr uint32_t NCOL = NT < 32 ? 32 : NT;         // TMEM columns (power of 2 >= 32)
+    // kind::f16 instruction descriptor: D FP32, A and B BF16, both K-major, N = NT, M = 128
+    static constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(NT >> 3) << 17) |
                                       ((uint32_t)(kTileM >> 4) << 24);
     // dynamic shared memory: the operand ring, raised so that the CTAs resident on one SM
     // never ask for more than the 512 TMEM columns (no CTA ever waits in tcgen05.alloc)
     // (plus 1 KiB: the ring starts at the next 1024-byte boundary of the dynamic buffer)
-    static constexpr int SMEM_RING = kStages * SBYTES + 1024;
+    static constexpr int SMEM_RING = ST * SBYTES + 1024;
     static constexpr int SMEM_TMEM = (int)NCOL * 460;
     static constexpr int SMEM = SMEM_RING > SMEM_TMEM ? SMEM_RING : SMEM_TMEM;
-    static_assert(CIN % 16 == 0 && COUT % 16 == 0 && COUT <= 256, "channel counts");
+    static_assert(CIN % 16 == 0 && NT % 16 == 0 && COUT % NT == 0 && NT <= 256, "channel counts");
 };
 
-template <int CIN, int COUT>
-__global__ void __launch_bounds__(128) k_conv_tc(ConvArgs a)
+template <int CIN, int COUT, int NT, int ST, int THREADS>
+__global__ void __launch_bounds__(THREADS) k_conv_tc(ConvArgs a)
 {
-    using S = ConvShape<CIN, COUT>;
+    using S = ConvShape<CIN, COUT, NT, ST, THREADS>;
+    constexpr int kStages = ST;
+    const int n0 = (int)blockIdx.y * NT;   // first output channel
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ __align__(8) uint64_t mbar[kStages];
     __shared__ uint32_t s_tmem;
@@ -258,7 +266,7 @@ __global__ void __launch_bounds__(128) k_conv_tc(ConvArgs a)
         // chunk j (channels 8j..8j+7) of row r at j*(rows*16) + r*16: 8-row core matrices
         // 128 bytes apart along M, the two K halves of a K=16 step rows*16 bytes apart
 #pragma unroll
-        for (int q = tid; q < kTileM * (S::KC / 8); q += 128) {
+        for (int q = tid; q < kTileM * (S::KC / 8); q += S::NTHR) {
             const int r = q / (S::KC / 8), j = q - r * (S::KC / 8);
             const long src = row0 + r + off;
             const bool ok = src >= 0 && src < a.d.np;
@@ -266,10 +274,10 @@ __global__ void __launch_bounds__(128) k_conv_tc(ConvArgs a)
             cp_async16(sA + (uint32_t)(j * (kTileM * 16) + r * 16), g, ok ? 16 : 0);
         }
 #pragma unroll
-        for (int q = tid; q < COUT * (S::KC / 8); q += 128) {
+        for (int q = tid; q < NT * (S::KC / 8); q += S::NTHR) {
             const int r = q / (S::KC / 8), j = q - r * (S::KC / 8);
-            const bf16 *g = a.w + ((long)tap * COUT + r) * CIN + kc * S::KC + j * 8;
-            cp_async16(sB + (uint32_t)(j * (COUT * 16) + r * 16), g, 16);
+            const bf16 *g = a.w + ((long)tap * COUT + n0 + r) * CIN + kc * S::KC + j * 8;
+            cp_async16(sB + (uint32_t)(j * (NT * 16) + r * 16), g, 16);
         }
     };
 
@@ -303,7 +311,7 @@ __global__ void __launch_bounds__(128) k_conv_tc(ConvArgs a)
 #pragma unroll
             for (int k = 0; k < S::KC / 16; k++) {
                 const uint64_t da = smem_desc(sA + (uint32_t)(2 * k * kTileM * 16), kTileM * 16, 128);
-                const uint64_t db = smem_desc(sB + (uint32_t)(2 * k * COUT * 16), COUT * 16, 128);
+                const uint64_t db = smem_desc(sB + (uint32_t)(2 * k * NT * 16), NT * 16, 128);
                 tc_mma(tmem, da, db, S::IDESC, (i > 0 || k > 0) ? 1u : 0u);
             }
             asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
@@ -327,24 +335,24 @@ __global__ void __launch_bounds__(128) k_conv_tc(ConvArgs a)
             if (issued > 0) mbar_wait(smem_u32(&mbar[(issued - 1) % kStages]), ((issued - 1) / kStages) & 1);
         }
         __syncthreads();
-    } else {
+    } else if (warp < 4) {
         tc_fence_after();
         const long p = row0 + warp * 32 + lane;
         const bool valid = p < a.d.np && interior_row(p, a.d);
 #pragma unroll
-        for (int c0 = 0; c0 < COUT; c0 += 16) {
+        for (int c0 = 0; c0 < NT; c0 += 16) {
             float v[16];
             tc_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, v);   // whole warp
             if (valid) {
                 if (a.bias) {
 #pragma unroll
-                    for (int q = 0; q < 16; q++) v[q] += a.bias[c0 + q];
+                    for (int q = 0; q < 16; q++) v[q] += a.bias[n0 + c0 + q];
                 }
                 if (a.add) {
 #pragma unroll
                     for (int h = 0; h < 2; h++) {
                         float f[8];
-                        unpack8(*reinterpret_cast<const uint4 *>(a.add + p * COUT + c0 + 8 * h), f);
+                        unpack8(*reinterpret_cast<const uint4 *>(a.add + p * COUT + n0 + c0 + 8 * h), f);
 #pragma unroll
                         for (int q = 0; q < 8; q++) v[8 * h + q] += f[q];
                     }
@@ -357,7 +365,7 @@ __global__ void __launch_bounds__(128) k_conv_tc(ConvArgs a)
 #pragma unroll
                     for (int h = 0; h < 2; h++) {
                         float f[8];
-                        unpack8(*reinterpret_cast<const uint4 *>(a.mask + p * COUT + c0 + 8 * h), f);
+                        unpack8(*reinterpret_cast<const uint4 *>(a.mask + p * COUT + n0 + c0 + 8 * h), f);
 #pragma unroll
                         for (int q = 0; q < 8; q++) v[8 * h + q] = f[q] > 0.0f ? v[8 * h + q] : 0.0f;
                     }
@@ -368,13 +376,13 @@ __global__ void __launch_bounds__(128) k_conv_tc(ConvArgs a)
                         float f[8];
 #pragma unroll
                         for (int q = 0; q < 8; q++) f[q] = v[8 * h + q];
-                        *reinterpret_cast<uint4 *>(a.out + p * COUT + c0 + 8 * h) = pack8(f);
+                        *reinterpret_cast<uint4 *>(a.out + p * COUT + n0 + c0 + 8 * h) = pack8(f);
                     }
                 }
                 if (a.out32) {
 #pragma unroll
                     for (int q = 0; q < 16; q += 4)
-                        *reinterpret_cast<float4 *>(a.out32 + p * COUT + c0 + q) = make_float4(v[q], v[q + 1], v[q + 2], v[q + 3]);
+                        *reinterpret_cast<float4 *>(a.out32 + p * COUT + n0 + c0 + q) = make_float4(v[q], v[q + 1], v[q + 2], v[q + 3]);
                 }
             }
         }
@@ -1432,10 +1440,10 @@ cudaError_t persistent_setup(K kernel, int smem, int max_per_sm, LaunchSetup (&c
     return cudaSuccess;
 }
 
-template <int CIN, int COUT>
-cudaError_t launch_conv_t(const ConvArgs &a, cudaStream_t st)
+template <int CIN, int COUT, int NT, int ST, int THREADS>
+cudaError_t launch_conv_n(const ConvArgs &a, cudaStream_t st)
 {
-    using S = ConvShape<CIN, COUT>;
+    using S = ConvShape<CIN, COUT, NT, ST, THREADS>;
     static bool attr[kMaxDev] = {};
     int dev = 0;
     cudaError_t e0 = cudaGetDevice(&dev);
@@ -1444,13 +1452,28 @@ cudaError_t launch_conv_t(const ConvArgs &a, cudaStream_t st)
     {
         std::lock_guard<std::mutex> lock(g_setup_mu);
         if (!attr[dev]) {
-            cudaError_t e = cudaFuncSetAttribute(k_conv_tc<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM);
+            cudaError_t e = cudaFuncSetAttribute(k_conv_tc<CIN, COUT, NT, ST, THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM);
             if (e != cudaSuccess) return e;
             attr[dev] = true;
         }
     }
-    k_conv_tc<CIN, COUT><<<nblk(a.d.np, kTileM), 128, S::SMEM, st>>>(a);
+    k_conv_tc<CIN, COUT, NT, ST, THREADS><<<dim3(nblk(a.d.np, kTileM), COUT / NT), THREADS, S::SMEM, st>>>(a);
     return cudaGetLastError();
+}
+
+// 16 output channels per CTA while the CTAs of all channels fit the SMs in one wave, else 32 under the
+// same condition, else the whole width.  On B200: 128 -> 128 channels on 5^3 and 9^3 nodes (3 and
+// 11 row tiles) 88 -> 59 us, 64 -> 64 on 9^3 37 -> 32 us; 64 -> 64 on 17^3 (54 tiles) takes 37 us whole, 35
+// with 32 channels and 61 with 16, whose 216 CTAs are two waves
+template <int CIN, int COUT>
+cudaError_t launch_conv_t(const ConvArgs &a, cudaStream_t st)
+{
+    const long tiles = nblk(a.d.np, kTileM);
+    if constexpr (COUT > 16 && CIN >= 32)
+        if (tiles * (COUT / 16) <= 148) return launch_conv_n<CIN, COUT, 16, 8, 256>(a, st);
+    if constexpr (COUT > 32 && CIN >= 32)
+        if (tiles * (COUT / 32) <= 148) return launch_conv_n<CIN, COUT, 32, 8, 256>(a, st);
+    return launch_conv_n<CIN, COUT, COUT, kStages, 128>(a, st);
 }
 
 // persistent grid of the brick kernel: every resident CTA on every SM, at most one per tile
@@ -1631,6 +1654,10 @@ struct i3g_unet {
     int *derr = nullptr;
     float *wpart = nullptr;                     // per-CTA weight-gradient sums of k_wgrad_tc
     int wpart_slots = 0;
+    // the weight gradients of the wide layers (CUDA cores) depend on a layer's input and output gradient
+    // alone: they run on a second stream beside the chain of input gradients
+    cudaStream_t st2 = nullptr;
+    cudaEvent_t ready[kLayers] = {}, joined = nullptr;
     Scales sc = {21.0f, 0.5f, 3300.0f, 0.01f, 1e-10f, 1e6f};
     int adam_t = 0;
 };
@@ -1704,8 +1731,13 @@ int backward(i3g_unet *u)
         const LayerDef &ld = kL[l];
         const int in = ld.in, out = ld.out;
         const Dims &d = u->L[kT[out].lev];
+        const bool beside = kT[in].ch > 32 || kT[out].ch > 32;
+        if (beside) {
+            UCHK(cudaEventRecord(u->ready[l], u->st));
+            UCHK(cudaStreamWaitEvent(u->st2, u->ready[l], 0));
+        }
         UCHK(launch_wgrad(kT[in].ch, kT[out].ch, u->act[in], u->grd[out], u->grad + u->woff[l], u->grad + u->boff[l], d,
-                          u->off[kT[out].lev], u->wpart, u->wpart_slots, u->derr, u->st));
+                          u->off[kT[out].lev], u->wpart, u->wpart_slots, u->derr, beside ? u->st2 : u->st));
         if (l == 0) break;
         ConvArgs a = conv_args(u, kT[out].lev);
         a.in = u->grd[out];
@@ -1730,6 +1762,9 @@ int backward(i3g_unet *u)
                                                                        kT[src].ch, f, c, 0.125f);
         }
     }
+    // the next pass overwrites the activations and gradients that the second stream reads
+    UCHK(cudaEventRecord(u->joined, u->st2));
+    UCHK(cudaStreamWaitEvent(u->st, u->joined, 0));
     return 0;
 }
 
@@ -1796,6 +1831,12 @@ int i3g_unet_create(int nx, int ny, int nz, int capacity, uint64_t seed, i3g_une
         return r;
     };
     if (cudaStreamCreateWithFlags(&u->st, cudaStreamNonBlocking) != cudaSuccess) return cleanup(fail_cuda(cudaGetLastError(), "stream"));
+    if (cudaStreamCreateWithFlags(&u->st2, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaEventCreateWithFlags(&u->joined, cudaEventDisableTiming) != cudaSuccess)
+        return cleanup(fail_cuda(cudaGetLastError(), "stream"));
+    for (int l = 0; l < kLayers; l++)
+        if (cudaEventCreateWithFlags(&u->ready[l], cudaEventDisableTiming) != cudaSuccess)
+            return cleanup(fail_cuda(cudaGetLastError(), "event"));
     for (int l = 0; l < kLevels; l++) {
         const int s = 1 << l;
         u->L[l] = make_dims((nz - 1) / s + 1, (nx - 1) / s + 1, (ny - 1) / s + 1);
@@ -1877,6 +1918,13 @@ void i3g_unet_destroy(i3g_unet *u)
 {
     if (!u) return;
     if (u->st) cudaStreamSynchronize(u->st);
+    if (u->st2) {
+        cudaStreamSynchronize(u->st2);
+        cudaStreamDestroy(u->st2);
+    }
+    for (int l = 0; l < kLayers; l++)
+        if (u->ready[l]) cudaEventDestroy(u->ready[l]);
+    if (u->joined) cudaEventDestroy(u->joined);
     cudaFree(u->par);
     cudaFree(u->grad);
     cudaFree(u->am);

@@ -5,8 +5,9 @@ import pytest
 
 import cases
 import oracle as O
+import unet_ref as U
 from conftest import golden
-from i3elvis_b200 import abi, config, lib, model
+from i3elvis_b200 import abi, config, lib, model, warmstart
 from i3elvis_b200.prn import ROCK_FIELDS
 from test_oracle_markers import marker_setup
 
@@ -192,3 +193,23 @@ def test_marker_rheology_reads_what_it_needs(exact):
     # strains grow by dt * strain rate, stored as FP32; viscosities pass through pow and exp
     np.testing.assert_allclose(a.f32["marke"], b.f32["marke"], rtol=2e-7, atol=0)
     np.testing.assert_allclose(a.f32["markv"], b.f32["markv"], rtol=2e-7)
+
+
+@pytest.mark.parametrize("cin,cout", [(32, 32), (32, 64), (64, 32), (64, 64), (64, 128), (128, 64), (128, 128)])
+@pytest.mark.parametrize("dims", [(1, 1, 1), (10, 11, 14), (15, 17, 19), (27, 25, 29)])
+def test_wide_convolutions_for_every_channel_split(dims, cin, cout):
+    """1, 20, 53 and 190 tiles of 128 rows: 16 or 32 output channels per block, or the whole width.
+    FP32 sums of 27 * cin <= 3456 products against FP64: relative error far below 27 cin 2^-24 = 2e-4;
+    2e-5 of the largest output, as a random-sign sum of that length keeps."""
+    rng = np.random.default_rng(cin * 1000 + cout)
+    x = U.bf16(rng.normal(size=dims + (cin,)))
+    w = U.bf16(rng.normal(0, 1 / np.sqrt(27 * cin), size=(27, cout, cin)))
+    b = rng.normal(0, 0.1, size=cout).astype(np.float32)
+    rows = np.pad(x, ((1, 1), (1, 1), (1, 1), (0, 0))).reshape(-1, cin)
+    out = warmstart.conv_host(cin, cout, dims, U.bf16_bits(rows), U.bf16_bits(w), b, None, relu=False)
+    got = out.reshape(dims[0] + 2, dims[1] + 2, dims[2] + 2, cout)
+    inner = got[1:-1, 1:-1, 1:-1].copy()
+    ref = U.conv3(x, w, b.astype(np.float64))
+    assert np.max(np.abs(inner - ref)) <= 2e-5 * np.max(np.abs(ref)) + 1e-6
+    got[1:-1, 1:-1, 1:-1] = 0
+    assert not np.any(got)   # halo rows are not written
