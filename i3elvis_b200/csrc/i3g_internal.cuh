@@ -104,6 +104,11 @@ struct Transfer1D {
     double *w0 = nullptr, *w1 = nullptr;
     int *gptr = nullptr, *gf = nullptr;
     double *gw = nullptr;
+    // compact FP32 form (stokes.cu, CtView): four fine indices from cs[c] with weights cw[c]; cv[f]
+    bool compact = false;
+    int *cs = nullptr;
+    float4 *cw = nullptr;
+    float2 *cv = nullptr;
 };
 
 // staggering kinds: 0 grid line, 1 mid-point, 2 cell centre, 3 grid line with |d| weights
@@ -119,6 +124,8 @@ struct Level {
                                        // bit 4 + v: partner of in-kernel boundary rows of v (BcList::na)
     Fields<double> d;
     Fields<float> s;                    // scaled FP32 copy for the mixed-precision solver
+    bool compact = false;               // FP32 transfers from and to the finer level in compact form
+    float *iws[4] = {nullptr, nullptr, nullptr, nullptr};   // 1 / sum of restriction weights
     BcList bcl[4];
     Transfer1D tr[3][4];               // to the next coarser level: axis x,y,z; staggering
     long scratch_n = 0;
