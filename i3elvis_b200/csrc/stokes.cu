@@ -657,16 +657,17 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 6 : 4) k_relax_p_bc(View
 // ------------------------------------------------------------------------------------
 // residual (gausmat4 residual pass, move3mg.c:3136-3157)
 // ------------------------------------------------------------------------------------
-template <typename T>
+// ZERO: a zero right-hand side, not read
+template <typename T, bool ZERO = false>
 __device__ __forceinline__ void residual_at(const View<T> &L, long n)
 {
     int i, j, k;
     node_ijk(L, n, i, j, k);
     const uint8_t b = L.bc[n];
-    if (row_exists(0, i, j, k, L.nx, L.ny, L.nz) && !(b & 1)) { T s = L.f0[n]; crow<T, true>(L, i, j, k, n, s); L.r0[n] = s; }
-    if (row_exists(1, i, j, k, L.nx, L.ny, L.nz) && !(b & 2)) { T s = L.f1[n]; xrow<T, true>(L, i, j, k, n, s); L.r1[n] = s; }
-    if (row_exists(2, i, j, k, L.nx, L.ny, L.nz) && !(b & 4)) { T s = L.f2[n]; yrow<T, true>(L, i, j, k, n, s); L.r2[n] = s; }
-    if (row_exists(3, i, j, k, L.nx, L.ny, L.nz) && !(b & 8)) { T s = L.f3[n]; zrow<T, true>(L, i, j, k, n, s); L.r3[n] = s; }
+    if (row_exists(0, i, j, k, L.nx, L.ny, L.nz) && !(b & 1)) { T s = ZERO ? T(0) : L.f0[n]; crow<T, true>(L, i, j, k, n, s); L.r0[n] = s; }
+    if (row_exists(1, i, j, k, L.nx, L.ny, L.nz) && !(b & 2)) { T s = ZERO ? T(0) : L.f1[n]; xrow<T, true>(L, i, j, k, n, s); L.r1[n] = s; }
+    if (row_exists(2, i, j, k, L.nx, L.ny, L.nz) && !(b & 4)) { T s = ZERO ? T(0) : L.f2[n]; yrow<T, true>(L, i, j, k, n, s); L.r2[n] = s; }
+    if (row_exists(3, i, j, k, L.nx, L.ny, L.nz) && !(b & 8)) { T s = ZERO ? T(0) : L.f3[n]; zrow<T, true>(L, i, j, k, n, s); L.r3[n] = s; }
 }
 
 template <typename T>
@@ -679,7 +680,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 1) k_residual(View<T
 }
 
 // residual of boundary rows with their original (unflattened) partner
-template <typename T>
+template <typename T, bool ZERO = false>
 __device__ __forceinline__ void bc_residual_at(const View<T> &L, int V, int t, const int *node, const int *onode,
                                                const int *ocomp, const double *ok)
 {
@@ -688,7 +689,7 @@ __device__ __forceinline__ void bc_residual_at(const View<T> &L, int V, int t, c
     T *f[4] = {L.f0, L.f1, L.f2, L.f3};
     T *r[4] = {L.r0, L.r1, L.r2, L.r3};
     const int nd = node[t];
-    T s = f[V][nd];
+    T s = ZERO ? T(0) : f[V][nd];
     s = A::sub(s, A::mul(T(1), u[V][nd]));
     if (onode[t] >= 0) s = A::sub(s, A::mul((T)(-ok[t]), u[ocomp[t]][onode[t]]));
     r[V][nd] = s;
@@ -714,7 +715,7 @@ struct BcDev4 {
 // (they write only boundary nodes, which the row threads skip, and read no residual).  One thread
 // computes the four rows of a node, which share most of their loads (one thread per row and
 // component took 25 % longer with a cold L2).
-template <typename T>
+template <typename T, bool ZERO>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 1) k_residual_bc(View<T> L, BcDev4 B, unsigned rowblocks)
 {
     pdl_enter();
@@ -722,7 +723,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 1) k_residual_bc(Vie
         int t = (int)(blockIdx.x - rowblocks) * (int)blockDim.x + (int)threadIdx.x;
         for (int v = 0; v < 4; v++) {
             if (t < B.b[v].n) {
-                bc_residual_at<T>(L, v, t, B.b[v].node, B.b[v].onode, B.b[v].ocomp, B.b[v].ok);
+                bc_residual_at<T, ZERO>(L, v, t, B.b[v].node, B.b[v].onode, B.b[v].ocomp, B.b[v].ok);
                 return;
             }
             t -= B.b[v].n;
@@ -731,7 +732,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 1) k_residual_bc(Vie
     }
     const long n = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (n >= L.nxy * L.nz) return;
-    residual_at<T>(L, n);
+    residual_at<T, ZERO>(L, n);
 }
 
 // ------------------------------------------------------------------------------------
@@ -2178,7 +2179,7 @@ static void residual_t(i3g_ctx *c, int l)
         long nb = 0;
         for (int v = 0; v < 4; v++) { B.b[v] = bcdev(L.bcl[v]); nb += L.bcl[v].n; }
         const unsigned rows = nblk(L.n);
-        LAUNCH(k_residual_bc<T>, rows + nblk(nb), 256, V, B, rows);
+        LAUNCH((k_residual_bc<T, false>), rows + nblk(nb), 256, V, B, rows);
         return;
     }
     LAUNCH(k_residual<T>, nblk(L.n), 256, V);
@@ -2733,6 +2734,8 @@ struct KrylovState {
     double *W = nullptr;     // work vector (4N)
     double *F0 = nullptr;    // zero right-hand side (4N)
     double *part = nullptr;  // partial dot products [blocks][kKryNq]
+    double *mx = nullptr;    // block maxima of |v| over the velocity rows of the newest basis vector
+    unsigned *done = nullptr;   // blocks of the running projection that have finished
     double *hdev = nullptr;  // [3][kKryNq]: first and second projection, squared norm; then 2 weights
     double *hhost = nullptr; // pinned mirror of hdev
     double *save = nullptr;  // FP64 preconditioner: level-0 solution and right-hand side set aside (8N)
@@ -2744,20 +2747,22 @@ struct KrylovState {
 
 static KrylovState *kry(i3g_ctx *c) { return (KrylovState *)c->kry; }
 
-// FP64 preconditioner input: the vector to precondition (in the residual arrays) becomes the
-// right-hand side of the correction system, zero on boundary rows, with a zero start
-__global__ void k_corr64_in(long n, const double *r0, const double *r1, const double *r2, const double *r3, double *f0,
-                            double *f1, double *f2, double *f3, double *u0, double *u1, double *u2, double *u3,
-                            const uint8_t *bc)
+// FP64 preconditioner input: v / D, the unscaled vector to precondition, becomes the right-hand side
+// of the correction system, zero on boundary rows, with a zero start.  d[0] = velocity-row weight,
+// d[1] = pressure-row weight (device, so that the captured steps stay valid when the weights change
+// between restarts)
+__global__ void k_kr_to_f64(long n, const double *v, double *f0, double *f1, double *f2, double *f3, double *u0, double *u1, double *u2,
+                            double *u3, const uint8_t *bc, const double *d)
 {
     pdl_enter();
     long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n) return;
+    const double dv = d[0], dp = d[1];
     const uint8_t b = bc[t];
-    f0[t] = (b & 1) ? 0.0 : r0[t];
-    f1[t] = (b & 2) ? 0.0 : r1[t];
-    f2[t] = (b & 4) ? 0.0 : r2[t];
-    f3[t] = (b & 8) ? 0.0 : r3[t];
+    f0[t] = (b & 1) ? 0.0 : v[t] / dp;
+    f1[t] = (b & 2) ? 0.0 : v[n + t] / dv;
+    f2[t] = (b & 4) ? 0.0 : v[2 * n + t] / dv;
+    f3[t] = (b & 8) ? 0.0 : v[3 * n + t] / dv;
     u0[t] = 0.0; u1[t] = 0.0; u2[t] = 0.0; u3[t] = 0.0;
 }
 
@@ -2769,25 +2774,44 @@ __global__ void k_kr_store64(long N, double *z, const double *e0, const double *
     z[t] = e0[t]; z[N + t] = e1[t]; z[2 * N + t] = e2[t]; z[3 * N + t] = e3[t];
 }
 
-// d[0] = velocity-row weight, d[1] = pressure-row weight (device, so that the captured steps
-// stay valid when the weights change between restarts)
-__global__ void k_kr_from_r(long N, const double *r0, const double *r1, const double *r2, const double *r3, double *v,
-                            const double *d)
+// largest of x over the block, in every thread
+__device__ __forceinline__ double block_max(double x)
 {
-    pdl_enter();
-    long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= N) return;
-    const double dv = d[0], dp = d[1];
-    v[t] = dp * r0[t]; v[N + t] = dv * r1[t]; v[2 * N + t] = dv * r2[t]; v[3 * N + t] = dv * r3[t];
+    __shared__ double sh[32];
+    for (int o = 16; o > 0; o >>= 1) x = fmax(x, __shfl_xor_sync(0xffffffffu, x, o));
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = x;
+    __syncthreads();
+    x = sh[0];
+    for (int w = 1; w < (int)(blockDim.x >> 5); w++) x = fmax(x, sh[w]);
+    return x;
 }
 
-__global__ void k_kr_to_r(long N, const double *v, double *r0, double *r1, double *r2, double *r3, const double *d)
+// FP32 preconditioner input: v / D scaled as k_scale and k_to_f32 do (largest momentum entry to
+// order one), boundary rows and the start 0.  mx: kKrBlocks partial maxima of |v| over the velocity
+// rows, left by the kernel that wrote v; every block reduces them (2.8 MB of L2 reads in all), which
+// saves writing v / D, three maximum passes over it and a launch for the scale.  With the projections'
+// own last block adding their partial sums a step has seven launches less: a solve on 61 x 37 x 53
+// nodes takes 58 instead of 61 ms on B200, on 129^3 4 % less.
+__global__ void __launch_bounds__(256) k_kr_to_f32(long n, const double *v, const double *mx, int nmx, double h, double er, float *f0,
+                                                   float *f1, float *f2, float *f3, float *u0, float *u1, float *u2, float *u3,
+                                                   const uint8_t *bc, const double *d, double *scale)
 {
     pdl_enter();
-    long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= N) return;
     const double dv = d[0], dp = d[1];
-    r0[t] = v[t] / dp; r1[t] = v[N + t] / dv; r2[t] = v[2 * N + t] / dv; r3[t] = v[3 * N + t] / dv;
+    double m = 0;
+    for (int i = threadIdx.x; i < nmx; i += blockDim.x) m = fmax(m, mx[i]);
+    m = block_max(m) / dv;
+    if (!(m > 0)) m = 1.0;
+    const double sv = m * h * h / er, sm = h * h / (er * sv), sc = h / sv;
+    if (blockIdx.x == 0 && threadIdx.x == 0) { scale[0] = sm; scale[1] = sc; scale[2] = er * sv / h; scale[3] = sv; }
+    for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long)gridDim.x * blockDim.x) {
+        const uint8_t b = bc[t];
+        f0[t] = (b & 1) ? 0.f : (float)(v[t] / dp * sc);
+        f1[t] = (b & 2) ? 0.f : (float)(v[n + t] / dv * sm);
+        f2[t] = (b & 4) ? 0.f : (float)(v[2 * n + t] / dv * sm);
+        f3[t] = (b & 8) ? 0.f : (float)(v[3 * n + t] / dv * sm);
+        u0[t] = 0.f; u1[t] = 0.f; u2[t] = 0.f; u3[t] = 0.f;
+    }
 }
 
 // z = scaled FP32 correction (the FP64 image of the V-cycle's result)
@@ -2802,27 +2826,30 @@ __global__ void k_kr_store(long N, double *z, const float *e0, const float *e1, 
 }
 
 // One classical Gram-Schmidt pass over the 4N-vector w and the basis v_0..v_{NV-1}, per element
-//   MODE 0: x = w;
+//   MODE 0: x = d r, the residual r_0..r_3 row-weighted, stored into w (the start of a restart);
 //   MODE 1: x = -d w with the stopping test's row weight of the element's component (pressure
 //           rows d[1], velocity rows d[0]), stored back into w (the residual -A z becomes D A z);
 //   MODE 2: x = w - sum_i h_i v_i, stored back into w (the first projection removed);
-// and the block partial sums of x . v_i (i < NV) and x . x (slot NV).  A grid of a few CTAs per
-// SM with two elements in flight per thread keeps HBM busy; the basis is read once per pass.
+// and the sums x . v_i (i < NV) and x . x (slot NV) in out: block partial sums, which the last block
+// to finish adds in a fixed order.  A grid of a few CTAs per SM with two elements in flight per
+// thread keeps HBM busy; the basis is read once per pass.
 constexpr int kKrBlocks = 4 * 148;
+struct KrIn { const double *r[4]; };
 template <int NV, int MODE>
 __global__ void __launch_bounds__(256) k_kr_proj(double *__restrict__ w, const double *__restrict__ V, long N, long n4,
-                                                 const double *__restrict__ h, const double *__restrict__ d,
-                                                 double *__restrict__ part)
+                                                 const double *__restrict__ h, const double *__restrict__ d, const KrIn r,
+                                                 double *part, double *__restrict__ out, unsigned *done)
 {
     pdl_enter();
     __shared__ double sh[NV + 1][8];
+    __shared__ bool last;
     double q[NV + 1];
 #pragma unroll
     for (int i = 0; i <= NV; i++) q[i] = 0;
     double hh[NV > 0 ? NV : 1];
 #pragma unroll
     for (int i = 0; i < NV; i++) hh[i] = MODE == 2 ? h[i] : 0.0;
-    const double dp = MODE == 1 ? -d[1] : 0.0, dv = MODE == 1 ? -d[0] : 0.0;
+    const double dp = MODE == 1 ? -d[1] : MODE == 0 ? d[1] : 0.0, dv = MODE == 1 ? -d[0] : MODE == 0 ? d[0] : 0.0;
     const long stride = (long)gridDim.x * blockDim.x;
     for (long t0 = (long)blockIdx.x * blockDim.x + threadIdx.x; t0 < n4; t0 += 2 * stride) {
         double x[2], v[2][NV > 0 ? NV : 1];
@@ -2831,7 +2858,12 @@ __global__ void __launch_bounds__(256) k_kr_proj(double *__restrict__ w, const d
         for (int u = 0; u < 2; u++) {
             const long t = t0 + u * stride;
             in[u] = t < n4;
-            x[u] = in[u] ? w[t] : 0.0;
+            if (MODE == 0) {
+                const int q = t < N ? 0 : t < 2 * N ? 1 : t < 3 * N ? 2 : 3;
+                x[u] = in[u] ? r.r[q][t - q * N] : 0.0;
+            } else {
+                x[u] = in[u] ? w[t] : 0.0;
+            }
 #pragma unroll
             for (int i = 0; i < NV; i++) v[u][i] = in[u] ? __ldg(V + i * n4 + t) : 0.0;
         }
@@ -2839,11 +2871,11 @@ __global__ void __launch_bounds__(256) k_kr_proj(double *__restrict__ w, const d
         for (int u = 0; u < 2; u++) {
             const long t = t0 + u * stride;
             double y = x[u];
-            if (MODE == 1) y *= t < N ? dp : dv;
+            if (MODE != 2) y *= t < N ? dp : dv;
             if (MODE == 2)
 #pragma unroll
                 for (int i = 0; i < NV; i++) y -= hh[i] * v[u][i];
-            if (MODE != 0 && in[u]) w[t] = y;
+            if (in[u]) w[t] = y;
 #pragma unroll
             for (int i = 0; i < NV; i++) q[i] += y * v[u][i];
             q[NV] += y * y;
@@ -2860,42 +2892,56 @@ __global__ void __launch_bounds__(256) k_kr_proj(double *__restrict__ w, const d
         double r = 0;
         for (int a = 0; a < 8; a++) r += sh[threadIdx.x][a];
         part[(long)blockIdx.x * kKryNq + threadIdx.x] = r;
+        __threadfence();
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicInc(done, gridDim.x - 1) == gridDim.x - 1;   // back to 0 after the last
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    for (int i = wi; i <= NV; i += 8) {
+        double r = 0;
+        for (int b = ln; b < (int)gridDim.x; b += 32) r += __ldcg(part + (long)b * kKryNq + i);
+        r = warp_sum(r);
+        if (ln == 0) out[i] = r;
     }
 }
 
-__global__ void k_kr_dot_final(const double *part, int nblk, int nq, double *out)
+// v = (w - sum_i h_i v_i) / |.|, the squared norm taken as w.w - sum_i h_i^2 (hw[NV] = w.w from
+// the projection pass; v_0..v_{NV-1} are orthonormal; NV = 0: v = w / |w|), and the block maxima of
+// |v| over the velocity rows for the next step's scale
+template <int NV>
+__global__ void __launch_bounds__(256) k_kr_normalize(double *v, const double *w, const double *__restrict__ V, long N, long n4,
+                                                      const double *__restrict__ hw, double *mx)
 {
     pdl_enter();
-    const int qi = threadIdx.x >> 5, ln = threadIdx.x & 31;
-    if (qi >= nq) return;
-    double v = 0;
-    for (int b = ln; b < nblk; b += 32) v += part[(long)b * kKryNq + qi];
-    v = warp_sum(v);
-    if (ln == 0) out[qi] = v;
-}
-
-
-// v = (w - sum_i h_i v_i) / |.|, the squared norm taken as w.w - sum_i h_i^2 (hw[nv] = w.w from
-// the projection pass; v_0..v_{nv-1} are orthonormal)
-__global__ void k_kr_axpy_normalize(double *v, const double *w, const double *V, int nv, long n4, const double *hw)
-{
-    pdl_enter();
-    long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n4) return;
-    double nrm2 = hw[nv];
-    for (int i = 0; i < nv; i++) nrm2 -= hw[i] * hw[i];
-    double x = w[t];
-    for (int i = 0; i < nv; i++) x -= hw[i] * V[i * n4 + t];
-    v[t] = x / sqrt(nrm2);
-}
-
-// v = w / sqrt(nrm2)
-__global__ void k_kr_normalize(long n4, const double *w, double *v, const double *nrm2)
-{
-    pdl_enter();
-    long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n4) return;
-    v[t] = w[t] / sqrt(*nrm2);
+    double hh[NV > 0 ? NV : 1], nrm2 = hw[NV], m = 0;
+#pragma unroll
+    for (int i = 0; i < NV; i++) { hh[i] = hw[i]; nrm2 -= hh[i] * hh[i]; }
+    const double nrm = sqrt(nrm2);
+    const long stride = (long)gridDim.x * blockDim.x;
+    for (long t0 = (long)blockIdx.x * blockDim.x + threadIdx.x; t0 < n4; t0 += 2 * stride) {
+        double x[2], q[2][NV > 0 ? NV : 1];
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const long t = t0 + u * stride;
+            x[u] = t < n4 ? w[t] : 0.0;
+#pragma unroll
+            for (int i = 0; i < NV; i++) q[u][i] = t < n4 ? __ldg(V + i * n4 + t) : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const long t = t0 + u * stride;
+            double y = x[u];
+#pragma unroll
+            for (int i = 0; i < NV; i++) y -= hh[i] * q[u][i];
+            y /= nrm;
+            if (t < n4) v[t] = y;
+            if (t >= N && t < n4) m = fmax(m, fabs(y));
+        }
+    }
+    m = block_max(m);
+    if (threadIdx.x == 0) mx[blockIdx.x] = m;
 }
 
 struct KrY { double y[kKryMax]; };
@@ -2967,25 +3013,36 @@ __global__ void __launch_bounds__(256) k_guess_dots(View<double> L, const double
 // k_kr_proj<nv, mode> for a run-time basis size nv <= kKryMax
 template <int MODE>
 static void kr_proj_launch(i3g_ctx *c, int nv, double *w, const double *V, long N, long n4, const double *h, const double *d,
-                           double *part)
+                           double *part, double *out, unsigned *done)
 {
     switch (nv) {
-#define KR_CASE(k) case k: LAUNCH((k_kr_proj<k, MODE>), kKrBlocks, 256, w, V, N, n4, h, d, part); break;
-    KR_CASE(0) KR_CASE(1) KR_CASE(2) KR_CASE(3) KR_CASE(4) KR_CASE(5) KR_CASE(6) KR_CASE(7) KR_CASE(8)
+#define KR_CASE(k) case k: LAUNCH((k_kr_proj<k, MODE>), kKrBlocks, 256, w, V, N, n4, h, d, KrIn{}, part, out, done); break;
+    KR_CASE(1) KR_CASE(2) KR_CASE(3) KR_CASE(4) KR_CASE(5) KR_CASE(6) KR_CASE(7) KR_CASE(8)
     KR_CASE(9) KR_CASE(10) KR_CASE(11) KR_CASE(12) KR_CASE(13) KR_CASE(14) KR_CASE(15) KR_CASE(16)
 #undef KR_CASE
     default: break;
     }
 }
 
-static int kr_proj(i3g_ctx *c, int nv, int mode, double *w, long N, long n4, const double *h, const double *d, double *part)
+static int kr_proj(i3g_ctx *c, int nv, int mode, double *w, long N, long n4, const double *h, const double *d, double *out)
 {
-    if (nv < 0 || nv > kKryMax) return set_error(c, I3G_E_ARG, "Krylov basis of %d vectors above %d", nv, kKryMax);
-    const double *V = kry(c)->V;
-    if (mode == 0) kr_proj_launch<0>(c, nv, w, V, N, n4, h, d, part);
-    else if (mode == 1) kr_proj_launch<1>(c, nv, w, V, N, n4, h, d, part);
-    else kr_proj_launch<2>(c, nv, w, V, N, n4, h, d, part);
+    if (nv < 1 || nv > kKryMax) return set_error(c, I3G_E_ARG, "Krylov basis of %d vectors above %d", nv, kKryMax);
+    KrylovState *K = kry(c);
+    if (mode == 1) kr_proj_launch<1>(c, nv, w, K->V, N, n4, h, d, K->part, out, K->done);
+    else kr_proj_launch<2>(c, nv, w, K->V, N, n4, h, d, K->part, out, K->done);
     return 0;
+}
+
+static void kr_normalize(i3g_ctx *c, int nv, double *v, const double *w, long N, long n4, const double *hw)
+{
+    KrylovState *K = kry(c);
+    switch (nv) {
+#define KR_CASE(k) case k: LAUNCH((k_kr_normalize<k>), kKrBlocks, 256, v, w, (const double *)K->V, N, n4, hw, K->mx); break;
+    KR_CASE(0) KR_CASE(1) KR_CASE(2) KR_CASE(3) KR_CASE(4) KR_CASE(5) KR_CASE(6) KR_CASE(7) KR_CASE(8)
+    KR_CASE(9) KR_CASE(10) KR_CASE(11) KR_CASE(12) KR_CASE(13) KR_CASE(14) KR_CASE(15) KR_CASE(16)
+#undef KR_CASE
+    default: break;
+    }
 }
 
 static int kry_alloc(i3g_ctx *c, int m)
@@ -3003,6 +3060,9 @@ static int kry_alloc(i3g_ctx *c, int m)
     ALLOC(K->W, double, n4);
     ALLOC(K->F0, double, n4);
     ALLOC(K->part, double, (long)kKrBlocks * kKryNq);
+    ALLOC(K->mx, double, kKrBlocks);
+    ALLOC(K->done, unsigned, 1);
+    I3G_CUDA(cudaMemsetAsync(K->done, 0, sizeof(unsigned), c->st));
     ALLOC(K->hdev, double, 3 * kKryNq + 2);
     if (c->p.precision == 0) ALLOC(K->save, double, 2 * n4);
     I3G_CUDA(cudaMallocHost((void **)&K->hhost, (3 * kKryNq + 2) * sizeof(double)));
@@ -3016,7 +3076,8 @@ static void kry_free(i3g_ctx *c)
     KrylovState *K = kry(c);
     if (!K) return;
     for (int j = 0; j < kKryMax; j++) if (K->g[j]) cudaGraphExecDestroy(K->g[j]);
-    cudaFree(K->V); cudaFree(K->Z); cudaFree(K->W); cudaFree(K->F0); cudaFree(K->part); cudaFree(K->hdev);
+    cudaFree(K->V); cudaFree(K->Z); cudaFree(K->W); cudaFree(K->F0); cudaFree(K->part); cudaFree(K->mx); cudaFree(K->done);
+    cudaFree(K->hdev);
     cudaFree(K->save);
     cudaFreeHost(K->hhost);
     delete K;
@@ -3044,8 +3105,6 @@ static int kry_enqueue_step(i3g_ctx *c, int j, int multinum)
     double *vj = K->V + (long)j * n4, *zj = K->Z + (long)j * n4;
     // preconditioner: the V-cycle of this precision on the unscaled vector
     const double *d = K->hdev + 3 * kKryNq;
-    LAUNCH(k_kr_to_r, nblk(N), 256, N, (const double *)vj, L0.d.r[0], L0.d.r[1], L0.d.r[2], L0.d.r[3], d);
-    const int nb = c->red_blocks;
     if (c->p.precision == 0) {
         // FP64 V-cycle from zero on level 0's own arrays, whose solution and right-hand side
         // are set aside meanwhile (no scaling: the system is already FP64)
@@ -3053,9 +3112,8 @@ static int kry_enqueue_step(i3g_ctx *c, int j, int multinum)
             I3G_CUDA(cudaMemcpyAsync(K->save + v * N, L0.d.u[v], N * 8, cudaMemcpyDeviceToDevice, c->st));
             I3G_CUDA(cudaMemcpyAsync(K->save + (4 + v) * N, L0.d.f[v], N * 8, cudaMemcpyDeviceToDevice, c->st));
         }
-        LAUNCH(k_corr64_in, nblk(N), 256, N, (const double *)L0.d.r[0], (const double *)L0.d.r[1],
-               (const double *)L0.d.r[2], (const double *)L0.d.r[3], L0.d.f[0], L0.d.f[1], L0.d.f[2], L0.d.f[3],
-               L0.d.u[0], L0.d.u[1], L0.d.u[2], L0.d.u[3], (const uint8_t *)L0.bc);
+        LAUNCH(k_kr_to_f64, nblk(N), 256, N, (const double *)vj, L0.d.f[0], L0.d.f[1], L0.d.f[2], L0.d.f[3],
+               L0.d.u[0], L0.d.u[1], L0.d.u[2], L0.d.u[3], (const uint8_t *)L0.bc, d);
         vcycle_t<double>(c, multinum, true);
         LAUNCH(k_kr_store64, nblk(N), 256, N, zj, (const double *)L0.d.u[0], (const double *)L0.d.u[1],
                (const double *)L0.d.u[2], (const double *)L0.d.u[3]);
@@ -3064,13 +3122,9 @@ static int kry_enqueue_step(i3g_ctx *c, int j, int multinum)
             I3G_CUDA(cudaMemcpyAsync(L0.d.f[v], K->save + (4 + v) * N, N * 8, cudaMemcpyDeviceToDevice, c->st));
         }
     } else {
-        LAUNCH(k_max_abs, nb, 256, (const double *)L0.d.r[1], N, c->dred);
-        LAUNCH(k_max_abs, nb, 256, (const double *)L0.d.r[2], N, c->dred + nb);
-        LAUNCH(k_max_abs, nb, 256, (const double *)L0.d.r[3], N, c->dred + 2 * nb);
-        LAUNCH(k_scale, 1, 1024, (const double *)c->dred, 3 * nb, c->h_ref, c->eta_ref, c->dscale);
-        LAUNCH(k_to_f32, nblk(N), 256, N, (const double *)L0.d.r[0], (const double *)L0.d.r[1],
-               (const double *)L0.d.r[2], (const double *)L0.d.r[3], L0.s.f[0], L0.s.f[1], L0.s.f[2], L0.s.f[3],
-               L0.s.u[0], L0.s.u[1], L0.s.u[2], L0.s.u[3], (const uint8_t *)L0.bc, (const double *)c->dscale);
+        LAUNCH(k_kr_to_f32, std::min(nblk(N), (unsigned)kKrBlocks), 256, N, (const double *)vj, (const double *)K->mx, kKrBlocks, c->h_ref,
+               c->eta_ref, L0.s.f[0], L0.s.f[1], L0.s.f[2], L0.s.f[3], L0.s.u[0], L0.s.u[1], L0.s.u[2], L0.s.u[3],
+               (const uint8_t *)L0.bc, d, c->dscale);
         vcycle_t<float>(c, multinum, true);
         LAUNCH(k_kr_store, nblk(N), 256, N, zj, (const float *)L0.s.u[0], (const float *)L0.s.u[1],
                (const float *)L0.s.u[2], (const float *)L0.s.u[3], (const double *)c->dscale);
@@ -3084,7 +3138,7 @@ static int kry_enqueue_step(i3g_ctx *c, int j, int multinum)
         BcDev4 B;
         long nb = 0;
         for (int v = 0; v < 4; v++) { B.b[v] = bcdev(L0.bcl[v]); nb += L0.bcl[v].n; }
-        LAUNCH(k_residual_bc<double>, nblk(N) + nblk(nb), 256, Vz, B, nblk(N));
+        LAUNCH((k_residual_bc<double, true>), nblk(N) + nblk(nb), 256, Vz, B, nblk(N));
     } else {
         LAUNCH(k_residual<double>, nblk(N), 256, Vz);
         for (int v = 0; v < 4; v++) {
@@ -3097,12 +3151,9 @@ static int kry_enqueue_step(i3g_ctx *c, int j, int multinum)
     // second subtracts the first projection while it forms the second one and w.w, from which the
     // last kernel takes the norm while it subtracts the second projection and normalises
     double *h1 = K->hdev, *h2 = K->hdev + kKryNq;
-    if (int rc = kr_proj(c, j + 1, 1, K->W, N, n4, nullptr, d, K->part)) return rc;
-    LAUNCH(k_kr_dot_final, 1, 32 * (j + 2), (const double *)K->part, kKrBlocks, j + 2, h1);
-    if (int rc = kr_proj(c, j + 1, 2, K->W, N, n4, h1, d, K->part)) return rc;
-    LAUNCH(k_kr_dot_final, 1, 32 * (j + 2), (const double *)K->part, kKrBlocks, j + 2, h2);
-    LAUNCH(k_kr_axpy_normalize, nblk(n4), 256, K->V + (long)(j + 1) * n4, (const double *)K->W, (const double *)K->V,
-           j + 1, n4, (const double *)h2);
+    if (int rc = kr_proj(c, j + 1, 1, K->W, N, n4, nullptr, d, h1)) return rc;
+    if (int rc = kr_proj(c, j + 1, 2, K->W, N, n4, h1, d, h2)) return rc;
+    kr_normalize(c, j + 1, K->V + (long)(j + 1) * n4, K->W, N, n4, h2);
     I3G_CUDA(cudaMemcpyAsync(K->hhost, K->hdev, 2 * kKryNq * sizeof(double), cudaMemcpyDeviceToHost, c->st));
     return 0;
 }
@@ -3150,13 +3201,11 @@ static int kry_cycle(i3g_ctx *c, int multinum, double rtol, int maxsteps, int *s
     I3G_CUDA(cudaMemcpyAsync(K->hdev + 3 * kKryNq, K->hhost + 3 * kKryNq, 2 * sizeof(double), cudaMemcpyHostToDevice, c->st));
     const double *d = K->hdev + 3 * kKryNq;
     residual_t<double>(c, 0);
-    LAUNCH(k_kr_from_r, nblk(N), 256, N, (const double *)L0.d.r[0], (const double *)L0.d.r[1],
-           (const double *)L0.d.r[2], (const double *)L0.d.r[3], K->V, d);
     double *nrm = K->hdev + 2 * kKryNq;
-    if (int rc = kr_proj(c, 0, 0, K->V, N, n4, nullptr, d, K->part)) return rc;
-    LAUNCH(k_kr_dot_final, 1, 32, (const double *)K->part, kKrBlocks, 1, nrm);
+    LAUNCH((k_kr_proj<0, 0>), kKrBlocks, 256, K->V, (const double *)K->V, N, n4, (const double *)nullptr, d,
+           KrIn{{L0.d.r[0], L0.d.r[1], L0.d.r[2], L0.d.r[3]}}, K->part, nrm, K->done);
     I3G_CUDA(cudaMemcpyAsync(K->hhost + 2 * kKryNq, nrm, sizeof(double), cudaMemcpyDeviceToHost, c->st));
-    LAUNCH(k_kr_normalize, nblk(n4), 256, n4, (const double *)K->V, K->V, (const double *)nrm);
+    kr_normalize(c, 0, K->V, K->V, N, n4, nrm);
     I3G_CUDA(cudaStreamSynchronize(c->st));
     const double beta = std::sqrt(K->hhost[2 * kKryNq]);
     if (!(beta > 0)) return 0;
