@@ -1265,6 +1265,11 @@ struct EtaArgs {
     double nubeg, nuend;
     double *etac, *etaxy, *etaxz, *etayz;
     float *nd;
+    // scaled FP32 copies of the operator data, and the 12 solution, right-hand-side and residual
+    // arrays, which start a solve at zero
+    float *fc, *fxy, *fxz, *fyz, *fnd;
+    double inv_ref;
+    double *zero[12];
 };
 
 __device__ __forceinline__ double avg8(const float *nu, long v0, long NY, long NXY, int viscmod)
@@ -1336,20 +1341,13 @@ __global__ void k_eta(EtaArgs a)
     }
     a.etac[n] = ec; a.etaxy[n] = exy; a.etaxz[n] = exz; a.etayz[n] = eyz;
     a.nd[n] = (float)ec;
-}
-
-// scaled FP32 copies of the level operator data
-__global__ void k_eta_f32(long n, const double *ec, const double *exy, const double *exz, const double *eyz,
-                          const float *nd, float *fc, float *fxy, float *fxz, float *fyz, float *fnd, double inv_ref)
-{
-    pdl_enter();
-    long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n) return;
-    fc[t] = (float)(ec[t] * inv_ref);
-    fxy[t] = (float)(exy[t] * inv_ref);
-    fxz[t] = (float)(exz[t] * inv_ref);
-    fyz[t] = (float)(eyz[t] * inv_ref);
-    fnd[t] = (float)((double)nd[t] * inv_ref);
+    a.fc[n] = (float)(ec * a.inv_ref);
+    a.fxy[n] = (float)(exy * a.inv_ref);
+    a.fxz[n] = (float)(exz * a.inv_ref);
+    a.fyz[n] = (float)(eyz * a.inv_ref);
+    a.fnd[n] = (float)((double)(float)ec * a.inv_ref);
+#pragma unroll
+    for (int q = 0; q < 12; q++) a.zero[q][n] = 0.0;
 }
 
 // Pressure-update scale of the FP32 preconditioner's smoother.  The reference scales a cell's
@@ -2105,16 +2103,12 @@ int stokes_setup(i3g_ctx *c)
         a.nubeg = c->p.nubeg; a.nuend = c->p.nuend;
         a.etac = L.d.etac; a.etaxy = L.d.etaxy; a.etaxz = L.d.etaxz; a.etayz = L.d.etayz;
         a.nd = L.d.nd;
+        a.fc = L.s.etac; a.fxy = L.s.etaxy; a.fxz = L.s.etaxz; a.fyz = L.s.etayz; a.fnd = L.s.nd;
+        a.inv_ref = 1.0 / c->eta_ref;
+        for (int v = 0; v < 4; v++) { a.zero[v] = L.d.u[v]; a.zero[4 + v] = L.d.f[v]; a.zero[8 + v] = L.d.r[v]; }
         LAUNCH(k_eta, nblk(L.n), 256, a);
-        LAUNCH(k_eta_f32, nblk(L.n), 256, L.n, L.d.etac, L.d.etaxy, L.d.etaxz, L.d.etayz, (const float *)a.nd,
-               L.s.etac, L.s.etaxy, L.s.etaxz, L.s.etayz, L.s.nd, 1.0 / c->eta_ref);
         if (c->nd_schur > 0)
             LAUNCH(k_nd_schur, nblk(L.n), 256, view<double>(L, L.d), L.s.nd, 1.0 / c->eta_ref, (double)c->nd_schur);
-        for (int v = 0; v < 4; v++) {
-            I3G_CUDA(cudaMemsetAsync(L.d.u[v], 0, L.n * 8, c->st));
-            I3G_CUDA(cudaMemsetAsync(L.d.f[v], 0, L.n * 8, c->st));
-            I3G_CUDA(cudaMemsetAsync(L.d.r[v], 0, L.n * 8, c->st));
-        }
     }
     View<double> V0 = view<double>(L0, L0.d);
     LAUNCH(k_rhs0, nblk(L0.n), 256, V0, (const float *)c->ro, c->m.gxkoef, c->m.gykoef, c->m.gzkoef);
