@@ -115,6 +115,15 @@ struct Transfer1D {
 // (viscosity restriction)
 constexpr int kStagLine = 0, kStagMid = 1, kStagCell = 2, kStagAbs = 3;
 
+// Boundary rows of a level for the on-chip tail (stokes.cu, build_smtail).
+struct SmTailRows {
+    bool ok = false;
+    int nent = 0, cptr[5] = {};
+    unsigned *ent = nullptr;
+    uint16_t *first = nullptr;
+    int *cst = nullptr;
+};
+
 struct Level {
     int nx = 0, ny = 0, nz = 0;
     long n = 0;
@@ -124,6 +133,7 @@ struct Level {
                                        // bit 4 + v: partner of in-kernel boundary rows of v (BcList::na)
     Fields<double> d;
     Fields<float> s;                    // scaled FP32 copy for the mixed-precision solver
+    SmTailRows sm;
     bool compact = false;               // FP32 transfers from and to the finer level in compact form
     float *iws[4] = {nullptr, nullptr, nullptr, nullptr};   // 1 / sum of restriction weights
     BcList bcl[4];
@@ -197,6 +207,7 @@ struct i3g_ctx {
     int fuse = 1;                               // boundary rows inside the relaxation kernels of levels >= 1
                                                 // (3: level 0 too), residual and four-component transfer
                                                 // launches (0: one launch per pass)
+    bool smtail = false;                        // coarsest levels of a V-cycle in shared memory
     long pro_nodes = 0;                         // largest level whose relaxations start before their predecessor ends
     int coop_blocks = 0;                        // its grid: every CTA resident at once (0: no cooperative launch)
     unsigned *dbar = nullptr;                   // its grid barrier: arrival count, generation

@@ -82,9 +82,12 @@ struct View {
     const float *nd;
 };
 
+// The row functions take any view VW with View's members: the global arrays (View), or the
+// shared-memory copies of the coarse tail (SmView).
+
 // (i, j, k) of node n = (k * nx + i) * ny + j of a level (n < 2^31)
-template <typename T>
-__device__ __forceinline__ void node_ijk(const View<T> &L, long n, int &i, int &j, int &k)
+template <class VW>
+__device__ __forceinline__ void node_ijk(const VW &L, long n, int &i, int &j, int &k)
 {
     const unsigned u = (unsigned)n;
     const unsigned r = L.dny.div(u);
@@ -146,8 +149,8 @@ struct Row {
 
 // x-momentum row at node n = (i,j,k) (xstokserr, move3mg.c:718-903): c = A, B, Sy, Ny, Fz, Kz, Sx,
 // Nx, Fx, Kx
-template <typename T>
-__device__ __forceinline__ Row<T> xcoef(const View<T> &L, int i, int j, int k, long n)
+template <typename T, class VW>
+__device__ __forceinline__ Row<T> xcoef(const VW &L, int i, int j, int k, long n)
 {
     using A = Ar<T>;
     const long NY = L.ny, NXY = L.nxy;
@@ -170,11 +173,11 @@ __device__ __forceinline__ Row<T> xcoef(const View<T> &L, int i, int j, int k, l
 }
 
 // accumulates the row's 17 slots in the reference's order into s
-template <typename T, bool RES>
-__device__ __forceinline__ void xsum(const View<T> &L, const Row<T> &R, long n, T &s)
+template <typename T, bool RES, class VW>
+__device__ __forceinline__ void xsum(const VW &L, const Row<T> &R, long n, T &s)
 {
     const long NY = L.ny, NXY = L.nxy;
-    const T *vx = L.u1, *vy = L.u2, *vz = L.u3, *p = L.u0;
+    const auto &vx = L.u1, &vy = L.u2, &vz = L.u3, &p = L.u0;
     acc<T, RES>(s, R.d, vx[n]);
     acc<T, RES>(s, R.c[0], vx[n - NY]);
     acc<T, RES>(s, R.c[1], vx[n + NY]);
@@ -195,8 +198,8 @@ __device__ __forceinline__ void xsum(const View<T> &L, const Row<T> &R, long n, 
 }
 
 // y-momentum row (ystokserr, move3mg.c:910-1101): c = A, B, Wx, Ex, Fz, Kz, Wy, Ey, Fy, Ky
-template <typename T>
-__device__ __forceinline__ Row<T> ycoef(const View<T> &L, int i, int j, int k, long n)
+template <typename T, class VW>
+__device__ __forceinline__ Row<T> ycoef(const VW &L, int i, int j, int k, long n)
 {
     using A = Ar<T>;
     const long NY = L.ny, NXY = L.nxy;
@@ -218,11 +221,11 @@ __device__ __forceinline__ Row<T> ycoef(const View<T> &L, int i, int j, int k, l
     return R;
 }
 
-template <typename T, bool RES>
-__device__ __forceinline__ void ysum(const View<T> &L, const Row<T> &R, long n, T &s)
+template <typename T, bool RES, class VW>
+__device__ __forceinline__ void ysum(const VW &L, const Row<T> &R, long n, T &s)
 {
     const long NY = L.ny, NXY = L.nxy;
-    const T *vx = L.u1, *vy = L.u2, *vz = L.u3, *p = L.u0;
+    const auto &vx = L.u1, &vy = L.u2, &vz = L.u3, &p = L.u0;
     acc<T, RES>(s, R.d, vy[n]);
     acc<T, RES>(s, R.c[2], vy[n - NY]);
     acc<T, RES>(s, R.c[3], vy[n + NY]);
@@ -243,8 +246,8 @@ __device__ __forceinline__ void ysum(const View<T> &L, const Row<T> &R, long n, 
 }
 
 // z-momentum row (zstokserr, move3mg.c:1109-1301): c = A, B, Wx, Ex, Sy, Ny, Wz, Ez, Sz, Nz
-template <typename T>
-__device__ __forceinline__ Row<T> zcoef(const View<T> &L, int i, int j, int k, long n)
+template <typename T, class VW>
+__device__ __forceinline__ Row<T> zcoef(const VW &L, int i, int j, int k, long n)
 {
     using A = Ar<T>;
     const long NY = L.ny, NXY = L.nxy;
@@ -266,11 +269,11 @@ __device__ __forceinline__ Row<T> zcoef(const View<T> &L, int i, int j, int k, l
     return R;
 }
 
-template <typename T, bool RES>
-__device__ __forceinline__ void zsum(const View<T> &L, const Row<T> &R, long n, T &s)
+template <typename T, bool RES, class VW>
+__device__ __forceinline__ void zsum(const VW &L, const Row<T> &R, long n, T &s)
 {
     const long NY = L.ny, NXY = L.nxy;
-    const T *vx = L.u1, *vy = L.u2, *vz = L.u3, *p = L.u0;
+    const auto &vx = L.u1, &vy = L.u2, &vz = L.u3, &p = L.u0;
     acc<T, RES>(s, R.d, vz[n]);
     acc<T, RES>(s, R.c[2], vz[n - NY]);
     acc<T, RES>(s, R.c[3], vz[n + NY]);
@@ -291,31 +294,31 @@ __device__ __forceinline__ void zsum(const View<T> &L, const Row<T> &R, long n, 
 }
 
 // a whole row: accumulates it into s and returns the diagonal
-template <typename T, bool RES>
-__device__ __forceinline__ T xrow(const View<T> &L, int i, int j, int k, long n, T &s)
+template <typename T, bool RES, class VW>
+__device__ __forceinline__ T xrow(const VW &L, int i, int j, int k, long n, T &s)
 {
-    const Row<T> R = xcoef(L, i, j, k, n);
+    const Row<T> R = xcoef<T>(L, i, j, k, n);
     xsum<T, RES>(L, R, n, s);
     return R.d;
 }
-template <typename T, bool RES>
-__device__ __forceinline__ T yrow(const View<T> &L, int i, int j, int k, long n, T &s)
+template <typename T, bool RES, class VW>
+__device__ __forceinline__ T yrow(const VW &L, int i, int j, int k, long n, T &s)
 {
-    const Row<T> R = ycoef(L, i, j, k, n);
+    const Row<T> R = ycoef<T>(L, i, j, k, n);
     ysum<T, RES>(L, R, n, s);
     return R.d;
 }
-template <typename T, bool RES>
-__device__ __forceinline__ T zrow(const View<T> &L, int i, int j, int k, long n, T &s)
+template <typename T, bool RES, class VW>
+__device__ __forceinline__ T zrow(const VW &L, int i, int j, int k, long n, T &s)
 {
-    const Row<T> R = zcoef(L, i, j, k, n);
+    const Row<T> R = zcoef<T>(L, i, j, k, n);
     zsum<T, RES>(L, R, n, s);
     return R.d;
 }
 
 // continuity row of the cell with upper corner n = (i,j,k) (continerr, move3mg.c:1310-1425)
-template <typename T, bool RES>
-__device__ __forceinline__ void csum(const View<T> &L, T xk, T yk, T zk, long n, T &s)
+template <typename T, bool RES, class VW>
+__device__ __forceinline__ void csum(const VW &L, T xk, T yk, T zk, long n, T &s)
 {
     const long NY = L.ny, NXY = L.nxy;
     const long v0 = n - NXY - NY - 1;
@@ -326,8 +329,8 @@ __device__ __forceinline__ void csum(const View<T> &L, T xk, T yk, T zk, long n,
     acc<T, RES>(s, -zk, L.u3[v0]);
     acc<T, RES>(s, zk, L.u3[v0 + NXY]);
 }
-template <typename T, bool RES>
-__device__ __forceinline__ void crow(const View<T> &L, int i, int j, int k, long n, T &s)
+template <typename T, bool RES, class VW>
+__device__ __forceinline__ void crow(const VW &L, int i, int j, int k, long n, T &s)
 {
     csum<T, RES>(L, L.icx[i], L.icy[j], L.icz[k], n, s);
 }
@@ -339,8 +342,8 @@ __device__ __forceinline__ void crow(const View<T> &L, int i, int j, int k, long
 // y-pair (2*jh, 2*jh+1) of line (i,k), so a warp covers 64 consecutive y.
 // Node of thread t's row of colour `color` (the y-pair (2*jh, 2*jh+1) of line (i,k)); -1 when
 // the row does not exist.
-template <int V, typename T>
-__device__ __forceinline__ long vel_row_node(const View<T> &L, long t, int color, int &i, int &j, int &k)
+template <int V, class VW>
+__device__ __forceinline__ long vel_row_node(const VW &L, long t, int color, int &i, int &j, int &k)
 {
     const unsigned hy = (unsigned)((L.ny + 1) >> 1), u = (unsigned)t;
     const unsigned rest = L.dhy.div(u);
@@ -352,15 +355,15 @@ __device__ __forceinline__ long vel_row_node(const View<T> &L, long t, int color
     return (long)k * L.nxy + (long)i * L.ny + j;
 }
 
-template <typename T, int V>
-__device__ __forceinline__ Row<T> vcoef(const View<T> &L, int i, int j, int k, long n)
+template <typename T, int V, class VW>
+__device__ __forceinline__ Row<T> vcoef(const VW &L, int i, int j, int k, long n)
 {
-    return V == 1 ? xcoef(L, i, j, k, n) : V == 2 ? ycoef(L, i, j, k, n) : zcoef(L, i, j, k, n);
+    return V == 1 ? xcoef<T>(L, i, j, k, n) : V == 2 ? ycoef<T>(L, i, j, k, n) : zcoef<T>(L, i, j, k, n);
 }
 
 // the value the relaxation gives velocity row n of coefficients R
-template <typename T, int V>
-__device__ __forceinline__ T relaxed(const View<T> &L, const Row<T> &R, long n, T koef)
+template <typename T, int V, class VW>
+__device__ __forceinline__ T relaxed(const VW &L, const Row<T> &R, long n, T koef)
 {
     using A = Ar<T>;
     T s = -(V == 1 ? L.f1[n] : V == 2 ? L.f2[n] : L.f3[n]);
@@ -1220,6 +1223,280 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_vcycle_cluster(const __grid
     tail_body<T>(a, ClusterTeam());
 }
 
+// The tail on chip: one block holds the unknowns, viscosities, right-hand sides, boundary bytes and 1-D
+// tables of its levels in shared memory (61 bytes per node in FP32, 109 in FP64), so that a phase is
+// shared-memory loads, a row and a __syncthreads().  The general tail above reads all of it through L1
+// and L2, which every barrier's writes empty, and walks the boundary lists in separate phases: 16 us a
+// FP32 sweep at 12^3 nodes on B200, 11 us in FP64.  Same rows in the same order; a boundary row
+// x_b = +-x_p is written by its partner's thread right after the partner, and rows without a partner
+// stay zero, under the conditions checked in build_smtail.
+template <typename T>
+struct SmTailLevel {
+    View<T> v;                   // global arrays (f in, u out)
+    Ct4 tr;                      // FP32: transfers to the next coarser level
+    int ou, oe, of, ornd, ob, ot, on, ond, ofi;   // byte offsets in shared memory
+    const unsigned *ent;         // boundary entries: node - partner + 32768 << 16 | sign << 15 | 0x4000 if another follows
+    const uint16_t *first;       // [component][node]: first entry of a partner, 0xffff none
+    const int *cst;              // nodes of boundary rows without a partner, sorted by component
+    int nent, cptr[5];
+    int down, up;
+};
+constexpr size_t kSmTailBytes = 227 * 1024;
+constexpr int kSmTailLevels = 4;
+// threads: one round per colour at 12^3 within the register cap (72 in FP64, 64 in FP32)
+template <typename T>
+constexpr int kSmTailThreads = sizeof(T) == 4 ? 1024 : 896;
+template <typename T>
+struct SmTailArgs {
+    int nl;
+    T v0, p0, kv, kp;
+    SmTailLevel<T> L[sizeof(T) == 4 ? kSmTailLevels : 1];
+};
+
+// an array in the dynamic shared memory, by byte offset
+template <typename T>
+struct SmPtr {
+    int base;
+    __device__ __forceinline__ T &operator[](long n) const
+    {
+        extern __shared__ __align__(16) unsigned char sm_tail[];
+        return *(T *)(sm_tail + (base + (int)n * (int)sizeof(T)));
+    }
+};
+template <typename T>
+struct SmView {
+    int nx, ny, nz, nxy;
+    FastDiv dnx, dny, dhy;
+    SmPtr<uint8_t> bc;
+    SmPtr<T> u0, u1, u2, u3, f0, f1, f2, f3, r0, r1, r2, r3, etac, etaxy, etaxz, etayz, icx, isx, icy, isy, icz, isz;
+    SmPtr<float> nd;
+    SmPtr<unsigned> ent;
+    SmPtr<uint16_t> first;
+};
+
+template <typename T>
+__device__ __forceinline__ SmView<T> sm_view(const SmTailLevel<T> &G)
+{
+    SmView<T> W;
+    constexpr int S = (int)sizeof(T);
+    W.nx = G.v.nx; W.ny = G.v.ny; W.nz = G.v.nz; W.nxy = (int)G.v.nxy;
+    W.dnx = G.v.dnx; W.dny = G.v.dny; W.dhy = G.v.dhy;
+    const int N = S * W.nxy * W.nz;
+    W.u0.base = G.ou; W.u1.base = G.ou + N; W.u2.base = G.ou + 2 * N; W.u3.base = G.ou + 3 * N;
+    W.etac.base = G.oe; W.etaxy.base = G.oe + N; W.etaxz.base = G.oe + 2 * N; W.etayz.base = G.oe + 3 * N;
+    W.f0.base = G.of; W.f1.base = G.of + N; W.f2.base = G.of + 2 * N; W.f3.base = G.of + 3 * N;
+    W.r0.base = G.ornd; W.r1.base = G.ornd + N; W.r2.base = G.ornd + 2 * N; W.r3.base = G.ornd + 3 * N;
+    W.nd.base = G.ond;
+    W.bc.base = G.ob;
+    W.icx.base = G.ot; W.isx.base = W.icx.base + S * (W.nx + 1); W.icy.base = W.isx.base + S * (W.nx + 1);
+    W.isy.base = W.icy.base + S * (W.ny + 1); W.icz.base = W.isy.base + S * (W.ny + 1); W.isz.base = W.icz.base + S * (W.nz + 1);
+    W.ent.base = G.on;
+    W.first.base = G.ofi;
+    return W;
+}
+template <int V, typename T>
+__device__ __forceinline__ SmPtr<T> sm_u(const SmView<T> &W) { return V == 0 ? W.u0 : V == 1 ? W.u1 : V == 2 ? W.u2 : W.u3; }
+template <int V, typename T>
+__device__ __forceinline__ SmPtr<T> sm_f(const SmView<T> &W) { return V == 0 ? W.f0 : V == 1 ? W.f1 : V == 2 ? W.f2 : W.f3; }
+template <int V, typename T>
+__device__ __forceinline__ SmPtr<T> sm_r(const SmView<T> &W) { return V == 0 ? W.r0 : V == 1 ? W.r1 : V == 2 ? W.r2 : W.r3; }
+
+// row n's new value and the boundary rows that follow it
+template <int V, typename T>
+__device__ __forceinline__ void sm_store(const SmView<T> &W, int n, T un)
+{
+    const SmPtr<T> u = sm_u<V>(W);
+    u[n] = un;
+    unsigned e = W.first[V * W.nxy * W.nz + n];
+    if (e == 0xffffu) return;
+    for (;; e++) {
+        const unsigned x = W.ent[e];
+        u[n + (int)(x >> 16) - 32768] = Ar<T>::add(T(0), (x & 0x8000u) ? -un : un);
+        if (!(x & 0x4000u)) break;
+    }
+}
+
+// end of component V's rows; cst: zeros of its boundary rows without a partner (the first sweep after a
+// prolongation, which added to them)
+template <int V, typename T>
+__device__ __forceinline__ void sm_phase_end(const SmView<T> &W, const SmTailLevel<T> &G, bool cst)
+{
+    __syncthreads();
+    if (!cst || G.cptr[V] == G.cptr[V + 1]) return;
+    for (int t = G.cptr[V] + (int)threadIdx.x; t < G.cptr[V + 1]; t += kSmTailThreads<T>) sm_u<V>(W)[__ldg(G.cst + t)] = T(0);
+    __syncthreads();
+}
+
+template <int V, typename T>
+__device__ __forceinline__ void sm_colours(const SmView<T> &W, const SmTailLevel<T> &G, T v0, bool cst)
+{
+    const int total = ((W.ny + 1) >> 1) * W.nx * W.nz;
+#pragma unroll 1
+    for (int color = 0; color < 2; color++) {
+        for (int t = (int)threadIdx.x; t < total; t += kSmTailThreads<T>) {
+            int i, j, k;
+            const int n = (int)vel_row_node<V>(W, t, color, i, j, k);
+            if (n < 0 || (W.bc[n] & (1 << V))) continue;
+            sm_store<V>(W, n, relaxed<T, V>(W, vcoef<T, V>(W, i, j, k, n), n, v0));
+        }
+        sm_phase_end<V>(W, G, cst && color == 1);
+    }
+}
+
+template <int V>
+__device__ __forceinline__ void sm_restrict(const SmTailLevel<float> &F, const SmView<float> &Wf, const SmView<float> &Wc, int t, int i, int j, int k)
+{
+    float x = 0.f;
+    if (row_exists(V, i, j, k, Wc.nx, Wc.ny, Wc.nz) && !(Wc.bc[t] & (1 << V))) {
+        const float4 wx = __ldg(F.tr.t[V][0].w + i), wy = __ldg(F.tr.t[V][1].w + j), wz = __ldg(F.tr.t[V][2].w + k);
+        const int m = __ldg(F.tr.t[V][2].s + k) * Wf.nxy + __ldg(F.tr.t[V][0].s + i) * Wf.ny + __ldg(F.tr.t[V][1].s + j);
+        const SmPtr<float> r = sm_r<V>(Wf);
+        const float ax[4] = {wx.x, wx.y, wx.z, wx.w}, az[4] = {wz.x, wz.y, wz.z, wz.w};
+#pragma unroll
+        for (int ez = 0; ez < 4; ez++) {
+            float sx = 0.f;
+#pragma unroll
+            for (int ex = 0; ex < 4; ex++) {
+                const int q = m + ez * Wf.nxy + ex * Wf.ny;
+                sx += ax[ex] * (wy.x * r[q] + wy.y * r[q + 1] + wy.z * r[q + 2] + wy.w * r[q + 3]);
+            }
+            x += az[ez] * sx;
+        }
+        if (V == 0) x /= Wc.nd[t];
+        x *= __ldg(F.tr.iws[V] + t);
+    }
+    sm_f<V>(Wc)[t] = x;
+}
+
+template <int V>
+__device__ __forceinline__ void sm_prolong(const SmTailLevel<float> &F, const SmView<float> &Wf, const SmView<float> &Wc, float koef, int n, int i,
+                                           int j, int k)
+{
+    if (!row_exists(V, i, j, k, Wf.nx, Wf.ny, Wf.nz)) return;
+    const float2 wx = __ldg(F.tr.t[V][0].v + i), wy = __ldg(F.tr.t[V][1].v + j), wz = __ldg(F.tr.t[V][2].v + k);
+    const int m = __ldg(F.tr.t[V][2].a + k) * Wc.nxy + __ldg(F.tr.t[V][0].a + i) * Wc.ny + __ldg(F.tr.t[V][1].a + j), q = m + Wc.nxy;
+    const SmPtr<float> c = sm_u<V>(Wc);
+    const float a = wx.x * (wy.x * c[m] + wy.y * c[m + 1]) + wx.y * (wy.x * c[m + Wc.ny] + wy.y * c[m + Wc.ny + 1]);
+    const float b = wx.x * (wy.x * c[q] + wy.y * c[q + 1]) + wx.y * (wy.x * c[q + Wc.ny] + wy.y * c[q + Wc.ny + 1]);
+    sm_u<V>(Wf)[n] += koef * (wz.x * a + wz.y * b);
+}
+
+// the residual of level G as k_residual_f32 leaves it, restricted to the right-hand side of Gc
+__device__ __forceinline__ void sm_down(const SmTailLevel<float> &G, const SmTailLevel<float> &Gc)
+{
+    const SmView<float> W = sm_view(G), Wc = sm_view(Gc);
+    const int N = W.nxy * W.nz, Nc = Wc.nxy * Wc.nz;
+    for (int n = (int)threadIdx.x; n < N; n += kSmTailThreads<float>) {
+        int i, j, k;
+        node_ijk(W, n, i, j, k);
+        const uint8_t b = W.bc[n];
+        float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
+        if (row_exists(0, i, j, k, W.nx, W.ny, W.nz) && !(b & 1)) { s0 = W.f0[n]; crow<float, true>(W, i, j, k, n, s0); s0 *= W.nd[n]; }
+        if (row_exists(1, i, j, k, W.nx, W.ny, W.nz) && !(b & 2)) { s1 = W.f1[n]; xrow<float, true>(W, i, j, k, n, s1); }
+        if (row_exists(2, i, j, k, W.nx, W.ny, W.nz) && !(b & 4)) { s2 = W.f2[n]; yrow<float, true>(W, i, j, k, n, s2); }
+        if (row_exists(3, i, j, k, W.nx, W.ny, W.nz) && !(b & 8)) { s3 = W.f3[n]; zrow<float, true>(W, i, j, k, n, s3); }
+        W.r0[n] = s0; W.r1[n] = s1; W.r2[n] = s2; W.r3[n] = s3;
+    }
+    __syncthreads();
+    for (int t = (int)threadIdx.x; t < Nc; t += kSmTailThreads<float>) {
+        int i, j, k;
+        node_ijk(Wc, t, i, j, k);
+        sm_restrict<0>(G, W, Wc, t, i, j, k);
+        sm_restrict<1>(G, W, Wc, t, i, j, k);
+        sm_restrict<2>(G, W, Wc, t, i, j, k);
+        sm_restrict<3>(G, W, Wc, t, i, j, k);
+    }
+    __syncthreads();
+}
+
+__device__ __forceinline__ void sm_up(const SmTailLevel<float> &G, const SmTailLevel<float> &Gc, float kv, float kp)
+{
+    const SmView<float> W = sm_view(G), Wc = sm_view(Gc);
+    const int N = W.nxy * W.nz;
+    for (int n = (int)threadIdx.x; n < N; n += kSmTailThreads<float>) {
+        int i, j, k;
+        node_ijk(W, n, i, j, k);
+        sm_prolong<0>(G, W, Wc, kp, n, i, j, k);
+        sm_prolong<1>(G, W, Wc, kv, n, i, j, k);
+        sm_prolong<2>(G, W, Wc, kv, n, i, j, k);
+        sm_prolong<3>(G, W, Wc, kv, n, i, j, k);
+    }
+    __syncthreads();
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kSmTailThreads<T>, 1) k_vcycle_smtail(const __grid_constant__ SmTailArgs<T> a)
+{
+    constexpr int TH = kSmTailThreads<T>;
+    constexpr bool F32 = sizeof(T) == 4;
+    pdl_trigger();
+    // operator data before the wait (PRO's rule: the restriction before this launch writes none of it)
+    for (int q = 0; q < a.nl; q++) {
+        const SmTailLevel<T> &G = a.L[q];
+        const SmView<T> W = sm_view(G);
+        const int N = W.nxy * W.nz;
+        for (int n = (int)threadIdx.x; n < N; n += TH) {
+            W.etac[n] = G.v.etac[n]; W.etaxy[n] = G.v.etaxy[n]; W.etaxz[n] = G.v.etaxz[n]; W.etayz[n] = G.v.etayz[n];
+            W.nd[n] = G.v.nd[n];
+            W.bc[n] = G.v.bc[n];
+            W.u0[n] = T(0); W.u1[n] = T(0); W.u2[n] = T(0); W.u3[n] = T(0);
+            for (int v = 0; v < 4; v++) W.first[v * N + n] = G.first[v * N + n];
+        }
+        for (int n = (int)threadIdx.x; n <= W.nx; n += TH) { W.icx[n] = G.v.icx[n]; W.isx[n] = G.v.isx[n]; }
+        for (int n = (int)threadIdx.x; n <= W.ny; n += TH) { W.icy[n] = G.v.icy[n]; W.isy[n] = G.v.isy[n]; }
+        for (int n = (int)threadIdx.x; n <= W.nz; n += TH) { W.icz[n] = G.v.icz[n]; W.isz[n] = G.v.isz[n]; }
+        for (int n = (int)threadIdx.x; n < G.nent; n += TH) W.ent[n] = G.ent[n];
+    }
+    pdl_wait();
+    {
+        const SmTailLevel<T> &G = a.L[0];
+        const SmView<T> W = sm_view(G);
+        const int N = W.nxy * W.nz;
+        for (int n = (int)threadIdx.x; n < N; n += TH) {
+            W.f0[n] = G.v.f0[n]; W.f1[n] = G.v.f1[n]; W.f2[n] = G.v.f2[n]; W.f3[n] = G.v.f3[n];
+        }
+    }
+    __syncthreads();
+    // steps 0..nl-1 go down (the last one is the coarsest level), nl..2nl-2 back up
+#pragma unroll 1
+    for (int step = 0; step < 2 * a.nl - 1; step++) {
+        const bool upward = step >= a.nl;
+        const int q = upward ? 2 * a.nl - 2 - step : step;
+        const SmTailLevel<T> &G = a.L[q];
+        const SmView<T> W = sm_view(G);
+        const int N = W.nxy * W.nz;
+        const bool coarsest = q == a.nl - 1;
+        if constexpr (F32)
+            if (upward) sm_up(G, a.L[q + 1], a.kv, a.kp);
+        const int sweeps = upward || coarsest ? G.up : G.down;
+#pragma unroll 1
+        for (int s = 0; s < sweeps; s++) {
+            const bool cst = upward && s == 0;
+            sm_colours<1>(W, G, a.v0, cst);
+            sm_colours<2>(W, G, a.v0, cst);
+            sm_colours<3>(W, G, a.v0, cst);
+            for (int n = (int)threadIdx.x; n < N; n += TH) {
+                int i, j, k;
+                node_ijk(W, n, i, j, k);
+                if (!(i > 0 && j > 0 && k > 0) || (W.bc[n] & 1)) continue;
+                T r = -W.f0[n];
+                crow<T, false>(W, i, j, k, n, r);
+                sm_store<0>(W, n, Ar<T>::sub(W.u0[n], Ar<T>::mul(Ar<T>::mul(r, (T)W.nd[n]), a.p0)));
+            }
+            sm_phase_end<0>(W, G, cst);
+        }
+        if constexpr (F32)
+            if (!upward && !coarsest) sm_down(G, a.L[q + 1]);
+    }
+    // only the finest tail level's solution is read outside
+    const SmTailLevel<T> &G = a.L[0];
+    const SmView<T> W = sm_view(G);
+    const int N = W.nxy * W.nz;
+    for (int n = (int)threadIdx.x; n < N; n += TH) {
+        G.v.u0[n] = W.u0[n]; G.v.u1[n] = W.u1[n]; G.v.u2[n] = W.u2[n]; G.v.u3[n] = W.u3[n];
+    }
+}
+
 // ronurestrict (move3mg.c:2642-2741): FP32 accumulator as in nu[], FP64 weights
 __global__ void k_nu_restrict(const float *nuf, int fnx, int fny, int fnz, float *nuc, int cnx, int cny, int cnz,
                               TrView tx, TrView ty, TrView tz, int viscmod)
@@ -1688,6 +1965,61 @@ static int upload_f32_scaled(i3g_ctx *c, float *&dst, const std::vector<double> 
     return upload(c, dst, f);
 }
 
+// Boundary rows of one level for the on-chip tail: one list entry each, by partner.  The level
+// stays with the general tail when a chain's factors do not multiply to -1, 0 or 1, or a boundary row is
+// read by another row of its partner's phase, or (partner of the first colour) by a row of the second
+// colour, which sees the old value when the boundary pass follows both colours.
+// Up to kSmTailNodes nodes: with 12^3 the tail takes 39 us of a FP32 V-cycle against 66 for the general
+// tail, and a 33^3 FP64 solve 146 instead of 192 ms (B200); its time grows with the nodes on its one
+// SM, a launched FP32 sweep takes 17 us at any small size.
+constexpr long kSmTailNodes = 2500;
+static int build_smtail(i3g_ctx *c, Level &L, const std::vector<uint8_t> &mask, const std::vector<int> (&node)[4],
+                        const std::vector<int> (&pnode)[4], const std::vector<int> (&depth)[4], const std::vector<double> (&kk)[4])
+{
+    SmTailRows &R = L.sm;
+    if (L.n > kSmTailNodes) return 0;
+    std::vector<unsigned> hent;
+    std::vector<int> hcst;
+    std::vector<uint16_t> first(4 * (size_t)L.n, 0xffff);
+    R.cptr[0] = 0;
+    for (int v = 0; v < 4; v++) {
+        std::vector<std::pair<int, unsigned>> ent;   // partner, entry
+        for (size_t e = 0; e < node[v].size(); e++) {
+            const int b = node[v][e], p = pnode[v][e];
+            double K = 1.0;
+            for (int d = 0; d < depth[v][e]; d++) {
+                const double k = kk[v][e * kMaxBcDepth + d];
+                if (k != 0.0 && k != 1.0 && k != -1.0 && p >= 0) return 0;
+                K *= k;
+            }
+            if (p < 0 || K == 0.0) { hcst.push_back(b); continue; }
+            const int j = b % L.ny, i = (b / L.ny) % L.nx, k = b / (L.ny * L.nx);
+            const int pc = (p % L.ny + (p / L.ny) % L.nx + p / (L.ny * L.nx)) & 1;
+            const int di[6] = {-1, 1, 0, 0, 0, 0}, dj[6] = {0, 0, -1, 1, 0, 0}, dk[6] = {0, 0, 0, 0, -1, 1};
+            for (int d = 0; v > 0 && d < 6; d++) {
+                const int i2 = i + di[d], j2 = j + dj[d], k2 = k + dk[d];
+                if (i2 < 0 || j2 < 0 || k2 < 0 || i2 >= L.nx || j2 >= L.ny || k2 >= L.nz) continue;
+                const int q = (k2 * L.nx + i2) * L.ny + j2;
+                if (q == p || !row_exists(v, i2, j2, k2, L.nx, L.ny, L.nz) || (mask[q] & (1 << v))) continue;
+                if (pc == 0 || ((i2 + j2 + k2) & 1)) return 0;
+            }
+            ent.push_back({p, (K < 0 ? 0x8000u : 0u) | (unsigned)(b - p + 32768) << 16});
+        }
+        std::stable_sort(ent.begin(), ent.end(), [](const auto &x, const auto &y) { return x.first < y.first; });
+        for (size_t e = 0; e < ent.size(); e++) {
+            uint16_t &f = first[(size_t)v * L.n + ent[e].first];
+            if (f == 0xffff) f = (uint16_t)hent.size();
+            hent.push_back(ent[e].second | (e + 1 < ent.size() && ent[e + 1].first == ent[e].first ? 0x4000u : 0u));
+        }
+        R.cptr[v + 1] = (int)hcst.size();
+    }
+    R.nent = (int)hent.size();
+    int rc;
+    if ((rc = upload(c, R.ent, hent)) || (rc = upload(c, R.cst, hcst)) || (rc = upload(c, R.first, first))) return rc;
+    R.ok = true;
+    return 0;
+}
+
 // The packed form of one component's boundary rows (bc_packed); left out where a chain's factors do
 // not multiply to -1, 0 or 1 or a writer is not the partner.
 constexpr long kBcInline = 400000;
@@ -1891,6 +2223,8 @@ static int build_bc(i3g_ctx *c)
                 }
             }
         }
+        if (c->smtail && l > 0)
+            if (const int rc = build_smtail(c, L, mask, node, pnode, depth, kk)) return rc;
         if (getenv("I3G_TRACE"))
             for (int v = 0; v < 4; v++)
                 fprintf(stderr, "i3g: level %d component %d: %zu boundary rows, %s (%d by a row's thread)\n", l, v,
@@ -1925,6 +2259,13 @@ int stokes_alloc(i3g_ctx *c)
     // I3G_FUSE: 0 one launch per boundary pass, residual part and transfer component; 1 boundary
     // rows in-kernel on levels >= 1 (default); 3 on level 0 too
     if (const char *e = getenv("I3G_FUSE")) c->fuse = atoi(e);
+    // on-chip tail (I3G_SMTAIL=0, or a variable that chooses another tail, turns it off)
+    c->smtail = !getenv("I3G_TAIL_NODES") && !getenv("I3G_COOP_NODES") && !getenv("I3G_TAIL_CLUSTER") && c->fuse;
+    if (const char *e = getenv("I3G_SMTAIL")) c->smtail = c->smtail && atoi(e);
+    if (c->smtail) {
+        I3G_CUDA(cudaFuncSetAttribute(k_vcycle_smtail<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmTailBytes));
+        I3G_CUDA(cudaFuncSetAttribute(k_vcycle_smtail<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmTailBytes));
+    }
     c->pro_nodes = kProNodes;
     if (const char *e = getenv("I3G_PRO_NODES")) c->pro_nodes = atol(e);
     if (const char *e = getenv("I3G_ND_SCHUR")) c->nd_schur = std::max(0, atoi(e));
@@ -2071,6 +2412,7 @@ void stokes_free(i3g_ctx *c)
                 cudaFree(t.cs); cudaFree(t.cw); cudaFree(t.cv);
             }
         for (int v = 0; v < 4; v++) cudaFree(L.iws[v]);
+        cudaFree(L.sm.ent); cudaFree(L.sm.cst); cudaFree(L.sm.first);
     }
     cudaFree(c->dred);
     if (c->hred) cudaFreeHost(c->hred);
@@ -2363,19 +2705,92 @@ static void tail_launch(i3g_ctx *c, int lc, int multinum)
     LAUNCH(k_vcycle_tail<T>, 1, kTailThreads, a);
 }
 
+// Arguments and shared-memory layout of the on-chip tail for levels lc..multinum; the bytes used, 0 when
+// it does not take them.
+template <typename T>
+static size_t smtail_args(i3g_ctx *c, int lc, int multinum, SmTailArgs<T> *a)
+{
+    const int nl = multinum - lc + 1;
+    constexpr int S = (int)sizeof(T);
+    if (!c->smtail || nl > (S == 4 ? kSmTailLevels : 1)) return 0;
+    size_t use = 0;
+    auto take = [&](size_t n) { const size_t at = use; use += (n + 15) & ~(size_t)15; return (int)at; };
+    if (a) {
+        memset((void *)a, 0, sizeof *a);
+        a->nl = nl;
+        a->v0 = (T)c->p.v0koef; a->p0 = (T)c->p.p0koef; a->kv = (T)c->p.v1koef; a->kp = (T)c->p.p1koef;
+    }
+    for (int q = 0; q < nl; q++) {
+        Level &L = c->lev[lc + q];
+        if (!L.sm.ok || (q + 1 < nl && !c->lev[lc + q + 1].compact)) return 0;
+        const size_t N = (size_t)L.n;
+        SmTailLevel<T> G;
+        memset((void *)&G, 0, sizeof G);
+        G.ou = take(4 * S * N); G.oe = take(4 * S * N); G.of = take(4 * S * N); G.ond = take(4 * N); G.ob = take(N);
+        G.ot = take(2 * S * (size_t)(L.nx + L.ny + L.nz + 3)); G.on = take(4 * (size_t)L.sm.nent); G.ofi = take(8 * N);
+        if (q + 1 < nl) G.ornd = take(4 * S * N);
+        if (use > kSmTailBytes) return 0;
+        if (!a) continue;
+        G.v = view<T>(L, fields<T>(L));
+        if constexpr (S == 4)
+            if (q + 1 < nl) G.tr = ct4(L, c->lev[lc + q + 1]);
+        G.ent = L.sm.ent; G.first = L.sm.first; G.cst = L.sm.cst; G.nent = L.sm.nent;
+        for (int k = 0; k < 5; k++) G.cptr[k] = L.sm.cptr[k];
+        G.down = c->p.multinnn[0][lc + q];
+        G.up = c->p.multinnn[1][lc + q];
+        a->L[q] = G;
+    }
+    return use;
+}
+
+// First level of the on-chip tail: as many of the coarsest levels (>= 1) as fit one SM's shared memory
+// and have up to kSmTailNodes nodes (FP64: the coarsest alone, whose transfers keep the oracle's order); multinum + 1 when none.
+template <typename T>
+static int smtail_start(i3g_ctx *c, int multinum)
+{
+    int lc = multinum + 1;
+    for (int l = multinum; l >= 1; l--) {
+        if (c->lev[l].n > kSmTailNodes || !smtail_args<T>(c, l, multinum, nullptr)) break;
+        lc = l;
+    }
+    return lc;
+}
+
+template <typename T>
+static void smtail_launch(i3g_ctx *c, int lc, int multinum)
+{
+    SmTailArgs<T> a;
+    cudaLaunchConfig_t cfg = {};
+    cfg.dynamicSmemBytes = smtail_args<T>(c, lc, multinum, &a);
+    cfg.gridDim = dim3(1);
+    cfg.blockDim = dim3(kSmTailThreads<T>);
+    cfg.stream = c->st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = pdl_enabled() ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, k_vcycle_smtail<T>, a);
+    c->launches++;
+}
+
 // V-cycle with the schedule of move3mg.c:2173-2213; the small coarse levels run in the
-// one-block tail kernel.
+// one-block tail kernels.
 template <typename T>
 static void vcycle_t(i3g_ctx *c, int multinum, bool homogeneous)
 {
-    const int lc = tail_start(c, multinum);
+    int lc = tail_start(c, multinum);
+    const int ls = smtail_start<T>(c, multinum);
+    const bool onchip = ls <= multinum;
+    if (onchip) lc = ls;
     for (int l = 0; l < multinum && l < lc; l++) {
         const int n = c->p.multinnn[0][l];
         if (n > 0) smooth_t<T>(c, l, n, homogeneous, true);
         else residual_t<T>(c, l);
         restrict_t<T>(c, l + 1);
     }
-    if (lc <= multinum) tail_launch<T>(c, lc, multinum);
+    if (onchip) smtail_launch<T>(c, lc, multinum);
+    else if (lc <= multinum) tail_launch<T>(c, lc, multinum);
     for (int l = std::min(lc, multinum); l > 0; l--) {
         const int n = c->p.multinnn[1][l];
         if (n > 0 && l != lc) smooth_t<T>(c, l, n, homogeneous, false);
@@ -3487,7 +3902,11 @@ int stokes_time_kernel(i3g_ctx *c, int kind, int reps, double *ms, double *bytes
         if (kind >= 13 && l >= c->nlev) return set_error(c, I3G_E_ARG, "level %d does not exist", l);
         auto warm = [&]() {
             if (kind == 11) vcycle_t<float>(c, mn, true);
-            else if (kind == 12) { if (lc <= mn) tail_launch<float>(c, lc, mn); }
+            else if (kind == 12) {
+                const int ls = smtail_start<float>(c, mn);
+                if (ls <= mn) smtail_launch<float>(c, ls, mn);
+                else if (lc <= mn) tail_launch<float>(c, lc, mn);
+            }
             else smooth_t<float>(c, l, 1, true, false);
         };
         for (int w = 0; w < 2; w++) warm();
