@@ -6,7 +6,12 @@
 // relaxation with the reference's damped update, node-centred weighted restriction of the
 // residual, trilinear prolongation, and conductivity / heat capacity restricted with the
 // viscosity-restriction weights.  The converged temperature is that of the reference's rows.
-// FP64 arithmetic uses explicitly rounded operations in the reference's operand order.
+//
+// How many levels a solve needs follows from its coupling: with q the ratio of a row's neighbour
+// coefficients to its rho cp / dt, a red-black sweep reduces the error by (q / (1 + q))^2 at worst.
+// A time step limited by the flow has q far below 1 (0.1 on the benchmark model), where sweeps on
+// level 0 alone reach the tolerance and coarser levels would only add launches; q falls fourfold per
+// level, and the hierarchy is used down to the first level with q <= 1 (heat_plan).
 #include <algorithm>
 #include <cmath>
 #include <vector>
@@ -19,6 +24,14 @@ struct HeatLevel {
     float *kt = nullptr;            // level 0 points at the context's kt
     double *rocp = nullptr;
     double *dx = nullptr, *dy = nullptr, *dz = nullptr;   // raw spacings g[i]-g[i-1] (i >= 1)
+    // face factors of a row, 1 / (distance to the neighbour * distance between its two neighbours):
+    // [0] towards i - 1, [1] towards i + 1 (twice the face's half sum of conductivities times the
+    // reference's 2 / (g[i+1] - g[i-1]) over the spacing)
+    double *cx[2] = {nullptr, nullptr}, *cy[2] = {nullptr, nullptr}, *cz[2] = {nullptr, nullptr};
+    // boundary rows written by the black relaxation launch: entries [0, na) sorted by their partner, a
+    // black row whose thread writes them (first[]), [na, nbc) by extra blocks; -1: a separate launch
+    int na = -1;
+    int *first = nullptr;
     uint8_t *bc = nullptr;
     int nbc = 0;
     int *bnode = nullptr, *bpn = nullptr, *bdep = nullptr;
@@ -42,34 +55,29 @@ struct HView {
     double *u, *f, *r;
     const float *kt;
     const double *rocp;
-    const double *isx, *isy, *isz;    // 1/(g[i+1]-g[i-1])
-    const double *dx, *dy, *dz;       // g[i]-g[i-1]
+    const double *cx[2], *cy[2], *cz[2];   // face factors
     const uint8_t *bc;
-    double dt;
+    double idt;                       // 1 / dt
 };
 
 // diagonal and neighbour coefficients of the heat row at n (heaterr mode 1)
 struct HRow { double d, c[6]; };
 
-__device__ __forceinline__ double kflux(float ka, float kb, double xkf, double h)
-{
-    // (kt_a + kt_b)/2.0 * xkf / h, the FP32 sum first as in C
-    return __ddiv_rn(__dmul_rn(__ddiv_rn((double)__fadd_rn(ka, kb), 2.0), xkf), h);
-}
-
+// face coefficient (kt_a + kt_b) / 2 * 2 / (g[i+1] - g[i-1]) / spacing, the FP32 sum first as in C;
+// the grid factors come as one product from a table: six divisions per row were most of a sweep's
+// time
 __device__ __forceinline__ HRow hrow(const HView &V, int i, int j, int k, long n)
 {
     HRow R;
     const long NY = V.ny, NXY = V.nxy;
-    const double xkf = __dmul_rn(2.0, V.isx[i]), ykf = __dmul_rn(2.0, V.isy[j]), zkf = __dmul_rn(2.0, V.isz[k]);
     const float kn = V.kt[n];
-    double d = __ddiv_rn(V.rocp[n], V.dt), iv;
-    iv = kflux(V.kt[n - NY], kn, xkf, V.dx[i]);     R.c[0] = -iv; d = __dadd_rn(d, iv);   // v1 (x-)
-    iv = kflux(kn, V.kt[n + NY], xkf, V.dx[i + 1]); d = __dadd_rn(d, iv); R.c[1] = -iv;   // v5 (x+)
-    iv = kflux(V.kt[n - 1], kn, ykf, V.dy[j]);      R.c[2] = -iv; d = __dadd_rn(d, iv);   // v2 (y-)
-    iv = kflux(kn, V.kt[n + 1], ykf, V.dy[j + 1]);  d = __dadd_rn(d, iv); R.c[3] = -iv;   // v4 (y+)
-    iv = kflux(V.kt[n - NXY], kn, zkf, V.dz[k]);    R.c[4] = -iv; d = __dadd_rn(d, iv);   // v0 (z-)
-    iv = kflux(kn, V.kt[n + NXY], zkf, V.dz[k + 1]); d = __dadd_rn(d, iv); R.c[5] = -iv;  // v6 (z+)
+    double d = V.rocp[n] * V.idt, iv;
+    iv = (double)__fadd_rn(V.kt[n - NY], kn) * V.cx[0][i];  R.c[0] = -iv; d += iv;   // v1 (x-)
+    iv = (double)__fadd_rn(kn, V.kt[n + NY]) * V.cx[1][i];  R.c[1] = -iv; d += iv;   // v5 (x+)
+    iv = (double)__fadd_rn(V.kt[n - 1], kn) * V.cy[0][j];   R.c[2] = -iv; d += iv;   // v2 (y-)
+    iv = (double)__fadd_rn(kn, V.kt[n + 1]) * V.cy[1][j];   R.c[3] = -iv; d += iv;   // v4 (y+)
+    iv = (double)__fadd_rn(V.kt[n - NXY], kn) * V.cz[0][k]; R.c[4] = -iv; d += iv;   // v0 (z-)
+    iv = (double)__fadd_rn(kn, V.kt[n + NXY]) * V.cz[1][k]; R.c[5] = -iv; d += iv;   // v6 (z+)
     R.d = d;
     return R;
 }
@@ -85,9 +93,30 @@ __device__ __forceinline__ double hsum(const HView &V, const HRow &R, long n, do
     return s;
 }
 
-__global__ void __launch_bounds__(256) k_heat_relax(HView V, int color, double koef)
+// boundary rows of a level for the black launch
+struct HBc {
+    int n, na, use_c;
+    const int *node, *pn, *dep, *first;
+    const double *cc, *kk;
+};
+
+__device__ __forceinline__ double hbc_value(const HBc &B, int t, double v)
+{
+    for (int d = B.dep[t] - 1; d >= 0; d--)
+        v = __dadd_rn(B.use_c ? B.cc[t * kMaxBcDepth + d] : 0.0, __dmul_rn(B.kk[t * kMaxBcDepth + d], v));
+    return v;
+}
+
+// One colour; the black launch also writes the boundary rows (B.na >= 0), from a black partner's
+// thread right after its update, else on blocks past rowblocks
+__global__ void __launch_bounds__(256) k_heat_relax(HView V, int color, double koef, HBc B, unsigned rowblocks)
 {
     pdl_enter();
+    if (blockIdx.x >= rowblocks) {
+        const int t = B.na + (int)((blockIdx.x - rowblocks) * blockDim.x + threadIdx.x);
+        if (t < B.n) V.u[B.node[t]] = hbc_value(B, t, B.pn[t] >= 0 ? V.u[B.pn[t]] : 0.0);
+        return;
+    }
     const int hy = (V.ny + 1) >> 1;
     const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= (long)hy * V.nx * V.nz) return;
@@ -100,7 +129,11 @@ __global__ void __launch_bounds__(256) k_heat_relax(HView V, int color, double k
     if (V.bc[n]) return;
     const HRow R = hrow(V, i, j, k, n);
     const double s = hsum<false>(V, R, n, -V.f[n]);
-    V.u[n] = __dsub_rn(V.u[n], __dmul_rn(__ddiv_rn(s, R.d), koef));
+    const double un = V.u[n] = __dsub_rn(V.u[n], __dmul_rn(__ddiv_rn(s, R.d), koef));
+    if (color == 0 || B.na <= 0) return;
+    const int e0 = B.first[n];
+    if (e0 >= 0)
+        for (int t = e0; t < B.na && B.pn[t] == (int)n; t++) V.u[B.node[t]] = hbc_value(B, t, un);
 }
 
 __global__ void k_heat_residual(HView V)
@@ -126,17 +159,6 @@ __global__ void k_heat_bc(double *u, int n, const int *node, const int *pn, cons
     for (int d = dep[t] - 1; d >= 0; d--)
         v = __dadd_rn(use_c ? cc[t * kMaxBcDepth + d] : 0.0, __dmul_rn(kk[t * kMaxBcDepth + d], v));
     u[node[t]] = v;
-}
-
-__global__ void k_heat_bc_res(const double *u, const double *f, double *r, int n, const int *node, const int *on, const double *ok)
-{
-    pdl_enter();
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n) return;
-    const int nd = node[t];
-    double s = __dsub_rn(f[nd], __dmul_rn(1.0, u[nd]));
-    if (on[t] >= 0) s = __dsub_rn(s, __dmul_rn(-ok[t], u[on[t]]));
-    r[nd] = s;
 }
 
 struct TrV { const int *gptr, *gf; const double *gw; const int *a; const double *w0, *w1; };
@@ -226,9 +248,9 @@ struct H0Args {
 __global__ void k_heat_setup0(H0Args a)
 {
     pdl_enter();
-    __shared__ double sh[8];
+    __shared__ double sh[2][8];
     const long NY = a.ny, NXY = (long)a.nx * a.ny, N = NXY * a.nz;
-    double m = 0;
+    double m = 0, kap = 0;   // largest |rate| and largest k / (rho cp)
     for (long n = (long)blockIdx.x * blockDim.x + threadIdx.x; n < N; n += (long)gridDim.x * blockDim.x) {
         const float tkn = a.tk[n];
         a.tk0[n] = tkn; a.tk2[n] = tkn;
@@ -258,13 +280,18 @@ __global__ void k_heat_setup0(H0Args a)
         }
         a.tk1[n] = (float)iv;
         m = fmax(m, fabs(iv / (double)rocpf));
+        kap = fmax(kap, (double)(a.kt[n] / rocpf));
     }
-    for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_down_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = m;
+    for (int o = 16; o > 0; o >>= 1) {
+        m = fmax(m, __shfl_down_sync(0xffffffffu, m, o));
+        kap = fmax(kap, __shfl_down_sync(0xffffffffu, kap, o));
+    }
+    if ((threadIdx.x & 31) == 0) { sh[0][threadIdx.x >> 5] = m; sh[1][threadIdx.x >> 5] = kap; }
     __syncthreads();
     if (threadIdx.x == 0) {
-        for (int w = 1; w < (int)(blockDim.x >> 5); w++) m = fmax(m, sh[w]);
-        a.part[blockIdx.x] = m;
+        for (int w = 1; w < (int)(blockDim.x >> 5); w++) { m = fmax(m, sh[0][w]); kap = fmax(kap, sh[1][w]); }
+        a.part[2 * blockIdx.x] = m;
+        a.part[2 * blockIdx.x + 1] = kap;
     }
 }
 
@@ -353,10 +380,9 @@ static HView hview(i3g_ctx *c, int l, double dt)
     HView V;
     V.nx = L.nx; V.ny = L.ny; V.nz = L.nz; V.nxy = (long)L.nx * L.ny;
     V.u = H.u; V.f = H.f; V.r = H.r; V.kt = l == 0 ? c->kt : H.kt; V.rocp = H.rocp;
-    V.isx = L.d.ix[1]; V.isy = L.d.iy[1]; V.isz = L.d.iz[1];
-    V.dx = H.dx; V.dy = H.dy; V.dz = H.dz;
+    for (int q = 0; q < 2; q++) { V.cx[q] = H.cx[q]; V.cy[q] = H.cy[q]; V.cz[q] = H.cz[q]; }
     V.bc = H.bc;
-    V.dt = dt;
+    V.idt = 1.0 / dt;
     return V;
 }
 
@@ -391,6 +417,12 @@ int heat_alloc(i3g_ctx *c)
             for (int i = 1; i < nn[d]; i++) h[i] = g[d][i] - g[d][i - 1];
             int rc = up(c, *dd[d], h);
             if (rc) return rc;
+            double **cc[3] = {H.cx, H.cy, H.cz};
+            for (int q = 0; q < 2; q++) {
+                std::vector<double> f(nn[d] + 1, 0.0);
+                for (int i = 1; i < nn[d] - 1; i++) f[i] = 1.0 / (g[d][i + 1] - g[d][i - 1]) / h[i + q];
+                if ((rc = up(c, cc[d][q], f))) return rc;
+            }
         }
         std::vector<uint8_t> mask(L.n, 0);
         std::vector<int> bn, bp, bdp, bon;
@@ -430,7 +462,45 @@ int heat_alloc(i3g_ctx *c)
             for (int d = 0; d < kMaxBcDepth; d++) { bcc.push_back(d < dep ? chc[d] : 0.0); bck.push_back(d < dep ? chk[d] : 0.0); }
         }
         H.nbc = (int)bn.size();
+        // In-kernel boundary rows: a row with a black partner is written by the partner's thread and may
+        // be read by no other black row; any other is written by extra blocks of the black launch and
+        // may be read by no black row (the separate pass comes after the black rows).
+        std::vector<int> first(L.n, -1);
+        {
+            const int nbc = H.nbc;
+            std::vector<int> own, rest;
+            bool admit = true;
+            auto odd = [&](long q) { return ((q % L.ny + (q / L.ny) % L.nx + q / ((long)L.ny * L.nx)) & 1) != 0; };
+            for (int e = 0; e < nbc && admit; e++) {
+                const long q = bn[e];
+                const int j = (int)(q % L.ny), i = (int)((q / L.ny) % L.nx), k = (int)(q / ((long)L.ny * L.nx));
+                const bool mine = bp[e] >= 0 && odd(bp[e]);
+                const int di[6] = {-1, 1, 0, 0, 0, 0}, dj[6] = {0, 0, -1, 1, 0, 0}, dk[6] = {0, 0, 0, 0, -1, 1};
+                for (int d = 0; d < 6; d++) {
+                    const int i2 = i + di[d], j2 = j + dj[d], k2 = k + dk[d];
+                    if (i2 < 0 || j2 < 0 || k2 < 0 || i2 >= L.nx || j2 >= L.ny || k2 >= L.nz) continue;
+                    const long r = ((long)k2 * L.nx + i2) * L.ny + j2;
+                    if (!mask[r] && odd(r) && !(mine && r == bp[e])) admit = false;
+                }
+                (mine ? own : rest).push_back(e);
+            }
+            if (admit) {
+                std::stable_sort(own.begin(), own.end(), [&](int x, int y) { return bp[x] < bp[y]; });
+                std::vector<int> perm(own);
+                perm.insert(perm.end(), rest.begin(), rest.end());
+                auto permute = [&](auto &vec, int width) {
+                    auto old = vec;
+                    for (size_t e = 0; e < perm.size(); e++)
+                        for (int w = 0; w < width; w++) vec[e * width + w] = old[(size_t)perm[e] * width + w];
+                };
+                permute(bn, 1); permute(bp, 1); permute(bdp, 1); permute(bon, 1); permute(boc, 1); permute(bok, 1);
+                permute(bcc, kMaxBcDepth); permute(bck, kMaxBcDepth);
+                H.na = (int)own.size();
+                for (int e = H.na - 1; e >= 0; e--) first[bp[e]] = e;
+            }
+        }
         int rc;
+        if ((rc = up(c, H.first, first))) return rc;
         if ((rc = up(c, H.bc, mask)) || (rc = up(c, H.bnode, bn)) || (rc = up(c, H.bpn, bp)) || (rc = up(c, H.bdep, bdp)) ||
             (rc = up(c, H.bcc, bcc)) || (rc = up(c, H.bck, bck)) || (rc = up(c, H.bon, bon)) || (rc = up(c, H.boc, boc)) ||
             (rc = up(c, H.bok, bok)))
@@ -450,7 +520,7 @@ void heat_free(i3g_ctx *c)
     if (!S) return;
     for (int l = 0; l < c->nlev; l++) {
         HeatLevel &H = S->L[l];
-        void *p[] = {H.u, H.f, H.r, H.rocp, H.dx, H.dy, H.dz, H.bc, H.bnode, H.bpn, H.bdep, H.bcc, H.bck, H.bon, H.boc, H.bok};
+        void *p[] = {H.u, H.f, H.r, H.rocp, H.dx, H.dy, H.dz, H.cx[0], H.cx[1], H.cy[0], H.cy[1], H.cz[0], H.cz[1], H.first, H.bc, H.bnode, H.bpn, H.bdep, H.bcc, H.bck, H.bon, H.boc, H.bok};
         for (void *q : p) cudaFree(q);
         if (l > 0) cudaFree(H.kt);
     }
@@ -469,31 +539,64 @@ static void hbc(i3g_ctx *c, int l, bool use_c)
 static void hsmooth(i3g_ctx *c, int l, int n, double dt, bool res)
 {
     Level &L = c->lev[l];
+    HeatLevel &H = hs(c)->L[l];
     HView V = hview(c, l, dt);
-    const long tot = (long)((L.ny + 1) / 2) * L.nx * L.nz;
+    const unsigned rows = nb((long)((L.ny + 1) / 2) * L.nx * L.nz);
+    const HBc B{H.nbc, H.na, (int)(l == 0), H.bnode, H.bpn, H.bdep, H.first, H.bcc, H.bck};
     for (int s = 0; s < n; s++) {
-        LAUNCH(k_heat_relax, nb(tot), 256, V, 0, c->p.t0koef);
-        LAUNCH(k_heat_relax, nb(tot), 256, V, 1, c->p.t0koef);
-        hbc(c, l, l == 0);
+        LAUNCH(k_heat_relax, rows, 256, V, 0, c->p.t0koef, B, rows);
+        LAUNCH(k_heat_relax, rows + (H.na >= 0 ? nb(H.nbc - H.na) : 0), 256, V, 1, c->p.t0koef, B, rows);
+        if (H.na < 0) hbc(c, l, l == 0);
     }
-    if (res) {
-        LAUNCH(k_heat_residual, nb(L.n), 256, V);
-        HeatLevel &H = hs(c)->L[l];
-        if (H.nbc) LAUNCH(k_heat_bc_res, nb(H.nbc), 256, (const double *)H.u, (const double *)H.f, H.r, H.nbc,
-                          (const int *)H.bnode, (const int *)H.bon, (const double *)H.bok);
-    }
+    if (res) LAUNCH(k_heat_residual, nb(L.n), 256, V);   // boundary rows' residuals are not restricted
 }
 
-static void hvcycle(i3g_ctx *c, double dt)
+// What one cycle does: levels 0..last, two sweeps per leg and coarse sweeps on the last.
+struct HeatPlan { int last, sweeps; };
+
+// From the largest k / (rho cp) kap and the step dt: the last level is the first one whose coupling
+// q = 2 dt kap (1/hx^2 + 1/hy^2 + 1/hz^2), h its smallest spacings, is at most 1 (or the coarsest).  A
+// coarse level keeps level 0's three outermost lines at each end; the cells between them stay narrow
+// on every level and are not counted there.  The last level's sweeps reduce its error by 1e-3, or by
+// the tolerance itself when it is level 0, at most 16 (12 on level 0, where the norm is cheap next to
+// the sweeps).  The solve repeats cycles until the tolerance is met, so the plan decides time, not the
+// result.  With dt = 0.3 h^2 / kap (levels 0 and 1) four heat steps on 65^3 nodes with 7.1 M markers
+// take 4.4 ms on B200, with every level 6.2.
+static HeatPlan heat_plan(i3g_ctx *c, double kap, double dt, double rtol)
 {
-    const int L = c->nlev - 1;
+    HeatPlan P{c->nlev - 1, 16};
+    double q = 0;
+    for (int l = 0; l < c->nlev; l++) {
+        const Level &L = c->lev[l];
+        const double *g[3] = {L.gx, L.gy, L.gz};
+        const int n[3] = {L.nx, L.ny, L.nz};
+        q = 0;
+        for (int d = 0; d < 3; d++) {
+            const int e = l > 0 && n[d] > 5 ? 2 : 0;
+            double h = g[d][1 + e] - g[d][e];
+            for (int i = 2 + e; i < n[d] - e; i++) h = std::min(h, g[d][i] - g[d][i - 1]);
+            q += 2.0 * dt * kap / (h * h);
+        }
+        P.last = l;
+        if (q <= 1.0) break;
+    }
+    const double rate = std::max(1e-6, q / (1.0 + q) * (q / (1.0 + q)));
+    const double need = std::log(P.last == 0 ? rtol : 1e-3) / std::log(rate);
+    P.sweeps = (int)std::min(P.last == 0 ? 12.0 : 16.0, std::max(2.0, std::ceil(need)));
+    if (!(q == q) || !(need == need)) P.sweeps = 16;
+    return P;
+}
+
+static void hvcycle(i3g_ctx *c, double dt, HeatPlan P)
+{
+    const int L = P.last;
     for (int l = 0; l < L; l++) {
         hsmooth(c, l, 2, dt, true);
         Level &F = c->lev[l];
         LAUNCH(k_heat_restrict, nb(c->lev[l + 1].n), 256, hview(c, l, dt), hview(c, l + 1, dt), trv(F.tr[0][kStagLine]),
                trv(F.tr[1][kStagLine]), trv(F.tr[2][kStagLine]));
     }
-    hsmooth(c, L, 16, dt, false);
+    hsmooth(c, L, P.sweeps, dt, false);
     for (int l = L; l > 0; l--) {
         Level &F = c->lev[l - 1];
         LAUNCH(k_heat_prolong, nb(F.n), 256, hview(c, l - 1, dt), hview(c, l, dt), trv(F.tr[0][kStagLine]),
@@ -536,16 +639,13 @@ int heat_solve(i3g_ctx *c, double *timestep)
     a.bc = H0.bc;
     a.tk0 = S->tk0; a.tk1 = S->tk1; a.tk2 = S->tk2; a.rocp = H0.rocp; a.u = H0.u; a.part = S->part;
     LAUNCH(k_heat_setup0, c->red_blocks, 256, a);
-    I3G_CUDA(cudaMemcpyAsync(c->hstage, S->part, sizeof(double) * c->red_blocks, cudaMemcpyDeviceToHost, c->st));
-    // coarse-level coefficients
-    for (int l = 1; l < c->nlev; l++) {
-        Level &F = c->lev[l - 1];
-        LAUNCH(k_heat_coef_restrict, nb(c->lev[l].n), 256, hview(c, l - 1, 1.0), hview(c, l, 1.0), S->L[l].kt, S->L[l].rocp,
-               trv(F.tr[0][kStagAbs]), trv(F.tr[1][kStagAbs]), trv(F.tr[2][kStagAbs]));
-    }
+    I3G_CUDA(cudaMemcpyAsync(c->hstage, S->part, sizeof(double) * 2 * c->red_blocks, cudaMemcpyDeviceToHost, c->st));
     I3G_CUDA(cudaStreamSynchronize(c->st));
-    double maxrate = 0;
-    for (int b = 0; b < c->red_blocks; b++) maxrate = std::max(maxrate, c->hstage[b]);
+    double maxrate = 0, kap = 0;
+    for (int b = 0; b < c->red_blocks; b++) {
+        maxrate = std::max(maxrate, c->hstage[2 * b]);
+        kap = std::max(kap, c->hstage[2 * b + 1]);
+    }
     double tkstep = 1e30;
     if (maxrate > 0) tkstep = c->f.maxtkstep / maxrate;
     if (*timestep == 0 || tkstep == 0) return 0;
@@ -553,7 +653,7 @@ int heat_solve(i3g_ctx *c, double *timestep)
     double done = 0, rel = 0;
     const double rtol = c->p.heat_rtol > 0 ? c->p.heat_rtol : 1e-10;
     const int maxc = c->p.heat_maxcyc > 0 ? c->p.heat_maxcyc : 2000;
-    int cycles = 0, subs = 0;
+    int cycles = 0, subs = 0, built = 0;
     do {
         double dt = std::min(total, tkstep);
         if (dt > total - done) dt = total - done;
@@ -561,9 +661,15 @@ int heat_solve(i3g_ctx *c, double *timestep)
                (const double *)H0.rocp, (const uint8_t *)H0.bc, H0.u, H0.f, dt);
         if (H0.nbc) LAUNCH(k_bc_rhs_heat, nb(H0.nbc), 256, H0.f, H0.nbc, (const int *)H0.bnode, (const double *)H0.boc);
         hbc(c, 0, true);
+        const HeatPlan plan = heat_plan(c, kap, dt, rtol);
+        for (; built < plan.last; built++) {   // coefficients of the coarse levels in use
+            Level &F = c->lev[built];
+            LAUNCH(k_heat_coef_restrict, nb(c->lev[built + 1].n), 256, hview(c, built, 1.0), hview(c, built + 1, 1.0), S->L[built + 1].kt,
+                   S->L[built + 1].rocp, trv(F.tr[0][kStagAbs]), trv(F.tr[1][kStagAbs]), trv(F.tr[2][kStagAbs]));
+        }
         int it = 0;
         for (;;) {
-            hvcycle(c, dt);
+            hvcycle(c, dt, plan);
             it++;
             int rc = hrelres(c, dt, &rel);
             if (rc) return rc;
@@ -602,12 +708,13 @@ int heat_time_kernel(i3g_ctx *c, int reps, double *ms, double *bytes)
 {
     Level &L0 = c->lev[0];
     HView V = hview(c, 0, 1e13);
-    const long tot = (long)((L0.ny + 1) / 2) * L0.nx * L0.nz;
+    const unsigned rows = nb((long)((L0.ny + 1) / 2) * L0.nx * L0.nz);
+    const HBc B{};
     // one full sweep (both colours) with an empty L2; 32 B per node: T read and written (FP64),
     // k and rho cp (FP32), right-hand side (FP64)
     int rc = cold_time(c, reps, [&]() -> int {
-        LAUNCH(k_heat_relax, nb(tot), 256, V, 0, 1.0);
-        LAUNCH(k_heat_relax, nb(tot), 256, V, 1, 1.0);
+        LAUNCH(k_heat_relax, rows, 256, V, 0, 1.0, B, rows);
+        LAUNCH(k_heat_relax, rows, 256, V, 1, 1.0, B, rows);
         return 0;
     }, ms);
     if (rc) return rc;

@@ -195,6 +195,37 @@ def test_marker_rheology_reads_what_it_needs(exact):
     np.testing.assert_allclose(a.f32["markv"], b.f32["markv"], rtol=2e-7)
 
 
+@pytest.mark.parametrize("factor", [None, 0.5])
+@pytest.mark.parametrize("scale", [1e-2, 1.0, 30.0])
+def test_heat_from_uncoupled_to_stiff(scale, factor):
+    """Steps far below and far above the cells' diffusion time (level 0 alone, and all levels), with
+    the boundary rows' own factors and with 1/2.  The matrix has row sums rho cp / dt, so two solutions
+    with relative residuals 1e-13 agree to a few 1e-12; both are stored as FP32."""
+    out = []
+    for side in range(2):
+        p, mode, fx, _ = marker_setup("sphere13")
+        if factor is not None:
+            b = p.bond
+            heat = (b["row"] >= 8 * p.nodenum) & (b["partner1"] > 0)
+            assert heat.sum() > 100
+            b["k"][heat] = factor
+        buf = abi.ModelBuffers(p)
+        par, fp = abi.make_params(mode, heat_rtol=1e-13), abi.make_file_params(mode.files[0])
+        fp.maxtkstep = 1e9
+        dt = float(fx["fld_dt"][0]) * scale
+        c = lib.Context(buf, par, fp) if side == 0 else O.Oracle(buf, par, fp)
+        if side == 0:
+            c.heat(0, dt)
+            assert c.stats()["heat_rel"] <= 1e-13
+        else:
+            c.call("orc_heat", (O.C.c_double * 1)(dt))
+        c.download(abi.SYNC_ALL)
+        c.close()
+        out.append(buf.f32["tk"].copy())
+    assert np.all(np.isfinite(out[1]))
+    np.testing.assert_allclose(out[0], out[1], rtol=2e-7, atol=0)
+
+
 @pytest.mark.parametrize("cin,cout", [(32, 32), (32, 64), (64, 32), (64, 64), (64, 128), (128, 64), (128, 128)])
 @pytest.mark.parametrize("dims", [(1, 1, 1), (10, 11, 14), (15, 17, 19), (27, 25, 29)])
 def test_wide_convolutions_for_every_channel_split(dims, cin, cout):
