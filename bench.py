@@ -469,7 +469,7 @@ def main():
               "one level-0 multicolour sweep, %s (k_relax_vel x6, k_relax_p, boundary rows)" % ("FP32" if prec else "FP64"),
               "68 B/node FP32" if prec else "116 B/node FP64"),
              ("k_move", 5, 1.0, "RK4 marker advection", "45 B/marker + 13 nodal FP32 fields"),
-             ("k_r2n_cells", 4, 1.0, "marker -> node sums", "25 B/marker + 48 B/node"),
+             ("k_r2n_mma", 4, 1.0, "marker -> node sums", "25 B/marker + 48 B/node"),
              ("k_heat_mark_cells", 9, 1.0, "marker temperature update", "42 B/marker"),
              ("heat_sweep", 6, 4.0 * heat_cyc, "one level-0 heat sweep (k_heat_relax x2)", "32 B/node")]
     kernels = []
