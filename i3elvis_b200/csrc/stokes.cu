@@ -2744,7 +2744,9 @@ static size_t smtail_args(i3g_ctx *c, int lc, int multinum, SmTailArgs<T> *a)
 }
 
 // First level of the on-chip tail: as many of the coarsest levels (>= 1) as fit one SM's shared memory
-// and have up to kSmTailNodes nodes (FP64: the coarsest alone, whose transfers keep the oracle's order); multinum + 1 when none.
+// and have up to kSmTailNodes nodes; multinum + 1 when none.  FP64 takes the coarsest alone, since its
+// transfers keep the oracle's order; with the level above launched again a FP64 V-cycle of 15^3, 17^3,
+// 27^3 and 33^3 nodes takes 1.19, 1.25, 1.42 and 1.66 ms, in the general tail 1.29, 1.49, 1.65 and 2.21.
 template <typename T>
 static int smtail_start(i3g_ctx *c, int multinum)
 {
