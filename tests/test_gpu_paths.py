@@ -70,6 +70,24 @@ def test_vcycles_bit_exact_on_boxes(shape, multinum, pro, monkeypatch):
     _vcycles_match(*_random_box(shape, multinum, seed=sum(shape)))
 
 
+def test_vcycles_of_a_level_beyond_the_row_indexed_table(monkeypatch):
+    """Level 1 has 456,225 nodes: its packed boundary entries are found through the writer list, not the
+    table indexed by the row.  Bit for bit the same as one launch per boundary pass."""
+    sols = []
+    for fuse in ("1", "0"):
+        monkeypatch.setenv("I3G_FUSE", fuse)
+        p, mode = _random_box((149, 145, 153), 1, seed=7)
+        assert cases.level_sizes(p, 1)[1] > 400000
+        g = lib.Context(abi.ModelBuffers(p), abi.make_params(mode), abi.make_file_params(mode.files[0]))
+        g.call("i3g_stokes_setup")
+        g.call("i3g_stokes_vcycles", 1)
+        sols.append([g.get(abi.A_SOL, l, 4 * n) for l, n in enumerate(cases.level_sizes(p, 1))])
+        g.close()
+    for a, b in zip(*sols):
+        assert np.all(np.isfinite(a)) and np.any(a != 0)
+        assert np.array_equal(a, b)
+
+
 def _cloud(seed=5):
     """Reference fields of the 13^3 case with markers of every rock moved to uneven places: empty cells,
     cells of a few markers and cells of several hundred (more than a warp stages at once)."""
