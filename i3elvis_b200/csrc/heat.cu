@@ -7,15 +7,16 @@
 // residual, trilinear prolongation, and conductivity / heat capacity restricted with the
 // viscosity-restriction weights.  The converged temperature is that of the reference's rows.
 //
-// How many levels a solve needs follows from its coupling: with q the ratio of a row's neighbour
-// coefficients to its rho cp / dt, a red-black sweep reduces the error by (q / (1 + q))^2 at worst.
-// A time step limited by the flow has q far below 1 (0.1 on the benchmark model), where sweeps on
-// level 0 alone reach the tolerance and coarser levels would only add launches; q falls fourfold per
-// level, and the hierarchy is used down to the first level with q <= 1 (heat_plan).
+// How many levels a solve needs follows from its coupling (heat_plan.h): a time step limited by the
+// flow has a ratio q of a row's neighbour coefficients to its rho cp / dt far below 1 (0.1 on the
+// benchmark model), where sweeps on level 0 alone reach the tolerance and coarser levels would only
+// add launches; q falls fourfold per level, and the hierarchy is used down to the first level with
+// q <= 1.
 #include <algorithm>
 #include <cmath>
 #include <vector>
 #include "heat_markers.cuh"
+#include "heat_plan.h"
 
 namespace i3g {
 
@@ -551,40 +552,27 @@ static void hsmooth(i3g_ctx *c, int l, int n, double dt, bool res)
     if (res) LAUNCH(k_heat_residual, nb(L.n), 256, V);   // boundary rows' residuals are not restricted
 }
 
-// What one cycle does: levels 0..last, two sweeps per leg and coarse sweeps on the last.
-struct HeatPlan { int last, sweeps; };
-
-// From the largest k / (rho cp) kap and the step dt: the last level is the first one whose coupling
-// q = 2 dt kap (1/hx^2 + 1/hy^2 + 1/hz^2), h its smallest spacings, is at most 1 (or the coarsest).  A
-// coarse level keeps level 0's three outermost lines at each end; the cells between them stay narrow
-// on every level and are not counted there.  The last level's sweeps reduce its error by 1e-3, or by
-// the tolerance itself when it is level 0, at most 16 (12 on level 0, where the norm is cheap next to
-// the sweeps).  The solve repeats cycles until the tolerance is met, so the plan decides time, not the
-// result.  With dt = 0.3 h^2 / kap (levels 0 and 1) four heat steps on 65^3 nodes with 7.1 M markers
-// take 4.4 ms on B200, with every level 6.2.
-static HeatPlan heat_plan(i3g_ctx *c, double kap, double dt, double rtol)
+// Coupling of every level, from the largest k / (rho cp) kap of level 0's nodes and the step dt:
+// q = 2 dt kap (1/hx^2 + 1/hy^2 + 1/hz^2), h the level's smallest spacings.  A coarse level keeps level
+// 0's three outermost lines at each end; the cells between them stay narrow on every level and are
+// not counted there.  A row beside a much better conductor couples more strongly than its own k says,
+// and the damping of the coarse averages is not in it: an estimate, which heat_solve checks.  With dt =
+// 0.3 h^2 / kap (levels 0 and 1) four heat steps on 65^3 nodes with 7.1 M markers take 4.4 ms on B200,
+// with every level 6.2.
+static void heat_coupling(i3g_ctx *c, double kap, double dt, double *qs)
 {
-    HeatPlan P{c->nlev - 1, 16};
-    double q = 0;
     for (int l = 0; l < c->nlev; l++) {
         const Level &L = c->lev[l];
         const double *g[3] = {L.gx, L.gy, L.gz};
         const int n[3] = {L.nx, L.ny, L.nz};
-        q = 0;
+        qs[l] = 0;
         for (int d = 0; d < 3; d++) {
             const int e = l > 0 && n[d] > 5 ? 2 : 0;
             double h = g[d][1 + e] - g[d][e];
             for (int i = 2 + e; i < n[d] - e; i++) h = std::min(h, g[d][i] - g[d][i - 1]);
-            q += 2.0 * dt * kap / (h * h);
+            qs[l] += 2.0 * dt * kap / (h * h);
         }
-        P.last = l;
-        if (q <= 1.0) break;
     }
-    const double rate = std::max(1e-6, q / (1.0 + q) * (q / (1.0 + q)));
-    const double need = std::log(P.last == 0 ? rtol : 1e-3) / std::log(rate);
-    P.sweeps = (int)std::min(P.last == 0 ? 12.0 : 16.0, std::max(2.0, std::ceil(need)));
-    if (!(q == q) || !(need == need)) P.sweeps = 16;
-    return P;
 }
 
 static void hvcycle(i3g_ctx *c, double dt, HeatPlan P)
@@ -661,20 +649,24 @@ int heat_solve(i3g_ctx *c, double *timestep)
                (const double *)H0.rocp, (const uint8_t *)H0.bc, H0.u, H0.f, dt);
         if (H0.nbc) LAUNCH(k_bc_rhs_heat, nb(H0.nbc), 256, H0.f, H0.nbc, (const int *)H0.bnode, (const double *)H0.boc);
         hbc(c, 0, true);
-        const HeatPlan plan = heat_plan(c, kap, dt, rtol);
-        for (; built < plan.last; built++) {   // coefficients of the coarse levels in use
-            Level &F = c->lev[built];
-            LAUNCH(k_heat_coef_restrict, nb(c->lev[built + 1].n), 256, hview(c, built, 1.0), hview(c, built + 1, 1.0), S->L[built + 1].kt,
-                   S->L[built + 1].rocp, trv(F.tr[0][kStagAbs]), trv(F.tr[1][kStagAbs]), trv(F.tr[2][kStagAbs]));
-        }
+        double qs[I3G_MAXLEV];
+        heat_coupling(c, kap, dt, qs);
+        HeatPlan plan = heat_plan(qs, c->nlev, c->p.t0koef, rtol);
         int it = 0;
         for (;;) {
+            for (; built < plan.last; built++) {   // coefficients of the coarse levels in use
+                Level &F = c->lev[built];
+                LAUNCH(k_heat_coef_restrict, nb(c->lev[built + 1].n), 256, hview(c, built, 1.0), hview(c, built + 1, 1.0), S->L[built + 1].kt,
+                       S->L[built + 1].rocp, trv(F.tr[0][kStagAbs]), trv(F.tr[1][kStagAbs]), trv(F.tr[2][kStagAbs]));
+            }
             hvcycle(c, dt, plan);
             it++;
+            const double before = rel;
             int rc = hrelres(c, dt, &rel);
             if (rc) return rc;
             if (!(rel == rel)) return set_error(c, I3G_E_NAN, "NaN in the heat solve");
             if (rel <= rtol || it >= maxc) break;
+            if (it > 1 && rel > kHeatPlanFactor * before) plan = heat_plan_full(c->nlev);
         }
         cycles += it;
         LAUNCH(k_heat_store, nb(L0.n), 256, L0.n, (const double *)H0.u, c->tk);

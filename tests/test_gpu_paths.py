@@ -244,6 +244,62 @@ def test_heat_from_uncoupled_to_stiff(scale, factor):
     np.testing.assert_allclose(out[0], out[1], rtol=2e-7, atol=0)
 
 
+def _heat(edit, dt_scale, side, **kw):
+    """One heat step of the 13^3 case, dt_scale times its time step, on the GPU (side 0) or the oracle."""
+    p, mode, fx, _ = marker_setup("sphere13")
+    edit(p)
+    buf = abi.ModelBuffers(p)
+    par, fp = abi.make_params(mode, heat_rtol=kw.pop("heat_rtol")), abi.make_file_params(mode.files[0])
+    for f, v in kw.items():
+        setattr(par, f, v)
+    fp.maxtkstep = 1e30
+    dt = float(fx["fld_dt"][0]) * dt_scale
+    c = lib.Context(buf, par, fp) if side == 0 else O.Oracle(buf, par, fp)
+    stats = None
+    if side == 0:
+        c.heat(0, dt)
+        stats = c.stats()
+    else:
+        c.call("orc_heat", (O.C.c_double * 1)(dt))
+    c.download(abi.SYNC_ALL)
+    c.close()
+    return buf.f32["tk"].copy(), stats
+
+
+def test_heat_with_a_node_without_heat_capacity():
+    """A node with rho cp = 0 makes the largest k / (rho cp) infinite: the stiff step takes as many cycles as
+    with a heat capacity that is merely tiny there."""
+    cycles = []
+    for cp in (1e-9, 0.0):
+        def edit(p):
+            nx, ny, nz = p.shape
+            p.nodes["ht"][:] = 0
+            p.nodes["cp"][(nz // 2 * nx + nx // 2) * ny + ny // 2] = cp
+        got, stats = _heat(edit, 1e3, 0, heat_rtol=1e-10, frictyn=0)
+        assert np.all(np.isfinite(got)) and stats["heat_rel"] <= 1e-10
+        cycles.append(stats["heat_cycles"])
+    assert abs(cycles[1] - cycles[0]) <= 1, cycles
+
+
+@pytest.mark.parametrize("t0koef", [1.0, 0.8, 1.3])
+@pytest.mark.parametrize("scale", [0.1, 3.0])
+def test_heat_of_strong_contrasts(scale, t0koef):
+    """Good conductors (k and rho cp 1000 times larger) beside poor ones node by node: rows couple more strongly
+    than their own k / (rho cp) says, with and without damping.  The matrix has row sums rho cp / dt of
+    ratio 1000, so two solutions with relative residuals 1e-13 agree to a few 1e-9; both are stored as FP32."""
+    def edit(p):
+        nx, ny, nz = p.shape
+        z, x, y = np.meshgrid(np.arange(nz), np.arange(nx), np.arange(ny), indexing="ij")
+        good = ((x + y + z) & 1).reshape(-1) == 1
+        for f in ("kt", "cp"):
+            p.nodes[f] = np.where(good, 1000 * p.nodes[f], p.nodes[f]).astype(np.float32)
+    got, stats = _heat(edit, scale, 0, heat_rtol=1e-13, t0koef=t0koef)
+    assert stats["heat_rel"] <= 1e-13
+    want, _ = _heat(edit, scale, 1, heat_rtol=1e-13)
+    assert np.all(np.isfinite(want))
+    np.testing.assert_allclose(got, want, rtol=2e-7, atol=0)
+
+
 @pytest.mark.parametrize("cin,cout", [(32, 32), (32, 64), (64, 32), (64, 64), (64, 128), (128, 64), (128, 128)])
 @pytest.mark.parametrize("dims", [(1, 1, 1), (10, 11, 14), (15, 17, 19), (27, 25, 29)])
 def test_wide_convolutions_for_every_channel_split(dims, cin, cout):
