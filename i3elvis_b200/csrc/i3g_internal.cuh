@@ -104,10 +104,12 @@ struct Transfer1D {
     double *w0 = nullptr, *w1 = nullptr;
     int *gptr = nullptr, *gf = nullptr;
     double *gw = nullptr;
-    // compact FP32 form (stokes.cu, CtView): four fine indices from cs[c] with weights cw[c]; cv[f]
-    bool compact = false;
+    // compact FP32 form (stokes.cu, CtView): four fine indices from cs[c] with weights cw[c], or five with
+    // cw5[c] (compact = 4 or 5; 0: none); cv[f]
+    int compact = 0;
     int *cs = nullptr;
     float4 *cw = nullptr;
+    float *cw5 = nullptr;
     float2 *cv = nullptr;
 };
 
@@ -134,7 +136,8 @@ struct Level {
     Fields<double> d;
     Fields<float> s;                    // scaled FP32 copy for the mixed-precision solver
     SmTailRows sm;
-    bool compact = false;               // FP32 transfers from and to the finer level in compact form
+    int compact = 0;                    // FP32 transfers from and to the finer level in compact form: fine
+                                        // indices per axis, 4 or 5 (0: general transfers)
     float *iws[4] = {nullptr, nullptr, nullptr, nullptr};   // 1 / sum of restriction weights
     BcList bcl[4];
     Transfer1D tr[3][4];               // to the next coarser level: axis x,y,z; staggering

@@ -811,6 +811,10 @@ __global__ void __launch_bounds__(256) k_restrict(View<T> F, View<T> Cc, TrView 
 // which never change, are a table: the inner loop is four loads and four multiply-adds per line where
 // the general kernel walks index lists and FP64 weights and tests the boundary byte of up to 64
 // contributors (a V-cycle on 129^3 went from 1.47 to 1.33 ms, on 65^3 from 0.49 to 0.46, on B200).
+// Where the finer level has an even number of nodes the kept outer lines meet the halved spacing out of
+// step and a coarse index near the end gathers from five: w5 holds the fifth weight, of s[c] + 4 (W =
+// 5 in the kernels; one pair of levels in four on uniform grids of 9 to 259 lines; a V-cycle takes 1.24
+// ms instead of 1.29 with the general transfers there on 129^3, 0.41 instead of 0.45 on 59^3).
 struct CtView {
     const int *s, *a;
     const float4 *w;
@@ -820,9 +824,12 @@ struct Ct4 {
     CtView t[4][3];      // [component][axis]
     const float *iws[4]; // [component]: 1 / sum of weights per coarse node
 };
+struct Ct5 {
+    const float *w5[4][3];   // [component][axis]: fifth weights
+};
 
-template <int V>
-__device__ __forceinline__ void restrict_compact(const View<float> &F, const View<float> &Cc, const Ct4 &R, long n)
+template <int V, int W>
+__device__ __forceinline__ void restrict_compact(const View<float> &F, const View<float> &Cc, const Ct4 &R, const Ct5 &R5, long n)
 {
     int i, j, k;
     node_ijk(Cc, n, i, j, k);
@@ -833,15 +840,21 @@ __device__ __forceinline__ void restrict_compact(const View<float> &F, const Vie
     if (!row_exists(V, i, j, k, Cc.nx, Cc.ny, Cc.nz) || (Cc.bc[n] & (1 << V))) { cf_[n] = 0.f; return; }
     const float4 wx = __ldg(R.t[V][0].w + i), wy = __ldg(R.t[V][1].w + j), wz = __ldg(R.t[V][2].w + k);
     const float *p = fr + (long)__ldg(R.t[V][2].s + k) * F.nxy + (long)__ldg(R.t[V][0].s + i) * F.ny + __ldg(R.t[V][1].s + j);
-    const float x[4] = {wx.x, wx.y, wx.z, wx.w}, z[4] = {wz.x, wz.y, wz.z, wz.w};
+    const bool wide = W == 5;
+    const float x[5] = {wx.x, wx.y, wx.z, wx.w, wide ? __ldg(R5.w5[V][0] + i) : 0.f};
+    const float z[5] = {wz.x, wz.y, wz.z, wz.w, wide ? __ldg(R5.w5[V][2] + k) : 0.f};
+    const float y4 = wide ? __ldg(R5.w5[V][1] + j) : 0.f;
     float sum = 0.f;
 #pragma unroll
-    for (int ez = 0; ez < 4; ez++) {
+    for (int ez = 0; ez < W; ez++) {
+        if (ez == 4 && z[4] == 0.f) break;   // no fifth line: it may lie outside the level
         float sx = 0.f;
 #pragma unroll
-        for (int ex = 0; ex < 4; ex++) {
+        for (int ex = 0; ex < W; ex++) {
+            if (ex == 4 && x[4] == 0.f) break;
             const float *q = p + ez * F.nxy + ex * F.ny;
             sx += x[ex] * (wy.x * q[0] + wy.y * q[1] + wy.z * q[2] + wy.w * q[3]);
+            if (wide && y4 != 0.f) sx += x[ex] * (y4 * q[4]);
         }
         sum += z[ez] * sx;
     }
@@ -851,35 +864,42 @@ __device__ __forceinline__ void restrict_compact(const View<float> &F, const Vie
 
 // four CTAs per SM (64 registers): the 64 loads of a row wait on L2, a V-cycle on 129^3 takes 1.284 ms
 // against 1.296 with the 94 registers the compiler would take
-__global__ void __launch_bounds__(256, 4) k_restrict_f32(View<float> F, View<float> Cc, Ct4 R)
+template <int W>
+__global__ void __launch_bounds__(256, 4) k_restrict_f32(View<float> F, View<float> Cc, Ct4 R, Ct5 R5)
 {
     pdl_enter();
     const long n = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (n >= Cc.nxy * Cc.nz) return;
     switch (blockIdx.y) {
-    case 0: restrict_compact<0>(F, Cc, R, n); break;
-    case 1: restrict_compact<1>(F, Cc, R, n); break;
-    case 2: restrict_compact<2>(F, Cc, R, n); break;
-    default: restrict_compact<3>(F, Cc, R, n); break;
+    case 0: restrict_compact<0, W>(F, Cc, R, R5, n); break;
+    case 1: restrict_compact<1, W>(F, Cc, R, R5, n); break;
+    case 2: restrict_compact<2, W>(F, Cc, R, R5, n); break;
+    default: restrict_compact<3, W>(F, Cc, R, R5, n); break;
     }
 }
 
 // 1 / sum of the weights of the fine rows a coarse row gathers (set-up)
-__global__ void k_restrict_iws(int V, const uint8_t *fbc, int fnx, int fny, int fnz, int cnx, int cny, int cnz, CtView tx, CtView ty,
-                               CtView tz, float *iws)
+struct Axis5 {
+    const int *s;
+    const float4 *w;
+    const float *w5;
+    __device__ float at(int c, int e) const { return e == 4 ? w5[c] : (&w[c].x)[e]; }
+};
+__global__ void k_restrict_iws(int V, const uint8_t *fbc, int fnx, int fny, int fnz, int cnx, int cny, int cnz, Axis5 tx, Axis5 ty,
+                               Axis5 tz, float *iws)
 {
     const long n = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (n >= (long)cnx * cny * cnz) return;
     const int j = (int)(n % cny), i = (int)((n / cny) % cnx), k = (int)(n / ((long)cnx * cny));
-    const float4 wx = tx.w[i], wy = ty.w[j], wz = tz.w[k];
-    const float x[4] = {wx.x, wx.y, wx.z, wx.w}, y[4] = {wy.x, wy.y, wy.z, wy.w}, z[4] = {wz.x, wz.y, wz.z, wz.w};
     double ws = 0;
-    for (int ez = 0; ez < 4; ez++)
-        for (int ex = 0; ex < 4; ex++)
-            for (int ey = 0; ey < 4; ey++) {
+    for (int ez = 0; ez < 5; ez++)
+        for (int ex = 0; ex < 5; ex++)
+            for (int ey = 0; ey < 5; ey++) {
+                const float x = tx.at(i, ex), y = ty.at(j, ey), z = tz.at(k, ez);
+                if (x == 0.f || y == 0.f || z == 0.f) continue;   // also entries past the table's four
                 const int fk = tz.s[k] + ez, fi = tx.s[i] + ex, fj = ty.s[j] + ey;
                 if (!row_exists(V, fi, fj, fk, fnx, fny, fnz) || (fbc[((long)fk * fnx + fi) * fny + fj] & (1 << V))) continue;
-                ws += (double)x[ex] * y[ey] * z[ez];
+                ws += (double)x * y * z;
             }
     iws[n] = ws != 0 ? (float)(1.0 / ws) : 1.f;
 }
@@ -1898,15 +1918,19 @@ static void build_transfer(const double *gf, int nf, const double *gc, int nc, i
     t.nf = nf; t.nc = nc;
 }
 
-// The compact form of one axis (CtView): false when a coarse index gathers from more than four
-// consecutive fine indices
-static bool compact_transfer(int nf, int nc, const std::vector<int> &ha, const std::vector<double> &w0, const std::vector<double> &w1,
-                             std::vector<int> &cs, std::vector<float4> &cw, std::vector<float2> &cv)
+// The compact form of one axis (CtView): the number of consecutive fine indices a coarse index gathers
+// from, 4 or 5, and 0 when it is more.  Grid lines are stored in FP32, so staggered points that
+// coincide miss each other by their rounding: on uniform grids of 9 to 259 lines the weights are either
+// below 8e-6, from such points, or above 6e-3.  One below kNoWeight counts as none.
+constexpr double kNoWeight = 1e-4;
+static int compact_transfer(int nf, int nc, const std::vector<int> &ha, const std::vector<double> &w0, const std::vector<double> &w1,
+                            std::vector<int> &cs, std::vector<float4> &cw, std::vector<float> &cw5, std::vector<float2> &cv)
 {
     cs.assign(nc, 0);
     cw.assign(nc, make_float4(0, 0, 0, 0));
+    cw5.assign(nc, 0.f);
     cv.resize(nf);
-    if (nf < 4) return false;
+    if (nf < 4) return 0;
     std::vector<int> lo(nc, nf), hi(nc, -1);
     std::vector<std::vector<std::pair<int, float>>> lists(nc);
     for (int m = 0; m < nf; m++) {
@@ -1914,21 +1938,26 @@ static bool compact_transfer(int nf, int nc, const std::vector<int> &ha, const s
         for (int q = 0; q < 2; q++) {
             const int k = ha[m] + q;
             const double w = q ? w1[m] : w0[m];
-            if (k < 0 || k >= nc || w == 0.0) continue;
+            if (k < 0 || k >= nc || std::fabs(w) < kNoWeight) continue;
             lists[k].push_back({m, (float)w});
             lo[k] = std::min(lo[k], m);
             hi[k] = std::max(hi[k], m);
         }
-        if (ha[m] < 0 || ha[m] > nc - 2) return false;
+        if (ha[m] < 0 || ha[m] > nc - 2) return 0;
     }
+    int width = 4;
     for (int k = 0; k < nc; k++) {
         if (lists[k].empty()) continue;
         cs[k] = std::min(lo[k], nf - 4);
-        if (hi[k] - cs[k] > 3) return false;
-        float *w = &cw[k].x;
-        for (auto &e : lists[k]) w[e.first - cs[k]] += e.second;
+        if (hi[k] - cs[k] > 4) return 0;
+        if (hi[k] - cs[k] == 4) width = 5;
+        for (auto &e : lists[k]) {
+            const int d = e.first - cs[k];
+            if (d == 4) cw5[k] += e.second;
+            else (&cw[k].x)[d] += e.second;
+        }
     }
-    return true;
+    return width;
 }
 
 static int upload_transfer(i3g_ctx *c, const double *gf, int nf, const double *gc, int nc, int stag, Transfer1D &t)
@@ -1939,9 +1968,11 @@ static int upload_transfer(i3g_ctx *c, const double *gf, int nf, const double *g
     int rc;
     std::vector<int> cs;
     std::vector<float4> cw;
+    std::vector<float> cw5;
     std::vector<float2> cv;
-    t.compact = compact_transfer(nf, nc, ha, w0, w1, cs, cw, cv);
-    if (t.compact && ((rc = upload(c, t.cs, cs)) || (rc = upload(c, t.cw, cw)) || (rc = upload(c, t.cv, cv)))) return rc;
+    t.compact = compact_transfer(nf, nc, ha, w0, w1, cs, cw, cw5, cv);
+    if (t.compact && ((rc = upload(c, t.cs, cs)) || (rc = upload(c, t.cw, cw)) || (rc = upload(c, t.cw5, cw5)) || (rc = upload(c, t.cv, cv))))
+        return rc;
     if ((rc = upload(c, t.a, ha)) || (rc = upload(c, t.w0, w0)) || (rc = upload(c, t.w1, w1)) ||
         (rc = upload(c, t.gptr, gptr)) || (rc = upload(c, t.gf, gfv)) || (rc = upload(c, t.gw, gwv)))
         return rc;
@@ -2361,13 +2392,21 @@ int stokes_alloc(i3g_ctx *c)
     if (rc) return rc;
     for (int l = 1; l < c->nlev; l++) {   // weight sums of the FP32 restriction to level l
         Level &F = c->lev[l - 1], &Cc = c->lev[l];
-        Cc.compact = c->fuse != 0;
+        Cc.compact = c->fuse != 0 ? 4 : 0;
         for (int v = 0; v < 4; v++)
-            for (int ax = 0; ax < 3; ax++) Cc.compact = Cc.compact && F.tr[ax][kStag[v][ax]].compact;
+            for (int ax = 0; ax < 3; ax++) {
+                const int w = F.tr[ax][kStag[v][ax]].compact;
+                Cc.compact = Cc.compact && w ? std::max(Cc.compact, w) : 0;
+            }
+        if (getenv("I3G_TRACE")) fprintf(stderr, "i3g: FP32 transfers to level %d: %d fine indices an axis\n", l, Cc.compact);
         for (int v = 0; Cc.compact && v < 4; v++) {
+            Axis5 ax[3];
+            for (int d = 0; d < 3; d++) {
+                const Transfer1D &t = F.tr[d][kStag[v][d]];
+                ax[d] = Axis5{t.cs, t.cw, t.cw5};
+            }
             ALLOC(Cc.iws[v], float, Cc.n);
-            k_restrict_iws<<<nblk(Cc.n), 256, 0, c->st>>>(v, F.bc, F.nx, F.ny, F.nz, Cc.nx, Cc.ny, Cc.nz, ctview(F.tr[0][kStag[v][0]]),
-                                                          ctview(F.tr[1][kStag[v][1]]), ctview(F.tr[2][kStag[v][2]]), Cc.iws[v]);
+            k_restrict_iws<<<nblk(Cc.n), 256, 0, c->st>>>(v, F.bc, F.nx, F.ny, F.nz, Cc.nx, Cc.ny, Cc.nz, ax[0], ax[1], ax[2], Cc.iws[v]);
             c->launches++;
         }
     }
@@ -2411,7 +2450,7 @@ void stokes_free(i3g_ctx *c)
             for (int s = 0; s < 4; s++) {
                 Transfer1D &t = L.tr[d][s];
                 cudaFree(t.a); cudaFree(t.w0); cudaFree(t.w1); cudaFree(t.gptr); cudaFree(t.gf); cudaFree(t.gw);
-                cudaFree(t.cs); cudaFree(t.cw); cudaFree(t.cv);
+                cudaFree(t.cs); cudaFree(t.cw); cudaFree(t.cw5); cudaFree(t.cv);
             }
         for (int v = 0; v < 4; v++) cudaFree(L.iws[v]);
         cudaFree(L.sm.ent); cudaFree(L.sm.cst); cudaFree(L.sm.first);
@@ -2594,7 +2633,11 @@ static void restrict_t(i3g_ctx *c, int l)
     View<T> VF = view<T>(F, fields<T>(F)), VC = view<T>(Cc, fields<T>(Cc));
     if constexpr (std::is_same<T, float>::value)
         if (Cc.compact) {
-            LAUNCH(k_restrict_f32, dim3(nblk(Cc.n), 4), 256, VF, VC, ct4(F, Cc));
+            Ct5 R5;
+            for (int v = 0; v < 4; v++)
+                for (int ax = 0; ax < 3; ax++) R5.w5[v][ax] = F.tr[ax][kStag[v][ax]].cw5;
+            if (Cc.compact == 4) LAUNCH(k_restrict_f32<4>, dim3(nblk(Cc.n), 4), 256, VF, VC, ct4(F, Cc), R5);
+            else LAUNCH(k_restrict_f32<5>, dim3(nblk(Cc.n), 4), 256, VF, VC, ct4(F, Cc), R5);
             return;
         }
     if (c->fuse) {
@@ -2724,7 +2767,7 @@ static size_t smtail_args(i3g_ctx *c, int lc, int multinum, SmTailArgs<T> *a)
     }
     for (int q = 0; q < nl; q++) {
         Level &L = c->lev[lc + q];
-        if (!L.sm.ok || (q + 1 < nl && !c->lev[lc + q + 1].compact)) return 0;
+        if (!L.sm.ok || (q + 1 < nl && c->lev[lc + q + 1].compact != 4)) return 0;
         const size_t N = (size_t)L.n;
         SmTailLevel<T> G;
         memset((void *)&G, 0, sizeof G);

@@ -342,3 +342,33 @@ def test_fp32_cycles_of_every_tail_and_transfer(name, monkeypatch):
         assert abs(cycles[q] - cycles[0]) <= 1 + cycles[0] // 10, cycles
         for k in (1, 2, 3):
             assert np.linalg.norm(sols[q][:, k] - sols[0][:, k]) <= 1e-6 * np.linalg.norm(sols[0][:, k])
+
+
+@pytest.mark.parametrize("shape,multinum,widths", [((21, 21, 21), 2, [4, 4]), ((23, 23, 23), 2, [4, 4]), ((43, 21, 23), 3, [4, 4, 5]),
+                                                   ((27, 43, 35), 3, [4, 4, 5]), ((51, 51, 51), 3, [4, 4, 5])])
+def test_fp32_transfers_are_compact_on_every_grid(shape, multinum, widths, capfd, monkeypatch):
+    """Coarse lines that gather from four or five fine ones, on grids whose FP32-rounded lines leave weights of
+    1e-6 at coinciding points: every level takes the compact transfers, and the FP32 cycle preconditions as
+    with the general ones (one launch per pass): cycles within one in ten, solutions to the tolerance."""
+    sols, cycles = [], []
+    for fuse in ("1", "0"):
+        monkeypatch.setenv("I3G_FUSE", fuse)
+        monkeypatch.setenv("I3G_TRACE", "1")
+        p, mode = _random_box(shape, multinum, seed=11)
+        z, x, y = np.meshgrid(*(np.linspace(0, 1, n) for n in (shape[2], shape[0], shape[1])), indexing="ij")
+        eta = (1e21 * np.exp(1.5 * np.sin(5 * x + 2 * y) * np.cos(4 * z - y))).astype(np.float32).reshape(-1)
+        for f in ("nu", "nxx", "nxy", "nxz", "nyz"):
+            p.nodes[f] = eta.copy()
+        par = abi.make_params(mode, stokes_rtol=1e-10, stokes_maxcyc=3000, precision=1, krylov=8)
+        capfd.readouterr()
+        g = lib.Context(abi.ModelBuffers(p), par, abi.make_file_params(mode.files[0]))
+        seen = [int(s.split(": ")[2].split()[0]) for s in capfd.readouterr().err.splitlines() if "FP32 transfers" in s]
+        assert seen == (widths if fuse == "1" else [0] * multinum)
+        monkeypatch.delenv("I3G_TRACE")
+        g.stokes(0, 1e30)
+        cycles.append(g.stats()["stokes_cycles"])
+        sols.append(g.get(abi.A_SOL, 0, 4 * p.nodenum).reshape(-1, 4))
+        g.close()
+    assert abs(cycles[1] - cycles[0]) <= 1 + cycles[0] // 10, cycles
+    for k in (1, 2, 3):
+        assert np.linalg.norm(sols[1][:, k] - sols[0][:, k]) <= 1e-6 * np.linalg.norm(sols[0][:, k])
