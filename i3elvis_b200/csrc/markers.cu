@@ -1468,13 +1468,13 @@ struct NodeOut {
 };
 
 // node sums over the tile boxes holding the node (fixed tile order), then the normalisation of
-// mark3mg.c:938-1002
+// mark3mg.c:938-1002; nothing when the sums are to be repeated (ERR_REDO)
 __global__ void k_r2n_gather(const double *stage, TileGeo TG, int nx, int ny, int nz, NodeOut O, int vm, double nubeg,
-                             double nuend)
+                             double nuend, const int *err)
 {
     const long n = (long)blockIdx.x * blockDim.x + threadIdx.x;
     const long N = (long)nx * ny * nz;
-    if (n >= N) return;
+    if (n >= N || (*err & ERR_REDO)) return;
     const int y = (int)(n % ny), x = (int)((n / ny) % nx), z = (int)(n / ((long)nx * ny));
     int x0, x1, y0, y1, z0, z1;
     box_range(x, TX, TG.ntx, x0, x1);
@@ -1519,10 +1519,11 @@ __global__ void k_r2n_gather(const double *stage, TileGeo TG, int nx, int ny, in
 }
 
 // tkrecalc (heat3mg.c:849-899): T = c + k * T_before(partner)
-__global__ void k_tk_bc(float *tk, const float *tk1, int n, const int *node, const int *p, const double *c, const double *k)
+__global__ void k_tk_bc(float *tk, const float *tk1, int n, const int *node, const int *p, const double *c, const double *k,
+                        const int *err)
 {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n) return;
+    if (t >= n || (*err & ERR_REDO)) return;
     // the reference's bondv1 and tk arrays are FP32: tk = c; tk += k * tk1 in FP32
     float v = (float)c[t];
     if (p[t] >= 0) v = __fadd_rn(v, __fmul_rn((float)k[t], tk1[p[t]]));
@@ -2073,19 +2074,17 @@ int markers_to_nodes(i3g_ctx *c, double timestep)
     NodeOut O{c->lev[0].nu, c->nxx, c->nxy, c->nxz, c->nyz, c->ro, c->cp, c->kt, c->ht, c->et, c->tk, c->rr, S->tk1};
     auto average = [&]() {
         LAUNCH(k_r2n_gather, nb(N), 256, 0, (const double *)S->stage, T, (int)c->m.xnumx, (int)c->m.ynumy, (int)c->m.znumz, O,
-               c->p.viscmod, c->p.nubeg, c->p.nuend);
+               c->p.viscmod, c->p.nubeg, c->p.nuend, (const int *)S->err);
         if (S->tbc_n)
             LAUNCH(k_tk_bc, nb(S->tbc_n), 256, 0, c->tk, (const float *)S->tk1, S->tbc_n, (const int *)S->tbc_node,
-                   (const int *)S->tbc_p, (const double *)S->tbc_c, (const double *)S->tbc_k);
+                   (const int *)S->tbc_p, (const double *)S->tbc_c, (const double *)S->tbc_k, (const int *)S->err);
     };
     average();
     I3G_CUDA(cudaGetLastError());
     I3G_CUDA(cudaEventRecord(e1, c->st));
     rc = check_err(c, "ronurecalc");
     if (*S->herr & ERR_REDO) {
-        // a marker that k_r2n_mma does not take: the pass again from the temperatures before the
-        // boundary rows (nodes without markers keep theirs)
-        I3G_CUDA(cudaMemcpyAsync(c->tk, S->tk1, sizeof(float) * N, cudaMemcpyDeviceToDevice, c->st));
+        // a marker that k_r2n_mma does not take: no node field has been written, the pass again
         I3G_CUDA(cudaMemsetAsync(S->err, 0, sizeof(int), c->st));
         launch_r2n(c, S->a, (const int *)S->coff, T, timestep, S->stage, true);
         average();

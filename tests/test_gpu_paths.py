@@ -148,6 +148,33 @@ def test_node_sums_with_markers_without_viscosity(exact):
     _nodes_match(mode, 1e10, edit, exact)
 
 
+@pytest.mark.parametrize("exact", [0, 1])
+@pytest.mark.parametrize("field,value", [("markrr", np.inf), ("markrr", -np.inf), ("markrr", np.nan), ("markv", np.inf)])
+def test_node_sums_with_a_marker_that_is_not_finite(field, value, exact):
+    """A property that is not finite reaches the nodes its marker weighs on and no other: 0 x inf is NaN in a
+    matrix product.  Markers in crowded, sparse and otherwise empty cells, beside nodes without markers, which
+    keep what they had."""
+    _, mode, _, base = _cloud()
+    x, y, z = (base.f32[f] for f in ("markx", "marky", "markz"))
+    cell = (z / 8334).astype(int) * 144 + (x / 8334).astype(int) * 12 + (y / 8334).astype(int)
+    count = np.bincount(cell, minlength=1728)[cell]
+    at = [int(np.flatnonzero(count == count.max())[0])] + [int(i) for i in np.flatnonzero(count <= 2)[:3]]
+    empty = (x > 6e4) & (y > 6e4)   # leave this corner to one marker
+    keep = int(np.flatnonzero(empty)[0])
+
+    def edit(buf):
+        for f in ("markx", "marky"):
+            a = buf.f32[f][empty]
+            buf.f32[f][empty] = a - 5e4
+        for f, v in (("markx", 8.1e4), ("marky", 8.3e4), ("markz", 5.2e4)):
+            buf.f32[f][keep] = v
+        buf.f32[field][at + [keep]] = value
+        for f in NODE_SUMS:
+            if f not in ("nu", "tk"):
+                buf.f32[f][:] = 7.0
+    _nodes_match(mode, 1e10, edit, exact)
+
+
 def test_partial_download_after_a_sort():
     """A download that names a few marker arrays returns those in the original order, and fields that
     the sort does not move stay with their markers."""
