@@ -1724,8 +1724,8 @@ int forward(i3g_unet *u)
     return 0;
 }
 
-// Gradients of the loss for the sample in act[X0] whose dL/dy is in grd[Y]; accumulated into u->grad.
-int backward(i3g_unet *u)
+// The layers of backward(), weight gradients of the wide ones on the second stream
+int backward_layers(i3g_unet *u)
 {
     for (int l = kLayers - 1; l >= 0; l--) {
         const LayerDef &ld = kL[l];
@@ -1762,9 +1762,20 @@ int backward(i3g_unet *u)
                                                                        kT[src].ch, f, c, 0.125f);
         }
     }
-    // the next pass overwrites the activations and gradients that the second stream reads
-    UCHK(cudaEventRecord(u->joined, u->st2));
-    UCHK(cudaStreamWaitEvent(u->st, u->joined, 0));
+    return 0;
+}
+
+// Gradients of the loss for the sample in act[X0] whose dL/dy is in grd[Y]; accumulated into u->grad.
+// The next pass overwrites the activations and gradients that the second stream reads, so the streams
+// are joined on every way out, also after an error half way.
+int backward(i3g_unet *u)
+{
+    const int rc = backward_layers(u);
+    cudaError_t e = cudaEventRecord(u->joined, u->st2);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(u->st, u->joined, 0);
+    if (e != cudaSuccess) cudaStreamSynchronize(u->st2);
+    if (rc) return rc;
+    UCHK(e);
     return 0;
 }
 

@@ -149,6 +149,36 @@ def test_network_output_and_gradients_match_oracle():
     assert abs(net.loss([0]) - loss) <= 1e-6 * loss
 
 
+def test_gradients_do_not_depend_on_the_pass_before():
+    """Weight gradients of the wide layers run on a second stream: a sample's gradients are the same after
+    another sample's pass as in a new network, up to the order in which atomic adds meet (partial sums of at
+    most a few hundred blocks in FP32: 1e-4 of a layer's norm is far above it), and the narrow layers', whose
+    sums have a fixed order, bit for bit."""
+    from i3elvis_b200.warmstart import UNet
+    dims = (17, 25, 33)
+    par = U.init_params(seed=4)
+    a, b = _sample(dims, 1), _sample(dims, 2)
+
+    def network():
+        net = UNet(dims[1], dims[2], dims[0], capacity=1, seed=3)
+        net.set_params(par)
+        net.set_scales(21.0, 0.5, 3300.0, 0.0125, 1e-10, 1e6)
+        return net
+    fresh = network().eval_host(a[0], a[1], grads=True)
+    net = network()
+    net.eval_host(b[0], b[1], grads=True)
+    net.eval_host(b[0])
+    again = net.eval_host(a[0], a[1], grads=True)
+    assert np.array_equal(fresh[0], again[0])
+    offs, _ = U.param_offsets()
+    for (w, _), (cin, cout) in zip(offs, U.layer_shapes()):
+        x, y = fresh[2][w:w + 27 * cin * cout], again[2][w:w + 27 * cin * cout]
+        assert np.linalg.norm(x) > 0
+        if max(cin, cout) <= 32:
+            assert np.array_equal(x, y), (cin, cout)
+        assert np.linalg.norm(x - y) <= 1e-4 * np.linalg.norm(x), (cin, cout)
+
+
 def test_training_lowers_loss_and_never_worsens_the_start():
     """A short training run on library solves of seeded 17^3 inclusion models lowers the loss;
     on held-out models the learned start (its correction scaled by the residual-minimising
