@@ -1791,6 +1791,19 @@ static void launch_heat_mark(i3g_ctx *c, const Marks &M, const int *coff, const 
     }
 }
 
+// Allows a kernel the dynamic shared memory this context launches it with.  The limit belongs to the
+// function, not to the context: it is raised to all that the function's static part leaves, never
+// set to one context's size, which would take it from a larger model alive beside it.
+template <typename... A>
+static int allow_smem(i3g_ctx *c, void (*kern)(A...), size_t need)
+{
+    if (need <= 48 * 1024) return 0;   // every function's default
+    cudaFuncAttributes at;
+    I3G_CUDA(cudaFuncGetAttributes(&at, kern));
+    I3G_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max(need, 227 * 1024 - at.sharedSizeBytes)));
+    return 0;
+}
+
 int markers_alloc(i3g_ctx *c)
 {
     MarkerState *S = new MarkerState();
@@ -1868,21 +1881,17 @@ int markers_alloc(i3g_ctx *c)
         I3G_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_heat_mark_anti<false>, 256, grid_smem(c)));
         S->key_blocks = (unsigned)std::max(1, sms * std::max(std::min(a, b), 1));
     }
-    I3G_CUDA(cudaFuncSetAttribute(k_r2n_cells<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)r2n_smem(c)));
-    I3G_CUDA(cudaFuncSetAttribute(k_r2n_cells<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)r2n_smem(c)));
-    I3G_CUDA(cudaFuncSetAttribute((k_r2n_mma<true, 16>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)r2n_mma_smem<true>(c, 16)));
-    I3G_CUDA(cudaFuncSetAttribute((k_r2n_mma<false, 16>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)r2n_mma_smem<false>(c, 16)));
-    if (r2n_mma_smem<false>(c, 24) <= 227 * 1024)
-        I3G_CUDA(cudaFuncSetAttribute((k_r2n_mma<false, 24>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)r2n_mma_smem<false>(c, 24)));
-    if (r2n_mma_smem<false>(c, 32) <= 227 * 1024)
-        I3G_CUDA(cudaFuncSetAttribute((k_r2n_mma<false, 32>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)r2n_mma_smem<false>(c, 32)));
-    I3G_CUDA(cudaFuncSetAttribute((k_heat_mark_cells<true, 1>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)heat_mark_smem(c)));
-    I3G_CUDA(cudaFuncSetAttribute((k_heat_mark_cells<true, 2>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)heat_mark_smem(c)));
-    I3G_CUDA(cudaFuncSetAttribute((k_heat_mark_cells<false, 1>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)heat_mark_smem(c)));
-    I3G_CUDA(cudaFuncSetAttribute((k_heat_mark_cells<false, 2>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)heat_mark_smem(c)));
+    const size_t g = grid_smem(c);
+    if ((rc = allow_smem(c, k_r2n_cells<true>, r2n_smem(c))) || (rc = allow_smem(c, k_r2n_cells<false>, r2n_smem(c))) ||
+        (rc = allow_smem(c, k_r2n_mma<true, 16>, r2n_mma_smem<true>(c, 16))) || (rc = allow_smem(c, k_r2n_mma<false, 16>, r2n_mma_smem<false>(c, 16))))
+        return rc;
+    if (r2n_mma_smem<false>(c, 24) <= 227 * 1024 && (rc = allow_smem(c, k_r2n_mma<false, 24>, r2n_mma_smem<false>(c, 24)))) return rc;
+    if (r2n_mma_smem<false>(c, 32) <= 227 * 1024 && (rc = allow_smem(c, k_r2n_mma<false, 32>, r2n_mma_smem<false>(c, 32)))) return rc;
+    for (auto f : {k_heat_mark_cells<true, 1>, k_heat_mark_cells<true, 2>, k_heat_mark_cells<false, 1>, k_heat_mark_cells<false, 2>})
+        if ((rc = allow_smem(c, f, heat_mark_smem(c)))) return rc;
     for (int m = 2; m <= 4; m++)
         for (MoveKernel f : {move_kernel_t<true, true>(m), move_kernel_t<true, false>(m), move_kernel_t<false, true>(m), move_kernel_t<false, false>(m)})
-            I3G_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)grid_smem(c)));
+            if ((rc = allow_smem(c, f, g))) return rc;
     {
         int dev = 0, sms = 0;
         I3G_CUDA(cudaGetDevice(&dev));
@@ -1890,8 +1899,8 @@ int markers_alloc(i3g_ctx *c)
         if (int rc = move_blocks(c, sms)) return rc;
     }
     for (auto f : {k_heat_mark_anti<true>, k_heat_mark_anti<false>})
-        I3G_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)grid_smem(c)));
-    I3G_CUDA(cudaFuncSetAttribute(k_tile_key, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)grid_smem(c)));
+        if ((rc = allow_smem(c, f, g))) return rc;
+    if ((rc = allow_smem(c, k_tile_key, g))) return rc;
     I3G_CUDA(cudaStreamSynchronize(c->st));
     // upload the host markers
     return markers_upload(c, &c->m);

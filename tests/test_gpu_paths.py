@@ -175,6 +175,31 @@ def test_node_sums_with_a_marker_that_is_not_finite(field, value, exact):
     _nodes_match(mode, 1e10, edit, exact)
 
 
+def test_two_contexts_of_different_sizes():
+    """A smaller model created while a larger one is alive leaves the larger one's marker and heat kernels the
+    shared memory they need: the results are those of the model alone."""
+    def run(other):
+        p, mode, fx, buf = marker_setup("dp17")
+        g = lib.Context(buf, abi.make_params(mode), abi.make_file_params(mode.files[0]))
+        if other:
+            p2, mode2, _, buf2 = marker_setup("sphere13")
+            h = lib.Context(buf2, abi.make_params(mode2), abi.make_file_params(mode2.files[0]))
+        dt = float(fx["fld_dt"][0])
+        g.heat(0, dt)
+        g.move_markers(dt)
+        g.markers_to_nodes(dt)
+        if other:
+            h.markers_to_nodes(0.0)
+            h.close()
+        g.markers_to_nodes(0.0)
+        g.download(abi.SYNC_ALL)
+        g.close()
+        return buf
+    alone, beside = run(False), run(True)
+    for f in NODE_SUMS + ("markx", "markk", "markv"):
+        assert np.array_equal(alone.f32[f], beside.f32[f]), f
+
+
 def test_partial_download_after_a_sort():
     """A download that names a few marker arrays returns those in the original order, and fields that
     the sort does not move stay with their markers."""
