@@ -33,8 +33,7 @@ struct HeatLevel {
     int nbc = 0;
     int *bnode = nullptr, *bpn = nullptr, *bdep = nullptr;
     double *bcc = nullptr, *bck = nullptr;     // flattened chain
-    int *bon = nullptr;                        // original partner (residual)
-    double *boc = nullptr, *bok = nullptr;
+    double *boc = nullptr;                     // original constant (right-hand side of the row)
 };
 
 struct HeatState {
@@ -400,8 +399,8 @@ int heat_alloc(i3g_ctx *c)
             }
         }
         std::vector<uint8_t> mask(L.n, 0);
-        std::vector<int> bn, bp, bdp, bon;
-        std::vector<double> bcc, bck, boc, bok;
+        std::vector<int> bn, bp, bdp;
+        std::vector<double> bcc, bck, boc;
         for (long q = 0; q < L.n; q++) {
             const int b = rid[mgp[l] + q];
             const int j = (int)(q % L.ny), i = (int)((q / L.ny) % L.nx), k = (int)(q / ((long)L.ny * L.nx));
@@ -412,10 +411,7 @@ int heat_alloc(i3g_ctx *c)
             }
             mask[q] = 1;
             bn.push_back((int)q);
-            const long p1 = c->m.bond_partner1[b];
-            bon.push_back(p1 > 0 ? (int)(p1 - 1 - mgp[l]) : -1);
             boc.push_back(c->m.bond_c[b]);
-            bok.push_back(c->m.bond_k[b]);
             double chc[kMaxBcDepth], chk[kMaxBcDepth];
             int dep = 0, pn = -1;
             long cur = mgp[l] + q;
@@ -439,8 +435,7 @@ int heat_alloc(i3g_ctx *c)
         H.nbc = (int)bn.size();
         int rc;
         if ((rc = up(c, H.bc, mask)) || (rc = up(c, H.bnode, bn)) || (rc = up(c, H.bpn, bp)) || (rc = up(c, H.bdep, bdp)) ||
-            (rc = up(c, H.bcc, bcc)) || (rc = up(c, H.bck, bck)) || (rc = up(c, H.bon, bon)) || (rc = up(c, H.boc, boc)) ||
-            (rc = up(c, H.bok, bok)))
+            (rc = up(c, H.bcc, bcc)) || (rc = up(c, H.bck, bck)) || (rc = up(c, H.boc, boc)))
             return rc;
     }
     I3G_CUDA(cudaMalloc((void **)&S->tk0, sizeof(float) * N0));
@@ -457,7 +452,7 @@ void heat_free(i3g_ctx *c)
     if (!S) return;
     for (int l = 0; l < c->nlev; l++) {
         HeatLevel &H = S->L[l];
-        void *p[] = {H.u, H.f, H.r, H.rocp, H.dx, H.dy, H.dz, H.cx[0], H.cx[1], H.cy[0], H.cy[1], H.cz[0], H.cz[1], H.bc, H.bnode, H.bpn, H.bdep, H.bcc, H.bck, H.bon, H.boc, H.bok};
+        void *p[] = {H.u, H.f, H.r, H.rocp, H.dx, H.dy, H.dz, H.cx[0], H.cx[1], H.cy[0], H.cy[1], H.cz[0], H.cz[1], H.bc, H.bnode, H.bpn, H.bdep, H.bcc, H.bck, H.boc};
         for (void *q : p) cudaFree(q);
         if (l > 0) cudaFree(H.kt);
     }

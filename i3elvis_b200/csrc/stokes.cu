@@ -3188,7 +3188,7 @@ struct KrylovState {
     double *V = nullptr;     // m+1 basis vectors, vector j component v at V + (4j + v) N
     double *Z = nullptr;     // m preconditioned directions, same layout
     double *W = nullptr;     // work vector (4N)
-    double *F0 = nullptr;    // zero right-hand side (4N)
+    double *F0 = nullptr;    // zero right-hand side (4N) of the unfused residual (I3G_FUSE=0)
     double *part = nullptr;  // partial dot products [blocks][kKryNq]
     double *mx = nullptr;    // block maxima of |v| over the velocity rows of the newest basis vector
     unsigned *done = nullptr;   // blocks of the running projection that have finished
@@ -3514,7 +3514,7 @@ static int kry_alloc(i3g_ctx *c, int m)
     ALLOC(K->V, double, (m + 1) * n4);
     ALLOC(K->Z, double, m * n4);
     ALLOC(K->W, double, n4);
-    ALLOC(K->F0, double, n4);
+    if (!c->fuse) ALLOC(K->F0, double, n4);
     ALLOC(K->part, double, (long)kKrBlocks * kKryNq);
     ALLOC(K->mx, double, kKrBlocks);
     ALLOC(K->done, unsigned, 1);
@@ -3523,7 +3523,7 @@ static int kry_alloc(i3g_ctx *c, int m)
     if (c->p.precision == 0) ALLOC(K->save, double, 2 * n4);
     I3G_CUDA(cudaMallocHost((void **)&K->hhost, (3 * kKryNq + 2) * sizeof(double)));
     I3G_CUDA(cudaMemsetAsync(K->W, 0, n4 * 8, c->st));
-    I3G_CUDA(cudaMemsetAsync(K->F0, 0, n4 * 8, c->st));
+    if (K->F0) I3G_CUDA(cudaMemsetAsync(K->F0, 0, n4 * 8, c->st));
     return 0;
 }
 
@@ -3588,7 +3588,6 @@ static int kry_enqueue_step(i3g_ctx *c, int j, int multinum)
     // w = D A z_j: the FP64 residual of z_j with a zero right-hand side is -A z_j
     View<double> Vz = view<double>(L0, L0.d);
     Vz.u0 = zj; Vz.u1 = zj + N; Vz.u2 = zj + 2 * N; Vz.u3 = zj + 3 * N;
-    Vz.f0 = K->F0; Vz.f1 = K->F0 + N; Vz.f2 = K->F0 + 2 * N; Vz.f3 = K->F0 + 3 * N;
     Vz.r0 = K->W; Vz.r1 = K->W + N; Vz.r2 = K->W + 2 * N; Vz.r3 = K->W + 3 * N;
     if (c->fuse) {
         BcDev4 B;
@@ -3596,6 +3595,7 @@ static int kry_enqueue_step(i3g_ctx *c, int j, int multinum)
         for (int v = 0; v < 4; v++) { B.b[v] = bcdev(L0.bcl[v]); nb += L0.bcl[v].n; }
         LAUNCH((k_residual_bc<double, true>), nblk(N) + nblk(nb), 256, Vz, B, nblk(N));
     } else {
+        Vz.f0 = K->F0; Vz.f1 = K->F0 + N; Vz.f2 = K->F0 + 2 * N; Vz.f3 = K->F0 + 3 * N;
         LAUNCH(k_residual<double>, nblk(N), 256, Vz);
         for (int v = 0; v < 4; v++) {
             BcList &B = L0.bcl[v];
