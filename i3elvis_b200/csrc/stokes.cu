@@ -3508,7 +3508,6 @@ static int kry_alloc(i3g_ctx *c, int m)
     if (K) kry_free(c);
     K = new KrylovState();
     c->kry = K;
-    K->m = m;
     K->N = c->lev[0].n;
     const long n4 = 4 * K->N;
     ALLOC(K->V, double, (m + 1) * n4);
@@ -3524,6 +3523,7 @@ static int kry_alloc(i3g_ctx *c, int m)
     I3G_CUDA(cudaMallocHost((void **)&K->hhost, (3 * kKryNq + 2) * sizeof(double)));
     I3G_CUDA(cudaMemsetAsync(K->W, 0, n4 * 8, c->st));
     if (K->F0) I3G_CUDA(cudaMemsetAsync(K->F0, 0, n4 * 8, c->st));
+    K->m = m;   // complete: a state left by an error above is freed and built again by the next solve
     return 0;
 }
 
