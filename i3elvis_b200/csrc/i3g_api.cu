@@ -155,6 +155,8 @@ int i3g_create(const i3g_model *m, const i3g_params *p, i3g_ctx **out)
 int i3g_set_file_params(i3g_ctx *c, const i3g_file_params *f)
 {
     if (!c || !f) return I3G_E_ARG;
+    // the captured iterations hold the FP32 cycle's scale, the mean of the viscosity limits, by value
+    if (f->nubeg != c->p.nubeg || f->nuend != c->p.nuend) i3g::stokes_params_changed(c);
     c->f = *f;
     c->p.nubeg = f->nubeg;
     c->p.nuend = f->nuend;

@@ -424,3 +424,23 @@ def test_fp32_transfers_are_compact_on_every_grid(shape, multinum, widths, capfd
     assert abs(cycles[1] - cycles[0]) <= 1 + cycles[0] // 10, cycles
     for k in (1, 2, 3):
         assert np.linalg.norm(sols[1][:, k] - sols[0][:, k]) <= 1e-6 * np.linalg.norm(sols[0][:, k])
+
+
+@pytest.mark.parametrize("krylov", [8, 0])
+def test_viscosity_limits_of_the_next_output_row(krylov):
+    """Another row of the output plan may set other viscosity limits, whose mean scales the FP32 cycle: a solve
+    after the change takes as many cycles as in a context that had these limits from the start."""
+    p, mode, _ = golden("sphere17")
+    par = abi.make_params(mode, stokes_rtol=1e-8, stokes_maxcyc=3000, precision=1, krylov=krylov, warm_start=0)
+    wide, narrow = abi.make_file_params(mode.files[0]), abi.make_file_params(mode.files[0])
+    wide.nubeg, wide.nuend = 1e12, 1e24
+    narrow.nubeg, narrow.nuend = 1e20, 1e24
+    cycles = []
+    for first in (narrow, wide):
+        g = lib.Context(abi.ModelBuffers(p), par, first)
+        g.stokes(0, 1e30)
+        g.set_file_params(narrow)
+        g.stokes(0, 1e30)
+        cycles.append(g.stats()["stokes_cycles"])
+        g.close()
+    assert abs(cycles[1] - cycles[0]) <= 1, cycles
