@@ -397,9 +397,11 @@ __device__ __forceinline__ void relax_vel_at(const View<T> &L, long t, int color
 // store.  The kernel before a run of relaxations (a restriction, prolongation or conversion) lets its
 // successor launch only after its own wait, and it writes no operator data, so whatever set the
 // operator up has completed by then.  On B200 a sweep went from 25 to 16 us on levels of 12^3 to 33^3
-// (22 with the packed boundary rows alone) and from 30 to 22 at 65^3; at 129^3 it takes 107 us plain and
-// 114 with the prologue (blocks of 128 threads, registers held over the wait).
-constexpr long kProNodes = 400000;
+// (22 with the packed boundary rows alone); plain against prologue (blocks of 128 threads, registers
+// held over the wait), FP32 level 0: 31.0 / 22.5 us at 65^3, 39.9 / 34.6 at 81^3, 52.5 / 48.4 at 97^3, 63.9 /
+// 61.8 at 105^3, 77.5 / 79.0 at 113^3, 112 / 120 at 129^3.  A FP64 V-cycle whose level 1 has 0.75, 0.97 and 1.23
+// million nodes takes 3.93 / 3.90, 4.95 / 4.94 and 6.14 / 6.19 ms.  The line lies where the two meet.
+constexpr long kProNodes = 1100000;
 
 template <typename T, int V, bool PRO>
 __global__ void __launch_bounds__(PRO ? 128 : 256, PRO ? 1 : sizeof(T) == 4 ? 6 : 4) k_relax_vel(View<T> L, int color, T koef)
@@ -2003,9 +2005,11 @@ static int upload_f32_scaled(i3g_ctx *c, float *&dst, const std::vector<double> 
 // read by another row of its partner's phase, or (partner of the first colour) by a row of the second
 // colour, which sees the old value when the boundary pass follows both colours.
 // Up to kSmTailNodes nodes: with 12^3 the tail takes 39 us of a FP32 V-cycle against 66 for the general
-// tail, and a 33^3 FP64 solve 146 instead of 192 ms (B200); its time grows with the nodes on its one
-// SM, a launched FP32 sweep takes 17 us at any small size.
-constexpr long kSmTailNodes = 2500;
+// tail, and a 33^3 FP64 solve 146 instead of 192 ms (B200).  Its time grows with the nodes on its one SM,
+// a launched FP32 sweep takes 17 us at any small size: a two-level FP32 V-cycle launched against on chip
+// takes 0.140 / 0.126 ms with 2366 and 0.139 / 0.126 with 2548 nodes on the coarse level, 0.140 / 0.133
+// with 2744, 0.139 / 0.138 with 3150, 0.139 / 0.143 with 3600.  In FP64 the shared memory ends at 2080 nodes.
+constexpr long kSmTailNodes = 3000;
 static int build_smtail(i3g_ctx *c, Level &L, const std::vector<uint8_t> &mask, const std::vector<int> (&node)[4],
                         const std::vector<int> (&pnode)[4], const std::vector<int> (&depth)[4], const std::vector<double> (&kk)[4])
 {

@@ -88,6 +88,25 @@ def test_vcycles_of_a_level_beyond_the_row_indexed_table(monkeypatch):
         assert np.array_equal(a, b)
 
 
+@pytest.mark.parametrize("pro", ["1100000", "0"])
+def test_vcycles_with_and_without_prologue_beyond_the_row_indexed_table(pro, monkeypatch):
+    """The level of 456,225 nodes again, its packed entries read before and after the wait for the
+    predecessor: the solution of one launch per boundary pass bit for bit."""
+    sols = []
+    for fuse in ("1", "0"):
+        monkeypatch.setenv("I3G_FUSE", fuse)
+        monkeypatch.setenv("I3G_PRO_NODES", pro)
+        p, mode = _random_box((149, 145, 153), 1, seed=8)
+        g = lib.Context(abi.ModelBuffers(p), abi.make_params(mode), abi.make_file_params(mode.files[0]))
+        g.call("i3g_stokes_setup")
+        g.call("i3g_stokes_vcycles", 1)
+        sols.append([g.get(abi.A_SOL, l, 4 * n) for l, n in enumerate(cases.level_sizes(p, 1))])
+        g.close()
+    for a, b in zip(*sols):
+        assert np.all(np.isfinite(a)) and np.any(a != 0)
+        assert np.array_equal(a, b)
+
+
 def _cloud(seed=5):
     """Reference fields of the 13^3 case with markers of every rock moved to uneven places: empty cells,
     cells of a few markers and cells of several hundred (more than a warp stages at once)."""
@@ -396,7 +415,7 @@ def test_fp32_cycles_of_every_tail_and_transfer(name, monkeypatch):
             assert np.linalg.norm(sols[q][:, k] - sols[0][:, k]) <= 1e-6 * np.linalg.norm(sols[0][:, k])
 
 
-@pytest.mark.parametrize("shape,multinum,widths", [((21, 21, 21), 2, [4, 4]), ((23, 23, 23), 2, [4, 4]), ((43, 21, 23), 3, [4, 4, 5]),
+@pytest.mark.parametrize("shape,multinum,widths", [((23, 23, 23), 1, [4]), ((21, 21, 21), 2, [4, 4]), ((23, 23, 23), 2, [4, 4]), ((43, 21, 23), 3, [4, 4, 5]),
                                                    ((27, 43, 35), 3, [4, 4, 5]), ((51, 51, 51), 3, [4, 4, 5])])
 def test_fp32_transfers_are_compact_on_every_grid(shape, multinum, widths, capfd, monkeypatch):
     """Coarse lines that gather from four or five fine ones, on grids whose FP32-rounded lines leave weights of
