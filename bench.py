@@ -468,10 +468,10 @@ def main():
     specs = [("stokes_sweep_" + ("f32" if prec else "f64"), 8 if prec else 10, sweeps0 * cyc,
               "one level-0 multicolour sweep, %s (k_relax_vel x6, k_relax_p, boundary rows)" % ("FP32" if prec else "FP64"),
               "68 B/node FP32" if prec else "116 B/node FP64"),
-             ("k_move", 5, 1.0, "RK4 marker advection", "45 B/marker + 13 nodal FP32 fields"),
+             ("k_move", 5, 1.0, "RK4 marker advection", "45 B/marker + 20 B/node (velocities, pressure)"),
              ("k_r2n_mma", 4, 1.0, "marker -> node sums", "25 B/marker + 48 B/node"),
              ("k_heat_mark_cells", 9, 1.0, "marker temperature update", "42 B/marker"),
-             ("heat_sweep", 6, 4.0 * heat_cyc, "one level-0 heat sweep (k_heat_relax x2)", "32 B/node")]
+             ("heat_sweep", 6, 4.0 * heat_cyc, "one level-0 heat sweep (k_heat_relax x2), at least 4 a cycle", "32 B/node")]
     kernels = []
     for name, kind, per_step, what, unit_bytes in specs:
         kms, kbytes = ctx.time_kernel(kind, 10)

@@ -2136,9 +2136,11 @@ int markers_heat_update(i3g_ctx *c, double timestep, const float *tk0, const flo
 }
 
 // Kernel timing with an empty L2 before every repetition (cold_time).  Bytes per launch are the
-// algorithmic bytes per unit: 4 marker -> node sums (k_r2n_cells): 25 B per marker (x, y, z,
-// type, T, viscosity, rr) + 48 B per node (12 FP32 outputs); 5 RK4 advection (k_move): 45 B per
-// marker + 13 nodal FP32 fields; 9 marker temperature update (k_heat_mark_cells): 42 B per marker.
+// algorithmic bytes per unit: 4 marker -> node sums (k_r2n_mma): 25 B per marker (x, y, z, type, T,
+// viscosity, rr) + 48 B per node (12 FP32 outputs); 5 RK4 advection (k_move): 45 B per marker (x, y, z, T,
+// viscosity, strain, type in; position, viscosity, strain out) + 20 B per node (FP32 velocities,
+// FP64 pressure), and 48 more where some rock reads the invariants (strain rates and stresses);
+// 9 marker temperature update (k_heat_mark_cells): 42 B per marker.
 int markers_time_kernel(i3g_ctx *c, int kind, int reps, double *ms_out, double *bytes)
 {
     MarkerState *S = ms(c);
@@ -2161,7 +2163,7 @@ int markers_time_kernel(i3g_ctx *c, int kind, int reps, double *ms_out, double *
     if (rc) return rc;
     if (kind == 4) *bytes = (double)n * 25.0 + (double)N * 48.0;
     else if (kind == 9) *bytes = (double)n * 42.0;
-    else *bytes = (double)n * 45.0 + (double)N * 13.0 * 4.0;
+    else *bytes = (double)n * 45.0 + (double)N * (S->any_use ? 68.0 : 20.0);
     I3G_CUDA(cudaGetLastError());
     return 0;
 }

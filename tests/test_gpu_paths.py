@@ -219,6 +219,17 @@ def test_two_contexts_of_different_sizes():
         assert np.array_equal(alone.f32[f], beside.f32[f]), f
 
 
+def test_bytes_of_a_marker_move_count_the_fields_it_reads():
+    """Strain rates and stresses (12 FP32 fields) count only where a rock of the model reads their invariants."""
+    per_node = {}
+    for name in ("sphere13", "dp17"):
+        p, mode, _, buf = marker_setup(name)
+        g = lib.Context(buf, abi.make_params(mode), abi.make_file_params(mode.files[0]))
+        per_node[name] = (g.time_kernel(5, 1)[1] - 45.0 * buf.f32["markx"].size) / p.nodenum
+        g.close()
+    assert per_node == {"sphere13": 20.0, "dp17": 68.0}
+
+
 def test_partial_download_after_a_sort():
     """A download that names a few marker arrays returns those in the original order, and fields that
     the sort does not move stay with their markers."""
