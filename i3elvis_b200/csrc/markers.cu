@@ -46,6 +46,12 @@ struct Marks {
     float *w, *d, *ex, *ft, *rn;
 };
 
+// Invariants that the rocks of a model read: none, some of them the strain rate alone, or both each.
+// The move is compiled for each: on 65^3 nodes with 7.1 M markers, all yielding, it takes 1.12 ms with a
+// branch for strain rates alone and 1.10 without, 0.83 and 0.80 where one rock of many yields (B200).  In
+// the reference's operation order it is the other way round (1.70 and 1.76 ms), which keeps the branch.
+enum { kUseNone, kUseSome, kUseBoth };
+
 struct MarkerState {
     long n = 0;
     Marks a{}, b{};                 // current arrays and the sort target
@@ -59,7 +65,7 @@ struct MarkerState {
     double *stage = nullptr;        // [ntiles][NACC][NBOX] per-tile node-box sums (no atomics)
     float *tk1 = nullptr;           // copy of T before boundary rows
     double *rock = nullptr;         // [24 * rocknum]
-    uint8_t *use = nullptr;         // [128] invariants the rheology of each rock type reads
+    unsigned long long use[2] = {~0ull, ~0ull};   // bit t: the rheology of rock type t reads strain rates, stresses
     int *err = nullptr, *herr = nullptr;
     int tbc_n = 0;                  // temperature boundary rows (level 0)
     int *tbc_node = nullptr, *tbc_p = nullptr;
@@ -68,9 +74,9 @@ struct MarkerState {
     // register caps of the FP64-latency-bound marker kernels (resident CTAs per SM they allow)
     // k_move without and with invariants: 2 (128 registers), 3 or 4 (I3G_MOVE_OCC).  Without them, 129^3
     // with 56.6 M markers on B200: 5.86 ms with 2, 5.29 with 3 (28 bytes spilled), 6.47 with 4; with them
-    // the third CTA spills and gains nothing
-    int move_minb[2] = {3, 2};
-    bool any_use = true;            // some rock of the model reads an invariant
+    // the third CTA spills and gains nothing (index: kUse*)
+    int move_minb[3] = {3, 2, 2};
+    int any_use = kUseSome;         // which invariants the model's rocks read
     // k_heat_mark_cells: 2 CTAs per SM (64 registers; 4.5 ms instead of 6.6 ms at 129^3 with 56.6 M
     // markers on B200, its FP64 dependency chains need the extra warps), 1 with I3G_HEAT_OCC=1
     int heat_minb = 2;
@@ -350,15 +356,58 @@ __device__ __forceinline__ void eps_stencil(const Grid &G, double x, double y, d
     E.qx = clamped(S.mx); E.qy = clamped(S.my); E.qz = clamped(S.mz);
 }
 
-// the six components of a strain-rate or stress field at the point
-template <bool EX>
-__device__ __forceinline__ void eps_fields(const float *const *f, int NY, int NXY, const EStencil &E, double *e)
+// second invariant (mark3mg.c:73-74 computes it as pow(., 0.5)): the correctly rounded square
+// root of the same sum, which a pow of exponent 0.5 approximates to within its own error bound
+__device__ __forceinline__ double inv2(const double *e)
 {
+    return sqrt(0.5 * (e[0] * e[0] + e[1] * e[1] + e[2] * e[2]) + e[3] * e[3] + e[4] * e[4] + e[5] * e[5]);
+}
+
+// component c (xx, yy, zz, xy, xz, yz) of a strain-rate or stress field at the point
+template <bool EX>
+__device__ __forceinline__ double eps_field(const float *const *f, int c, int NY, int NXY, const EStencil &E)
+{
+    if (c == 3) return tri<EX>(f[3], NY, NXY, E.ix, E.iy, E.qz);
+    if (c == 4) return tri<EX>(f[4], NY, NXY, E.ix, E.qy, E.iz);
+    if (c == 5) return tri<EX>(f[5], NY, NXY, E.qx, E.iy, E.iz);
+    return tri<EX>(f[c], NY, NXY, E.cx, E.cy, E.cz);
+}
+
+// Second invariants of strain rate and stress and the pressure at the point, in one run of independent
+// sums: with strain and stress each in a branch of its own a move on 65^3 nodes whose rocks yield
+// took 1.14 ms (B200, 7.1 M markers; 1.81 in the reference's operation order) instead of 1.10 (1.70).
+// The order matters through the registers: with the reference's operations the shear pairs come first.
+template <bool EX>
+__device__ __forceinline__ void eps_invariants(const NodeF &F, const EStencil &E, double &eii, double &sii, double &pr)
+{
+    const int NY = (int)F.NY, NXY = (int)F.NXY;
+    double e[6], s[6];
+    if (EX) {
 #pragma unroll
-    for (int q = 0; q < 3; q++) e[q] = tri<EX>(f[q], NY, NXY, E.cx, E.cy, E.cz);
-    e[3] = tri<EX>(f[3], NY, NXY, E.ix, E.iy, E.qz);   // xy
-    e[4] = tri<EX>(f[4], NY, NXY, E.ix, E.qy, E.iz);   // xz
-    e[5] = tri<EX>(f[5], NY, NXY, E.qx, E.iy, E.iz);   // yz
+        for (int q = 0; q < 6; q++) {
+            const int c = (q + 3) % 6;
+            e[c] = eps_field<EX>(F.e, c, NY, NXY, E);
+            s[c] = eps_field<EX>(F.s, c, NY, NXY, E);
+        }
+    } else {
+#pragma unroll
+        for (int c = 0; c < 6; c++) e[c] = eps_field<EX>(F.e, c, NY, NXY, E);
+#pragma unroll
+        for (int c = 0; c < 6; c++) s[c] = eps_field<EX>(F.s, c, NY, NXY, E);
+    }
+    pr = tri64<EX>(F.pr, NY, NXY, E.cx, E.cy, E.cz);
+    eii = inv2(e);
+    sii = inv2(s);
+}
+
+// the strain rate's alone
+template <bool EX>
+__device__ __forceinline__ double eps_invariant(const NodeF &F, const EStencil &E)
+{
+    double e[6];
+#pragma unroll
+    for (int c = 0; c < 6; c++) e[c] = eps_field<EX>(F.e, c, (int)F.NY, (int)F.NXY, E);
+    return inv2(e);
 }
 
 // epscalc1 with the cell given (mark3mg.c:2535-2838)
@@ -489,7 +538,7 @@ struct Phys {
     int rocknum, densimod, viscmod, outgrid, markmod;
     double nubeg, nuend, nukoef, healrate, timesum;
     double zdeep, vdeep, tdeep, nudeep, teclmin, teclmax, eroslev, sedilev, waterlev;
-    const uint8_t *use;   // [128] per rock type: invariants its rheology reads (rheo_use)
+    unsigned long long use_strain, use_stress;   // bit t: invariants the rheology of rock type t reads (rheo_use)
     int *err;
 };
 
@@ -626,18 +675,11 @@ __device__ __forceinline__ void load_grid(const Grid &Gg, double *sh, Grid &G)
     }
 }
 
-// second invariant (mark3mg.c:73-74 computes it as pow(., 0.5)): the correctly rounded square
-// root of the same sum, which a pow of exponent 0.5 approximates to within its own error bound
-__device__ __forceinline__ double inv2(const double *e)
-{
-    return sqrt(0.5 * (e[0] * e[0] + e[1] * e[1] + e[2] * e[2]) + e[3] * e[3] + e[4] * e[4] + e[5] * e[5]);
-}
-
 // ------------------------------------------------------------------------------------
 // movemark: rheology update + RK4 (mark3mg.c:49-310)
 // ------------------------------------------------------------------------------------
-// one marker of movemark (mark3mg.c:49-310); USE = false: no rock of the model reads an invariant
-template <bool EX, bool USE>
+// one marker of movemark (mark3mg.c:49-310); USE: which invariants the model's rocks read
+template <bool EX, int USE>
 __device__ __forceinline__ void move_one(const Marks &M, long i, const Grid &G, const NodeF &F, const Phys &P, double timestep)
 {
     int t = M.t[i];
@@ -657,21 +699,19 @@ __device__ __forceinline__ void move_one(const Marks &M, long i, const Grid &G, 
         // The strain-rate and stress invariants are interpolated only for rocks whose rheology reads
         // them (rheo_use): 12 of the 13 nodal sums, both square roots and the power law of the
         // stress ratio drop out for a Newtonian or diffusion-creep rock without a yield strength.
-        const int use = USE ? P.use[t & 127] : 0;
+        const bool use = USE != kUseNone && (P.use_strain >> (t & 63) & 1);
+        const bool stress = USE == kUseBoth ? use : USE == kUseSome && (P.use_stress >> (t & 63) & 1);
         EStencil E;
-        eps_stencil<EX>(G, fx, fy, fz, wn, S0, use != 0, E);
-        const double mpb = tri64<EX>(F.pr, (int)F.NY, (int)F.NXY, E.cx, E.cy, E.cz) * 1e-5;
-        double eii = 0, sii = 0, q[6];
-        if (use) {
-            eps_fields<EX>(F.e, (int)F.NY, (int)F.NXY, E, q);
-            eii = inv2(q);
+        eps_stencil<EX>(G, fx, fy, fz, wn, S0, use, E);
+        double eii = 0, sii = 0, pr;
+        if (stress) eps_invariants<EX>(F, E, eii, sii, pr);
+        else {
+            pr = tri64<EX>(F.pr, (int)F.NY, (int)F.NXY, E.cx, E.cy, E.cz);
+            if (USE == kUseSome && use) eii = eps_invariant<EX>(F, E);
         }
-        if (use & kUseStress) {
-            eps_fields<EX>(F.s, (int)F.NY, (int)F.NXY, E, q);
-            sii = inv2(q);
-        }
+        const double mpb = pr * 1e-5;
         double rii = 1.0;
-        if ((use & kUseStress) && mv > 0 && fx > G.gx[3] && fx < G.gx[G.nx - 4] && fy > G.gy[3] && fy < G.gy[G.ny - 4] && fz > G.gz[3] && fz < G.gz[G.nz - 4])
+        if (stress && mv > 0 && fx > G.gx[3] && fx < G.gx[G.nx - 4] && fy > G.gy[3] && fy < G.gy[G.ny - 4] && fz > G.gz[3] && fz < G.gz[G.nz - 4])
             // the power law of the stress ratio; the fast arithmetic takes it as exp(0.87 log r)
             // (relative difference ~1e-15, far below the FP32 viscosity it feeds)
             rii *= EX ? pow(0.5 * sii / eii / mv, 0.87) : exp(0.87 * log(0.5 * sii / eii / mv));
@@ -722,7 +762,7 @@ __device__ __forceinline__ void move_one(const Marks &M, long i, const Grid &G, 
 // Persistent grid-stride launch (a few CTAs per SM): the grid lines are staged in shared memory
 // once per CTA instead of once per 256 markers.  Markers are in (tile, cell) order from the last
 // sort, so a warp's interpolation corners hit the same L1 lines.
-template <bool EX, int MINB, bool USE>
+template <bool EX, int MINB, int USE>
 __global__ void __launch_bounds__(256, MINB) k_move(Marks M, long n, Grid Gg, NodeF F, Phys P, double timestep)
 {
     extern __shared__ double shg[];
@@ -1696,7 +1736,7 @@ static Phys phys_of(i3g_ctx *c)
     P.zdeep = c->p.zdeep; P.vdeep = c->p.vdeep; P.tdeep = c->p.tdeep; P.nudeep = c->p.nudeep;
     P.teclmin = c->p.teclmin; P.teclmax = c->p.teclmax;
     P.eroslev = c->p.eroslev; P.sedilev = c->p.sedilev; P.waterlev = c->p.waterlev;
-    P.use = S->use;
+    P.use_strain = S->use[0]; P.use_stress = S->use[1];
     P.err = S->err;
     return P;
 }
@@ -1709,7 +1749,7 @@ static bool mexact(i3g_ctx *c) { return c->p.marker_exact != 0; }
 
 // k_move with the model's arithmetic, register cap and need of invariants
 using MoveKernel = void (*)(Marks, long, Grid, NodeF, Phys, double);
-template <bool EX, bool USE>
+template <bool EX, int USE>
 static MoveKernel move_kernel_t(int minb)
 {
     return minb == 4 ? k_move<EX, 4, USE> : minb == 3 ? k_move<EX, 3, USE> : k_move<EX, 2, USE>;
@@ -1718,8 +1758,9 @@ static MoveKernel move_kernel(i3g_ctx *c)
 {
     const MarkerState *S = ms(c);
     const int m = S->move_minb[S->any_use];
-    if (mexact(c)) return S->any_use ? move_kernel_t<true, true>(m) : move_kernel_t<true, false>(m);
-    return S->any_use ? move_kernel_t<false, true>(m) : move_kernel_t<false, false>(m);
+    if (mexact(c))
+        return S->any_use == kUseNone ? move_kernel_t<true, kUseNone>(m) : move_kernel_t<true, kUseSome>(m);
+    return S->any_use == kUseNone ? move_kernel_t<false, kUseNone>(m) : S->any_use == kUseBoth ? move_kernel_t<false, kUseBoth>(m) : move_kernel_t<false, kUseSome>(m);
 }
 
 // resident k_move CTAs on all SMs (the same for both arithmetic variants: both are capped at the same
@@ -1837,14 +1878,14 @@ int markers_alloc(i3g_ctx *c)
         for (int t = 0; t < rn; t++) rk[(size_t)f * rn + t] = c->m.rock[f] ? c->m.rock[f][t] : 0.0;
     I3G_CUDA(cudaMalloc((void **)&S->rock, sizeof(double) * rk.size()));
     I3G_CUDA(cudaMemcpyAsync(S->rock, rk.data(), sizeof(double) * rk.size(), cudaMemcpyHostToDevice, c->st));
-    std::vector<uint8_t> use(128, kUseStrain | kUseStress);
-    S->any_use = false;
-    for (int t = 0; t < std::min(rn, 128); t++) {
-        use[t] = rheo_use(c->m.rock, t);
-        S->any_use = S->any_use || use[t];
+    S->any_use = kUseNone;
+    for (int t = 0; t < std::min(rn, 64); t++) {   // types from 50 on are refused by the kernels
+        const int use = rheo_use(c->m.rock, t);
+        if (!(use & kUseStrain)) S->use[0] &= ~(1ull << t);
+        if (!(use & kUseStress)) S->use[1] &= ~(1ull << t);
+        if (use == kUseStrain) S->any_use = kUseSome;
+        else if (use && S->any_use == kUseNone) S->any_use = kUseBoth;
     }
-    I3G_CUDA(cudaMalloc((void **)&S->use, use.size()));
-    I3G_CUDA(cudaMemcpyAsync(S->use, use.data(), use.size(), cudaMemcpyHostToDevice, c->st));
     I3G_CUDA(cudaMalloc((void **)&S->err, sizeof(int)));
     I3G_CUDA(cudaMallocHost((void **)&S->herr, sizeof(int)));
     // temperature boundary rows of level 0 (bondm[8*nodenum + node], heat3mg.c:859-889)
@@ -1874,7 +1915,7 @@ int markers_alloc(i3g_ctx *c)
         int dev = 0, sms = 0;
         I3G_CUDA(cudaGetDevice(&dev));
         I3G_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        if (const char *e = getenv("I3G_MOVE_OCC")) S->move_minb[0] = S->move_minb[1] = std::min(4, std::max(2, atoi(e)));
+        if (const char *e = getenv("I3G_MOVE_OCC")) S->move_minb[0] = S->move_minb[1] = S->move_minb[2] = std::min(4, std::max(2, atoi(e)));
         if (const char *e = getenv("I3G_HEAT_OCC")) S->heat_minb = std::min(2, std::max(1, atoi(e)));
         int a = 0, b = 0;
         I3G_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_tile_key, 256, grid_smem(c)));
@@ -1890,7 +1931,8 @@ int markers_alloc(i3g_ctx *c)
     for (auto f : {k_heat_mark_cells<true, 1>, k_heat_mark_cells<true, 2>, k_heat_mark_cells<false, 1>, k_heat_mark_cells<false, 2>})
         if ((rc = allow_smem(c, f, heat_mark_smem(c)))) return rc;
     for (int m = 2; m <= 4; m++)
-        for (MoveKernel f : {move_kernel_t<true, true>(m), move_kernel_t<true, false>(m), move_kernel_t<false, true>(m), move_kernel_t<false, false>(m)})
+        for (MoveKernel f : {move_kernel_t<true, kUseNone>(m), move_kernel_t<true, kUseSome>(m),
+                             move_kernel_t<false, kUseNone>(m), move_kernel_t<false, kUseSome>(m), move_kernel_t<false, kUseBoth>(m)})
             if ((rc = allow_smem(c, f, g))) return rc;
     {
         int dev = 0, sms = 0;
@@ -1915,7 +1957,7 @@ void markers_free(i3g_ctx *c)
     free_marks(S->b);
     for (float *p : {S->a.w, S->a.d, S->a.ex, S->a.ft, S->a.rn}) cudaFree(p);
     cudaFree(S->key); cudaFree(S->cnt); cudaFree(S->coff); cudaFree(S->off); cudaFree(S->cur); cudaFree(S->bsum); cudaFree(S->acc); cudaFree(S->stage); cudaFree(S->tk1);
-    cudaFree(S->rock); cudaFree(S->use); cudaFree(S->err);
+    cudaFree(S->rock); cudaFree(S->err);
     if (S->herr) cudaFreeHost(S->herr);
     if (S->up_ev) cudaEventDestroy(S->up_ev);
     cudaFree(S->tbc_node); cudaFree(S->tbc_p); cudaFree(S->tbc_c); cudaFree(S->tbc_k);

@@ -295,6 +295,50 @@ def test_marker_rheology_reads_what_it_needs(exact):
     np.testing.assert_allclose(a.f32["markv"], b.f32["markv"], rtol=2e-7)
 
 
+@pytest.mark.parametrize("exact", [0, 1])
+@pytest.mark.parametrize("which", ["all yield", "one yields", "power law alone", "none"])
+def test_marker_rheology_for_every_kind_of_rock_table(which, exact):
+    """Tables whose rocks all yield, one of them, none but with power-law creep, and none that reads an
+    invariant: each has its own kernel.  Positions as the oracle's to the bit, strains within their FP32
+    rounding, viscosities through pow and exp."""
+    bufs = []
+    for side in range(2):
+        p, mode, fx, buf = marker_setup("sphere13")
+        rock = dict(zip(ROCK_FIELDS, buf.rocks))
+        rock["n0"][:], rock["n1"][:] = 1e5, 1e35
+        rng = np.random.default_rng(6)
+        n = buf.f32["markx"].size
+        buf.markt[:] = rng.integers(2, 4, n)
+        for t in (2, 3):
+            for f, v in dict(nu=1e21, dh=0.0, dv=0.0, ss=0.0, mm=1.0, a0=0.0, a1=0.0, b0=0.0, b1=0.0).items():
+                rock[f][t] = v
+            if which == "all yield" or (which == "one yields" and t == 3):
+                rock["a0"][t] = rock["a1"][t] = 1e6
+                rock["b0"][t] = rock["b1"][t] = 0.1
+            if which == "power law alone" and t == 3:
+                rock["nu"][t], rock["ss"][t], rock["mm"][t] = 1e9, 1e4, 3.0
+        buf.f32["marke"][:] = rng.uniform(-1, 1, n)
+        buf.f32["markv"][:] = 1e20
+        par, fp = abi.make_params(mode, marker_exact=exact), abi.make_file_params(mode.files[0])
+        fp.nubeg, fp.nuend = 1e5, 1e35
+        dt = float(fx["fld_dt"][0])
+        c = lib.Context(buf, par, fp) if side == 0 else O.Oracle(buf, par, fp)
+        if side == 0:
+            c.move_markers(dt)
+        else:
+            c.call("orc_move_markers", dt)
+        c.download(abi.SYNC_ALL)
+        c.close()
+        bufs.append(buf)
+    a, b = bufs
+    for f in ("markx", "marky", "markz"):
+        assert np.array_equal(a.f32[f], b.f32[f]), f
+    if "yield" in which:
+        assert int((b.f32["marke"] > 0).sum()) > 0
+    np.testing.assert_allclose(a.f32["marke"], b.f32["marke"], rtol=2e-7, atol=0)
+    np.testing.assert_allclose(a.f32["markv"], b.f32["markv"], rtol=2e-7)
+
+
 @pytest.mark.parametrize("factor", [None, 0.5])
 @pytest.mark.parametrize("scale", [1e-2, 1.0, 30.0])
 def test_heat_from_uncoupled_to_stiff(scale, factor):
