@@ -24,7 +24,7 @@ struct HeatLevel {
     double *u = nullptr, *f = nullptr, *r = nullptr;
     float *kt = nullptr;            // level 0 points at the context's kt
     double *rocp = nullptr;
-    double *dx = nullptr, *dy = nullptr, *dz = nullptr;   // raw spacings g[i]-g[i-1] (i >= 1)
+    double *dx = nullptr, *dy = nullptr, *dz = nullptr;   // level 0: raw spacings g[i]-g[i-1] (i >= 1)
     // face factors of a row, 1 / (distance to the neighbour * distance between its two neighbours):
     // [0] towards i - 1, [1] towards i + 1 (twice the face's half sum of conductivities times the
     // reference's 2 / (g[i+1] - g[i-1]) over the spacing)
@@ -389,7 +389,7 @@ int heat_alloc(i3g_ctx *c)
         for (int d = 0; d < 3; d++) {
             std::vector<double> h(nn[d] + 1, 0.0);
             for (int i = 1; i < nn[d]; i++) h[i] = g[d][i] - g[d][i - 1];
-            int rc = up(c, *dd[d], h);
+            int rc = l == 0 ? up(c, *dd[d], h) : 0;
             if (rc) return rc;
             double **cc[3] = {H.cx, H.cy, H.cz};
             for (int q = 0; q < 2; q++) {

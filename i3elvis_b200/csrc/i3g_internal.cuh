@@ -9,6 +9,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <utility>
+#include <vector>
 #include <cuda_runtime.h>
 #include "../../include/i3g.h"
 
@@ -135,6 +136,7 @@ struct Level {
                                        // bit 4 + v: partner of in-kernel boundary rows of v (BcList::na)
     Fields<double> d;
     Fields<float> s;                    // scaled FP32 copy for the mixed-precision solver
+    std::vector<void *> tables;         // device memory of the tables below and above (stokes.cu, TablePack)
     SmTailRows sm;
     int compact = 0;                    // FP32 transfers from and to the finer level in compact form: fine
                                         // indices per axis, 4 or 5 (0: general transfers)

@@ -1862,6 +1862,43 @@ static int upload(i3g_ctx *c, T *&dst, const std::vector<T> &src)
     return 0;
 }
 
+// The tables of one level, copied to the device in one piece: a level has about a hundred of a few
+// hundred bytes, and an allocation, a copy and a wait for each were most of creating a small model.
+// A table of kPackBytes or more gets its own.  The memory belongs to the level (Level::tables).
+constexpr size_t kPackBytes = 65536;
+struct TablePack {
+    i3g_ctx *c;
+    Level &L;
+    std::vector<unsigned char> h;
+    std::vector<std::pair<void **, size_t>> at;   // pointers to set, offsets
+
+    template <typename T>
+    int add(T *&dst, const std::vector<T> &src)
+    {
+        const size_t bytes = sizeof(T) * src.size();
+        if (bytes >= kPackBytes) {
+            if (const int rc = upload(c, dst, src)) return rc;
+            L.tables.push_back((void *)dst);
+            return 0;
+        }
+        const size_t o = (h.size() + 255) & ~(size_t)255;   // as aligned as an allocation
+        h.resize(o + std::max(bytes, sizeof(T)));
+        if (bytes) memcpy(h.data() + o, src.data(), bytes);
+        at.push_back({(void **)&dst, o});
+        return 0;
+    }
+    int flush()
+    {
+        unsigned char *base = nullptr;
+        if (const int rc = upload(c, base, h)) return rc;
+        L.tables.push_back(base);
+        for (auto &e : at) *e.first = base + e.second;
+        h.clear();
+        at.clear();
+        return 0;
+    }
+};
+
 static CtView ctview(const Transfer1D &t) { return CtView{t.cs, t.a, t.cw, t.cv}; }
 
 // one-dimensional transfer stencil (host, FP64, the reference's expressions)
@@ -1962,21 +1999,22 @@ static int compact_transfer(int nf, int nc, const std::vector<int> &ha, const st
     return width;
 }
 
-static int upload_transfer(i3g_ctx *c, const double *gf, int nf, const double *gc, int nc, int stag, Transfer1D &t)
+static int add_transfer(TablePack &P, const double *gf, int nf, const double *gc, int nc, int stag, Transfer1D &t)
 {
     std::vector<int> ha, gptr, gfv;
     std::vector<double> w0, w1, gwv;
     build_transfer(gf, nf, gc, nc, stag, t, ha, w0, w1, gptr, gfv, gwv);
     int rc;
-    std::vector<int> cs;
-    std::vector<float4> cw;
-    std::vector<float> cw5;
-    std::vector<float2> cv;
-    t.compact = compact_transfer(nf, nc, ha, w0, w1, cs, cw, cw5, cv);
-    if (t.compact && ((rc = upload(c, t.cs, cs)) || (rc = upload(c, t.cw, cw)) || (rc = upload(c, t.cw5, cw5)) || (rc = upload(c, t.cv, cv))))
-        return rc;
-    if ((rc = upload(c, t.a, ha)) || (rc = upload(c, t.w0, w0)) || (rc = upload(c, t.w1, w1)) ||
-        (rc = upload(c, t.gptr, gptr)) || (rc = upload(c, t.gf, gfv)) || (rc = upload(c, t.gw, gwv)))
+    if (stag != kStagAbs) {   // the viscosity restriction has no FP32 form
+        std::vector<int> cs;
+        std::vector<float4> cw;
+        std::vector<float> cw5;
+        std::vector<float2> cv;
+        t.compact = compact_transfer(nf, nc, ha, w0, w1, cs, cw, cw5, cv);
+        if (t.compact && ((rc = P.add(t.cs, cs)) || (rc = P.add(t.cw, cw)) || (rc = P.add(t.cw5, cw5)) || (rc = P.add(t.cv, cv)))) return rc;
+    }
+    if ((rc = P.add(t.a, ha)) || (rc = P.add(t.w0, w0)) || (rc = P.add(t.w1, w1)) || (rc = P.add(t.gptr, gptr)) ||
+        (rc = P.add(t.gf, gfv)) || (rc = P.add(t.gw, gwv)))
         return rc;
     return 0;
 }
@@ -1993,11 +2031,11 @@ static void inv_tables(const double *g, int n, std::vector<double> &ic, std::vec
     for (int i = 1; i < n - 1; i++) is[i] = 1.0 / (g[i + 1] - g[i - 1]);
 }
 
-static int upload_f32_scaled(i3g_ctx *c, float *&dst, const std::vector<double> &src, double scale)
+static std::vector<float> scaled_f32(const std::vector<double> &src, double scale)
 {
     std::vector<float> f(src.size());
     for (size_t i = 0; i < src.size(); i++) f[i] = (float)(src[i] * scale);
-    return upload(c, dst, f);
+    return f;
 }
 
 // Boundary rows of one level for the on-chip tail: one list entry each, by partner.  The level
@@ -2010,7 +2048,7 @@ static int upload_f32_scaled(i3g_ctx *c, float *&dst, const std::vector<double> 
 // takes 0.140 / 0.126 ms with 2366 and 0.139 / 0.126 with 2548 nodes on the coarse level, 0.140 / 0.133
 // with 2744, 0.139 / 0.138 with 3150, 0.139 / 0.143 with 3600.  In FP64 the shared memory ends at 2080 nodes.
 constexpr long kSmTailNodes = 3000;
-static int build_smtail(i3g_ctx *c, Level &L, const std::vector<uint8_t> &mask, const std::vector<int> (&node)[4],
+static int build_smtail(TablePack &P, Level &L, const std::vector<uint8_t> &mask, const std::vector<int> (&node)[4],
                         const std::vector<int> (&pnode)[4], const std::vector<int> (&depth)[4], const std::vector<double> (&kk)[4])
 {
     SmTailRows &R = L.sm;
@@ -2052,7 +2090,7 @@ static int build_smtail(i3g_ctx *c, Level &L, const std::vector<uint8_t> &mask, 
     }
     R.nent = (int)hent.size();
     int rc;
-    if ((rc = upload(c, R.ent, hent)) || (rc = upload(c, R.cst, hcst)) || (rc = upload(c, R.first, first))) return rc;
+    if ((rc = P.add(R.ent, hent)) || (rc = P.add(R.cst, hcst)) || (rc = P.add(R.first, first))) return rc;
     R.ok = true;
     return 0;
 }
@@ -2065,7 +2103,7 @@ __global__ void k_bc_inline(int4 *inl, const int4 *w4, const int *writer, int na
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e < na && w4[e].w) inl[writer[e]] = w4[e];   // a writer's first entry holds its rows
 }
-static int pack_bc(i3g_ctx *c, const Level &L, BcList &B, int na, const std::vector<int> &node, const std::vector<int> &pnode,
+static int pack_bc(TablePack &P, BcList &B, int na, const std::vector<int> &node, const std::vector<int> &pnode,
                    const std::vector<int> &depth, const std::vector<double> &kk, const std::vector<int> &writer, const std::vector<int> &first)
 {
     const int n = (int)node.size();
@@ -2097,13 +2135,7 @@ static int pack_bc(i3g_ctx *c, const Level &L, BcList &B, int na, const std::vec
         ext.push_back(make_int4(node[e], pnode[e], bits, 0));
     }
     int rc;
-    if ((rc = upload(c, B.w4, w4)) || (rc = upload(c, B.ext, ext))) return rc;
-    if (L.n <= kBcInline && na > 0) {
-        ALLOC(B.inl, int4, L.n);
-        I3G_CUDA(cudaMemsetAsync(B.inl, 0, sizeof(int4) * L.n, c->st));
-        k_bc_inline<<<nblk(na), 256, 0, c->st>>>(B.inl, B.w4, B.writer, na);
-        c->launches++;
-    }
+    if ((rc = P.add(B.w4, w4)) || (rc = P.add(B.ext, ext))) return rc;
     B.packed = true;
     return 0;
 }
@@ -2260,8 +2292,9 @@ static int build_bc(i3g_ctx *c)
                 }
             }
         }
+        TablePack P{c, L};
         if (c->smtail && l > 0)
-            if (const int rc = build_smtail(c, L, mask, node, pnode, depth, kk)) return rc;
+            if (const int rc = build_smtail(P, L, mask, node, pnode, depth, kk)) return rc;
         if (getenv("I3G_TRACE"))
             for (int v = 0; v < 4; v++)
                 fprintf(stderr, "i3g: level %d component %d: %zu boundary rows, %s (%d by a row's thread)\n", l, v,
@@ -2272,13 +2305,21 @@ static int build_bc(i3g_ctx *c)
             BcList &B = L.bcl[v];
             B.n = (int)node[v].size();
             B.na = na[v];
-            if (na[v] > 0 && ((rc = upload(c, B.first, first[v])) || (rc = upload(c, B.writer, writer[v])))) return rc;
-            if ((rc = upload(c, B.node, node[v])) || (rc = upload(c, B.pnode, pnode[v])) ||
-                (rc = upload(c, B.depth, depth[v])) || (rc = upload(c, B.c, cc[v])) || (rc = upload(c, B.k, kk[v])) ||
-                (rc = upload(c, B.onode, onode[v])) || (rc = upload(c, B.ocomp, ocomp[v])) ||
-                (rc = upload(c, B.oc, oc[v])) || (rc = upload(c, B.ok, ok[v])))
+            if (na[v] > 0 && ((rc = P.add(B.first, first[v])) || (rc = P.add(B.writer, writer[v])))) return rc;
+            if ((rc = P.add(B.node, node[v])) || (rc = P.add(B.pnode, pnode[v])) || (rc = P.add(B.depth, depth[v])) ||
+                (rc = P.add(B.c, cc[v])) || (rc = P.add(B.k, kk[v])) || (rc = P.add(B.onode, onode[v])) ||
+                (rc = P.add(B.ocomp, ocomp[v])) || (rc = P.add(B.oc, oc[v])) || (rc = P.add(B.ok, ok[v])))
                 return rc;
-            if (na[v] >= 0 && (rc = pack_bc(c, L, B, na[v], node[v], pnode[v], depth[v], kk[v], writer[v], first[v]))) return rc;
+            if (na[v] >= 0 && (rc = pack_bc(P, B, na[v], node[v], pnode[v], depth[v], kk[v], writer[v], first[v]))) return rc;
+        }
+        if ((rc = P.flush())) return rc;
+        for (int v = 0; v < 4 && L.n <= kBcInline; v++) {
+            BcList &B = L.bcl[v];
+            if (!B.packed || B.na <= 0) continue;
+            ALLOC(B.inl, int4, L.n);
+            I3G_CUDA(cudaMemsetAsync(B.inl, 0, sizeof(int4) * L.n, c->st));
+            k_bc_inline<<<nblk(B.na), 256, 0, c->st>>>(B.inl, B.w4, B.writer, B.na);
+            c->launches++;
         }
     }
     return 0;
@@ -2370,24 +2411,26 @@ int stokes_alloc(i3g_ctx *c)
         const int nn[3] = {L.nx, L.ny, L.nz};
         double **di[3][2] = {{&L.d.ix[0], &L.d.ix[1]}, {&L.d.iy[0], &L.d.iy[1]}, {&L.d.iz[0], &L.d.iz[1]}};
         float **fi[3][2] = {{&L.s.ix[0], &L.s.ix[1]}, {&L.s.iy[0], &L.s.iy[1]}, {&L.s.iz[0], &L.s.iz[1]}};
+        TablePack P{c, L};
         for (int d = 0; d < 3; d++) {
             std::vector<double> ic, is;
             inv_tables(g[d], nn[d], ic, is);
             int rc;
-            if ((rc = upload(c, *di[d][0], ic)) || (rc = upload(c, *di[d][1], is)) ||
-                (rc = upload_f32_scaled(c, *fi[d][0], ic, c->h_ref)) || (rc = upload_f32_scaled(c, *fi[d][1], is, c->h_ref)))
+            if ((rc = P.add(*di[d][0], ic)) || (rc = P.add(*di[d][1], is)) || (rc = P.add(*fi[d][0], scaled_f32(ic, c->h_ref))) ||
+                (rc = P.add(*fi[d][1], scaled_f32(is, c->h_ref))))
                 return rc;
         }
+        if (const int rc = P.flush()) return rc;
     }
     for (int l = 0; l + 1 < c->nlev; l++) {
         Level &F = c->lev[l], &Cc = c->lev[l + 1];
         const double *gf[3] = {F.gx, F.gy, F.gz}, *gc[3] = {Cc.gx, Cc.gy, Cc.gz};
         const int nf[3] = {F.nx, F.ny, F.nz}, ncn[3] = {Cc.nx, Cc.ny, Cc.nz};
+        TablePack P{c, F};
         for (int d = 0; d < 3; d++)
-            for (int s = 0; s < 4; s++) {
-                int rc = upload_transfer(c, gf[d], nf[d], gc[d], ncn[d], s, F.tr[d][s]);
-                if (rc) return rc;
-            }
+            for (int s = 0; s < 4; s++)
+                if (const int rc = add_transfer(P, gf[d], nf[d], gc[d], ncn[d], s, F.tr[d][s])) return rc;
+        if (const int rc = P.flush()) return rc;
     }
     c->red_blocks = 2 * 148;
     ALLOC(c->dred, double, (long)c->red_blocks * kRedQ + 16);
@@ -2439,25 +2482,13 @@ void stokes_free(i3g_ctx *c)
         for (int v = 0; v < 4; v++) {
             cudaFree(L.d.u[v]); cudaFree(L.d.f[v]); cudaFree(L.d.r[v]);
             cudaFree(L.s.u[v]); cudaFree(L.s.f[v]); cudaFree(L.s.r[v]);
-            BcList &B = L.bcl[v];
-            cudaFree(B.node); cudaFree(B.pnode); cudaFree(B.depth); cudaFree(B.c); cudaFree(B.k);
-            cudaFree(B.onode); cudaFree(B.ocomp); cudaFree(B.oc); cudaFree(B.ok); cudaFree(B.first); cudaFree(B.writer);
-            cudaFree(B.inl); cudaFree(B.w4); cudaFree(B.ext);
+            cudaFree(L.bcl[v].inl);
         }
         cudaFree(L.d.etac); cudaFree(L.d.etaxy); cudaFree(L.d.etaxz); cudaFree(L.d.etayz); cudaFree(L.d.nd);
         cudaFree(L.s.etac); cudaFree(L.s.etaxy); cudaFree(L.s.etaxz); cudaFree(L.s.etayz); cudaFree(L.s.nd);
-        for (int a = 0; a < 2; a++) {
-            cudaFree(L.d.ix[a]); cudaFree(L.d.iy[a]); cudaFree(L.d.iz[a]);
-            cudaFree(L.s.ix[a]); cudaFree(L.s.iy[a]); cudaFree(L.s.iz[a]);
-        }
-        for (int d = 0; d < 3; d++)
-            for (int s = 0; s < 4; s++) {
-                Transfer1D &t = L.tr[d][s];
-                cudaFree(t.a); cudaFree(t.w0); cudaFree(t.w1); cudaFree(t.gptr); cudaFree(t.gf); cudaFree(t.gw);
-                cudaFree(t.cs); cudaFree(t.cw); cudaFree(t.cw5); cudaFree(t.cv);
-            }
         for (int v = 0; v < 4; v++) cudaFree(L.iws[v]);
-        cudaFree(L.sm.ent); cudaFree(L.sm.cst); cudaFree(L.sm.first);
+        for (void *t : L.tables) cudaFree(t);
+        L.tables.clear();
     }
     cudaFree(c->dred);
     if (c->hred) cudaFreeHost(c->hred);
