@@ -483,23 +483,28 @@ static void hsmooth(i3g_ctx *c, int l, int n, double dt, bool res)
 
 // Coupling of every level, from the largest k / (rho cp) kap of level 0's nodes and the step dt:
 // q = 2 dt kap (1/hx^2 + 1/hy^2 + 1/hz^2), h the level's smallest spacings.  A coarse level keeps level
-// 0's three outermost lines at each end; the cells between them stay narrow on every level and are
-// not counted there.  A row beside a much better conductor couples more strongly than its own k says,
-// and the damping of the coarse averages is not in it: an estimate, which heat_solve checks.  With dt =
-// 0.3 h^2 / kap (levels 0 and 1) four heat steps on 65^3 nodes with 7.1 M markers take 4.4 ms on B200,
-// with every level 6.2.
-static void heat_coupling(i3g_ctx *c, double kap, double dt, double *qs)
+// 0's three outermost lines at each end; the cells between them stay narrow on every level and count
+// in qall alone.  A row beside a much better conductor couples more strongly than its own k says, and
+// the damping of the coarse averages is not in it: an estimate, which heat_solve checks.  With dt = 0.3
+// h^2 / kap (levels 0 and 1) four heat steps on 65^3 nodes with 7.1 M markers take 4.4 ms on B200, with
+// every level 6.2.
+static void heat_coupling(i3g_ctx *c, double kap, double dt, double *q, double *qall)
 {
     for (int l = 0; l < c->nlev; l++) {
         const Level &L = c->lev[l];
         const double *g[3] = {L.gx, L.gy, L.gz};
         const int n[3] = {L.nx, L.ny, L.nz};
-        qs[l] = 0;
+        q[l] = qall[l] = 0;
         for (int d = 0; d < 3; d++) {
             const int e = l > 0 && n[d] > 5 ? 2 : 0;
-            double h = g[d][1 + e] - g[d][e];
-            for (int i = 2 + e; i < n[d] - e; i++) h = std::min(h, g[d][i] - g[d][i - 1]);
-            qs[l] += 2.0 * dt * kap / (h * h);
+            double h = 1e300, hall = 1e300;
+            for (int i = 1; i < n[d]; i++) {
+                const double s = g[d][i] - g[d][i - 1];
+                hall = std::min(hall, s);
+                if (i > e && i < n[d] - e) h = std::min(h, s);
+            }
+            q[l] += 2.0 * dt * kap / (h * h);
+            qall[l] += 2.0 * dt * kap / (hall * hall);
         }
     }
 }
@@ -578,9 +583,9 @@ int heat_solve(i3g_ctx *c, double *timestep)
                (const double *)H0.rocp, (const uint8_t *)H0.bc, H0.u, H0.f, dt);
         if (H0.nbc) LAUNCH(k_bc_rhs_heat, nb(H0.nbc), 256, H0.f, H0.nbc, (const int *)H0.bnode, (const double *)H0.boc);
         hbc(c, 0, true);
-        double qs[I3G_MAXLEV];
-        heat_coupling(c, kap, dt, qs);
-        HeatPlan plan = heat_plan(qs, c->nlev, c->p.t0koef, rtol);
+        double q[I3G_MAXLEV], qall[I3G_MAXLEV];
+        heat_coupling(c, kap, dt, q, qall);
+        HeatPlan plan = heat_plan(q, qall, c->nlev, c->p.t0koef, rtol);
         int it = 0;
         for (;;) {
             for (; built < plan.last; built++) {   // coefficients of the coarse levels in use

@@ -1877,9 +1877,9 @@ struct TablePack {
     {
         const size_t bytes = sizeof(T) * src.size();
         if (bytes >= kPackBytes) {
-            if (const int rc = upload(c, dst, src)) return rc;
-            L.tables.push_back((void *)dst);
-            return 0;
+            const int rc = upload(c, dst, src);
+            if (dst) L.tables.push_back((void *)dst);
+            return rc;
         }
         const size_t o = (h.size() + 255) & ~(size_t)255;   // as aligned as an allocation
         h.resize(o + std::max(bytes, sizeof(T)));
@@ -1890,8 +1890,9 @@ struct TablePack {
     int flush()
     {
         unsigned char *base = nullptr;
-        if (const int rc = upload(c, base, h)) return rc;
-        L.tables.push_back(base);
+        const int rc = upload(c, base, h);
+        if (base) L.tables.push_back(base);
+        if (rc) return rc;
         for (auto &e : at) *e.first = base + e.second;
         h.clear();
         at.clear();

@@ -14,17 +14,17 @@ def plan(tmp_path_factory):
     d = tmp_path_factory.mktemp("plan")
     src = d / "plan.cpp"
     src.write_text('#include "heat_plan.h"\n'
-                   'extern "C" int plan(const double *q, int n, double w, double rtol, int *sweeps)\n'
-                   '{ const i3g::HeatPlan P = i3g::heat_plan(q, n, w, rtol); *sweeps = P.sweeps; return P.last; }\n'
+                   'extern "C" int plan(const double *q, const double *qall, int n, double w, double rtol, int *sweeps)\n'
+                   '{ const i3g::HeatPlan P = i3g::heat_plan(q, qall, n, w, rtol); *sweeps = P.sweeps; return P.last; }\n'
                    'extern "C" double rate(double q, double w) { return i3g::heat_sweep_rate(q, w); }\n')
     subprocess.run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-I", CSRC, str(src), "-o", str(d / "plan.so")], check=True)
     L = C.CDLL(str(d / "plan.so"))
-    L.plan.argtypes = [C.POINTER(C.c_double), C.c_int, C.c_double, C.c_double, C.POINTER(C.c_int)]
+    L.plan.argtypes = [C.POINTER(C.c_double), C.POINTER(C.c_double), C.c_int, C.c_double, C.c_double, C.POINTER(C.c_int)]
     L.rate.argtypes, L.rate.restype = [C.c_double, C.c_double], C.c_double
 
-    def run(q, w=1.0, rtol=1e-10):
+    def run(q, w=1.0, rtol=1e-10, qall=None):
         s = C.c_int()
-        last = L.plan((C.c_double * len(q))(*q), len(q), w, rtol, C.byref(s))
+        last = L.plan((C.c_double * len(q))(*q), (C.c_double * len(q))(*(qall or q)), len(q), w, rtol, C.byref(s))
         return last, s.value
     run.rate = L.rate
     return run
@@ -52,6 +52,17 @@ def test_weak_coupling_stays_on_level_0(plan):
     # coarser levels: down to the first with q <= 1, which reduces its error by 1e-3
     assert plan([4.0, 1.0, 0.25]) == (1, 5)
     assert plan([1e3, 250.0, 60.0]) == (2, 16)
+
+
+def test_narrow_outer_cells_ask_for_sweeps_of_a_coarse_level(plan):
+    q = [1.8, 0.45]
+    assert plan(q) == (1, 3)
+    assert plan(q, qall=[1.8, 1.8]) == (1, 3)      # a quarter of their error in one sweep
+    q = [36.0, 9.0, 2.3, 0.6]
+    assert plan(q, qall=[36.0] * 4) == (3, 6)      # (36 / 37)^2 = 0.947 a sweep
+    q = [120.0, 30.0, 7.5, 1.9, 0.5]
+    assert plan(q, qall=[120.0] * 5) == (4, 16)
+    assert plan([0.5, 0.2], qall=[0.5, np.inf]) == (0, 11)   # level 0 has no cells of another kind
 
 
 @pytest.mark.parametrize("w", [0.5, 0.9, 1.0, 1.2, 1.6])
