@@ -39,8 +39,8 @@ inline double heat_sweeps_for(double q, double w, double left)
 // What a solve's couplings ask for.  q[l]: of level l's cells without the outermost, which stay as
 // narrow on every level as on level 0; qall[l] with them.  The last level used is the first one with q[l]
 // <= 1 (or the coarsest).  Its sweeps reduce the error by 1e-3, or by the tolerance when it is level
-// 0; at most 16, or 12 where level 0 alone is weakly coupled, since the norm after a cycle costs as
-// little there as one sweep.  A rate of 1 (rho cp / dt lost against the neighbour coefficients, or zero)
+// 0; at most 16, or 12 where coarser levels are left out, since the norm after a cycle costs as little
+// there as one sweep.  A rate of 1 (rho cp / dt lost against the neighbour coefficients, or zero)
 // takes all 16.  On a coarse level the narrow cells have to lose a quarter of their error too: with the
 // few sweeps that the others ask for, a step of ten diffusion times on 65^3 stretched nodes and four
 // coarse levels diverged, where 16 sweeps took 16 cycles.
@@ -54,7 +54,7 @@ inline HeatPlan heat_plan(const double *q, const double *qall, int nlev, double 
     P.last = l;
     double need = heat_sweeps_for(q[l], w, l == 0 ? rtol : 1e-3);
     if (l > 0) need = std::max(need, heat_sweeps_for(qall[l], w, 0.75));
-    const double most = l == 0 && q[0] <= 1.0 && heat_sweep_rate(q[0], w) < 1.0 ? 12.0 : kHeatMaxSweeps;
+    const double most = l == 0 && nlev > 1 && q[0] <= 1.0 && heat_sweep_rate(q[0], w) < 1.0 ? 12.0 : kHeatMaxSweeps;
     P.sweeps = (int)std::min(most, std::max(2.0, need));
     return P;
 }

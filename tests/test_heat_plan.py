@@ -49,6 +49,7 @@ def test_weak_coupling_stays_on_level_0(plan):
     assert plan([0.1, 0.02]) == (0, 5)
     assert plan([0.0, 0.0]) == (0, 2)
     assert plan([1.0, 0.25]) == (0, 12)
+    assert plan([1.0]) == (0, 16)
     # coarser levels: down to the first with q <= 1, which reduces its error by 1e-3
     assert plan([4.0, 1.0, 0.25]) == (1, 5)
     assert plan([1e3, 250.0, 60.0]) == (2, 16)
